@@ -511,8 +511,10 @@ __device__ __forceinline__ int64_t elemOf(AsmArgs const & a, int64_t i)
 }
 
 void launchAssembleQ1(AsmArgs const & a, cudaStream_t s, bool fp64, bool perThread, int threads);
-// the FP64 one-thread-per-element Q1 kernel (pxg_q1f64.cu), the default
+// the default Q1 kernels of the FP64 arithmetic (pxg_q1f64.cu)
 void launchAssembleQ1F64(AsmArgs const & a, cudaStream_t s, int threads);
+// its fixed-point kernel (pxg_q1fx.cu), for constant and sin sin sin loads
+void launchAssembleQ1Fx(AsmArgs const & a, cudaStream_t s, int threads);
 // element colouring (pxg_colour.cu); built once per mesh
 pxg_status buildColouring(pxg_ctx * c);
 

@@ -1,0 +1,459 @@
+// Q1 hexahedron element in 64-bit fixed point (pxg_fx.h): the steps of an element's
+// geometry, stiffness and mass tables, entries and sine load, as functions of one
+// coordinate, one quadrature point or one table, which the kernel deals to its warps.  The
+// same quantities as the FP64 form computes (pxg_q1f64.cu, whose notation this keeps), in
+// a shape that suits the format: determinants from the Jacobian's cofactors (the Gram
+// determinant, their square, would double the lost bits) and contractions on moments,
+// sums and differences of the points' values, as additions cost little and products much.
+// Compiles for the host too, where its accuracy is tested.
+//
+// Magnitudes.  Coordinates are differences to vertex 0 in units of 2^sc, the power of
+// two above the largest; the Jacobian columns (half edges) are shifted left by n_a until
+// a bound of their 1-norm over the points is in [1/2, 1), so that cofactors, their
+// products and the determinants all stay below one.  |det| is shifted to a largest value
+// in [1/2, 1) again, 1 / |det| to at most one.  Refused are elements whose columns need
+// more than 6 bits (aspect ratios beyond about 1:16), whose determinant is below 2^-7 of
+// that scale, or varies by more than 2^5 between the points: there the format could carry
+// fewer significant bits than FP64.
+#pragma once
+
+#include "pxg_fx.h"
+
+namespace pxg
+{
+namespace q1x
+{
+using namespace fx;
+
+// Constants at F = 64: g = 0.5773502691896258 (src/qr.cpp:27) and the moments' factors of
+// the 1D weights.  With m0 = v(-g) + v(g) and m1 = v(g) - v(-g): sum l_a v = (m0 + e_a g
+// m1) / 2, sum l_a l_a v = a m0 + e_a b m1, sum l_0 l_1 v = c m0, where a = (1 + g^2) / 4,
+// b = g / 2, c = (1 - g^2) / 4, e_0 = -1, e_1 = 1.
+constexpr Cst kB = cst(0x49e69d1640cc7400ll); // g / 2
+constexpr Cst kGG = cst(0x5555555555555bcall); // g^2
+// 2 W W of the two-axis tables
+constexpr Cst kAA = cst(0x38e38e38e38e3b0all); // 2 a a
+constexpr Cst kAC = cst(0x1c71c71c71c71be8ll); // 2 a c
+constexpr Cst kCC = cst(0x0e38e38e38e38d26ll); // 2 c c
+constexpr Cst kAB = cst(0x314468b980884e44ll); // 2 a b
+constexpr Cst kCB = cst(0x18a2345cc04425bcll); // 2 c b
+constexpr Cst kBB = cst(0x2aaaaaaaaaaaade5ll); // 2 b b
+// 2 l l W of the mixed tables: l = (1 + e g m1 / m0) / 2
+constexpr Cst kUA = cst(0x2aaaaaaaaaaaab79ll); // a / 2
+constexpr Cst kUC = cst(0x1555555555555487ll); // c / 2
+constexpr Cst kUB = cst(0x24f34e8b20663a00ll); // b / 2
+constexpr Cst kUAg = cst(0x18a2345cc0442722ll); // a g / 2
+constexpr Cst kUCg = cst(0x0c511a2e602212dell); // c g / 2
+constexpr Cst kUBg = cst(0x15555555555556f2ll); // b g / 2
+constexpr Cst kUAgg = cst(0x0e38e38e38e38f91ll); // a g^2 / 2
+constexpr Cst kUCgg = cst(0x071c71c71c71c761ll); // c g^2 / 2
+constexpr Cst kUBgg = cst(0x0c511a2e60221444ll); // b g^2 / 2
+// 8 W W W of the mass table
+constexpr Cst kAAA = cst(0x4bda12f684bda57dll); // 8 a a a
+constexpr Cst kAAC = cst(0x25ed097b425ed098ll); // 8 a a c
+constexpr Cst kACC = cst(0x12f684bda12f6738ll); // 8 a c c
+constexpr Cst kCCC = cst(0x097b425ed097b313ll); // 8 c c c
+constexpr Cst kAAB = cst(0x41b08ba200b5beeell); // 8 a a b
+constexpr Cst kACB = cst(0x20d845d1005add9all); // 8 a c b
+constexpr Cst kCCB = cst(0x106c22e8802d6ddell); // 8 c c b
+constexpr Cst kABB = cst(0x38e38e38e38e3e44ll); // 8 a b b
+constexpr Cst kCBB = cst(0x1c71c71c71c71d85ll); // 8 c b b
+constexpr Cst kBBB = cst(0x314468b98088510fll); // 8 b b b
+// 2 l l l of the load
+constexpr Cst kL0 = cst(0x4000000000000000ll); // 1 / 4
+constexpr Cst kL1 = cst(0x24f34e8b20663a00ll); // g / 4
+constexpr Cst kL2 = cst(0x15555555555556f2ll); // g^2 / 4
+constexpr Cst kL3 = cst(0x0c511a2e60221444ll); // g^3 / 4
+
+// sum and difference
+PXG_HD void pairSum(int64_t & a, int64_t & b)
+{
+  int64_t const s = a + b, d = b - a;
+  a = s, b = d;
+}
+// a -+ b: the values of classes 0 and 1 from the even and odd moments
+PXG_HD void pairExpand(int64_t & a, int64_t & b)
+{
+  int64_t const s = a - b, d = a + b;
+  a = s, b = d;
+}
+// moments over the three bits of the index (a set bit: difference), and back
+PXG_HD void moments(int64_t (&v)[8])
+{
+#pragma unroll
+  for (int s = 1; s < 8; s *= 2)
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (!(q & s))
+        pairSum(v[q], v[q | s]);
+}
+PXG_HD void expand(int64_t (&v)[8])
+{
+#pragma unroll
+  for (int s = 1; s < 8; s *= 2)
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (!(q & s))
+        pairExpand(v[q], v[q | s]);
+}
+PXG_HD void expand2(int64_t & v0, int64_t & v1, int64_t & v2, int64_t & v3)
+{
+  pairExpand(v0, v1), pairExpand(v2, v3);
+  pairExpand(v0, v2), pairExpand(v1, v3);
+}
+PXG_HD int64_t shl(int64_t x, int k) { return (int64_t)((uint64_t)x << k); }
+
+// ------------------------------------------------------------------- geometry
+// Columns of one coordinate r from its eight vertex values' differences to vertex 0 (d,
+// index bits x, y, z; d[0] = 0) in units of 2^sc: col[a][p] at F = 62 for the column a at
+// the points p = (qy, qz), (qx, qz), (qx, qy) (first bit lowest), and their largest high
+// words per column.
+PXG_HD void coordColumns(double const (&d)[8], int sc, int64_t (&col)[3][4], uint32_t (&cmax)[3])
+{
+  int64_t H[8];
+  H[0] = 0;
+#pragma unroll
+  for (int v = 1; v < 8; ++v)
+    H[v] = roundToInt(scaleExp(d[v], 59 - sc));
+  // the Walsh-Hadamard transform, at most 7 2^59, is eight times the mean: F = 62
+  moments(H);
+  int64_t const a110 = 2 * mulc(kB, H[3]), a101 = 2 * mulc(kB, H[5]), a011 = 2 * mulc(kB, H[6]),
+                a111 = mulc(kGG, H[7]);
+#pragma unroll
+  for (int p = 0; p < 2; ++p)
+  {
+    int64_t const u1 = p ? H[1] + a110 : H[1] - a110, u2 = p ? H[2] + a110 : H[2] - a110,
+                  u3 = p ? H[4] + a101 : H[4] - a101;
+    int64_t const w1 = p ? a101 + a111 : a101 - a111, w2 = p ? a011 + a111 : a011 - a111;
+    col[0][p] = u1 - w1, col[0][p + 2] = u1 + w1; // (qy = p, qz)
+    col[1][p] = u2 - w2, col[1][p + 2] = u2 + w2; // (qx = p, qz)
+    col[2][p] = u3 - w2, col[2][p + 2] = u3 + w2; // (qx = p, qy)
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+  {
+    uint32_t m = 0;
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+    {
+      int32_t const h = hi32(col[a][p]);
+      uint32_t const t = (uint32_t)(h < 0 ? -h : h);
+      m = t > m ? t : m;
+    }
+    cmax[a] = m;
+  }
+}
+// exponent of the largest difference: sc, and whether the format takes it (finite, and
+// the conversions' exponents in range)
+PXG_HD int coordScale(int32_t maxHi) { return (maxHi >> 20) - 1022; }
+PXG_HD bool coordScaleOk(int sc) { return sc >= -300 && sc <= 59; }
+
+// Column shifts from the largest high words cmax[a * 3 + r]
+struct Shifts
+{
+  int n[3], nmin, nmax;
+};
+PXG_HD bool columnShifts(uint32_t const (&cmax)[9], Shifts & s)
+{
+  bool ok = true;
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+  {
+    s.n[a] = clz32(cmax[3 * a] + cmax[3 * a + 1] + cmax[3 * a + 2]) - 2;
+    ok = ok && s.n[a] >= 0 && s.n[a] <= 6;
+  }
+  s.nmax = s.n[0] > s.n[1] ? s.n[0] : s.n[1];
+  s.nmax = s.nmax > s.n[2] ? s.nmax : s.n[2];
+  s.nmin = s.n[0] < s.n[1] ? s.n[0] : s.n[1];
+  s.nmin = s.nmin < s.n[2] ? s.nmin : s.n[2];
+  return ok;
+}
+
+// One point: the cofactors A, B, C of its shifted columns a, b, d, |det| and the products
+// xx yy zz xy xz yz, all at F = 60
+PXG_HD int64_t pointProducts(Sp const (&a)[3], Sp const (&b)[3], Sp const (&d)[3], int64_t (&G)[6])
+{
+  Sp A[3], B[3], C[3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+  {
+    int const s = (r + 1) % 3, t = (r + 2) % 3;
+    A[r] = split(shl(dot2(b[s], d[t], neg(b[t]), d[s]), 2)); // F = 62
+    B[r] = split(shl(dot2(d[s], a[t], d[t], neg(a[s])), 2));
+    C[r] = split(shl(dot2(a[s], b[t], a[t], neg(b[s])), 2));
+  }
+  int64_t const v = dot3(a, A);
+  G[0] = dot3(A, A), G[1] = dot3(B, B), G[2] = dot3(C, C);
+  G[3] = dot3(A, B), G[4] = dot3(A, C), G[5] = dot3(B, C);
+  return v < 0 ? -v : v;
+}
+
+// Shifts of the determinants from the high words of |det| at the eight points: nd to the
+// left (the largest in [1/2, 1) at F = 60), then 2^-k for the inverses (at most one)
+PXG_HD bool detShifts(uint32_t lo, uint32_t hi, int & nd, int & k)
+{
+  nd = clz32(hi) - 4;
+  bool const ok = nd >= 0 && nd <= 6 && (lo << (nd & 7)) > (1u << 22);
+  k = clz32(lo) - 4 - nd + 1; // lo 2^nd >= 2^(28 - k)
+  return ok;
+}
+// The largest diagonal product of a point, aligned to the common exponent (high word),
+// and the shift to the left its maximum over the points leaves
+PXG_HD uint32_t productSize(int64_t const (&G)[6], Shifts const & s)
+{
+  uint32_t const a = (uint32_t)hi32(G[0]) >> (2 * (s.nmax - s.n[0])), b = (uint32_t)hi32(G[1]) >> (2 * (s.nmax - s.n[1])),
+                 c = (uint32_t)hi32(G[2]) >> (2 * (s.nmax - s.n[2]));
+  uint32_t const m = a > b ? a : b;
+  return m > c ? m : c;
+}
+PXG_HD int productShift(uint32_t size)
+{
+  int const k = clz32(size) - 4;
+  return k < 0 ? 0 : (k > 12 ? 12 : k);
+}
+// exponents: det = det' 2^-60 2^eD (after the shift nd), G = G' 2^-58 2^eG
+PXG_HD int detExponent(int sc, Shifts const & s, int nd) { return 3 * sc - (s.n[0] + s.n[1] + s.n[2]) - nd; }
+PXG_HD int tensorExponent(int sc, Shifts const & s, int nd, int k, int sg)
+{
+  return k + nd + sc - (s.n[0] + s.n[1] + s.n[2]) + 2 * s.nmax - sg;
+}
+// G = km |J| (J^T J)^-1 at one point (F = 58) from its products and shifted det: times
+// 2^-k km / |det|, the components aligned to one exponent
+PXG_HD void pointInverse(int64_t det, int k, int sg, Sp km, Shifts const & s, int64_t (&G)[6])
+{
+  Sp const y = split(shl(mul(split(shl(recip(det), 6 - k)), km), 2));
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+  {
+    int const a = c < 3 ? c : (c == 5 ? 1 : 0), b = c < 3 ? c : (c == 3 ? 1 : 2);
+    int const t = sg - (2 * s.nmax - s.n[a] - s.n[b]);
+    G[c] = mul(split(shl(G[c], t > 0 ? t : 0)), y) >> (t > 0 ? 0 : -t);
+  }
+}
+
+// --------------------------------------------------------------------- tables
+// Class tables of the stiffness, twice the sums over the points at the scale of G: class
+// 0 / 1 of two equal 1D indices, 2 of a mixed pair.  S_x[cy][cz], S_y[cx][cz], S_z[cx][cy]
+// (S[c][ce][cf]) and U_xy[jx][iy][cz], U_xz[jx][iz][cy], U_yz[jy][iz][cx] (U[c][a][b][w]),
+// numbered one after the other.
+constexpr int kTables = 63;
+PXG_HD constexpr int idxS(int c, int ce, int cf) { return c * 9 + ce * 3 + cf; }
+PXG_HD constexpr int idxU(int c, int a, int b, int w) { return 27 + c * 12 + (a * 2 + b) * 3 + w; }
+// S of one component from its points v: bit 0 the axis summed out, W over bits 1 and 2
+PXG_HD void tableS(int64_t const (&v)[8], int64_t (&S)[9])
+{
+  int64_t n00 = v[0] + v[1], n10 = v[2] + v[3], n01 = v[4] + v[5], n11 = v[6] + v[7];
+  pairSum(n00, n10), pairSum(n01, n11);
+  pairSum(n00, n01), pairSum(n10, n11);
+  S[0] = mulc(kAA, n00), S[3] = mulc(kAB, n10), S[1] = mulc(kAB, n01), S[4] = mulc(kBB, n11);
+  expand2(S[0], S[3], S[1], S[4]);
+  S[2] = mulc(kAC, n00), S[5] = mulc(kCB, n10);
+  S[6] = S[2], S[7] = mulc(kCB, n01);
+  pairExpand(S[2], S[5]), pairExpand(S[6], S[7]);
+  S[8] = mulc(kCC, n00);
+}
+// U of one component: l over bits 0 (a) and 1 (b), W over bit 2
+PXG_HD void tableU(int64_t (&m)[8], int64_t (&U)[12])
+{
+  moments(m);
+  int64_t A[4], B[4], C[4]; // index a + 2 b
+  A[0] = mulc(kUA, m[0]), A[1] = mulc(kUAg, m[1]), A[2] = mulc(kUAg, m[2]), A[3] = mulc(kUAgg, m[3]);
+  B[0] = mulc(kUB, m[4]), B[1] = mulc(kUBg, m[5]), B[2] = mulc(kUBg, m[6]), B[3] = mulc(kUBgg, m[7]);
+  C[0] = mulc(kUC, m[0]), C[1] = mulc(kUCg, m[1]), C[2] = mulc(kUCg, m[2]), C[3] = mulc(kUCgg, m[3]);
+  expand2(A[0], A[1], A[2], A[3]), expand2(B[0], B[1], B[2], B[3]), expand2(C[0], C[1], C[2], C[3]);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+  {
+    int const u = ((k & 1) * 2 + (k >> 1)) * 3;
+    U[u] = A[k] - B[k], U[u + 1] = A[k] + B[k], U[u + 2] = C[k];
+  }
+}
+
+PXG_HD constexpr int cls(int a, int b) { return a == b ? a : 2; }
+template <bool PLUS>
+PXG_HD int64_t acc(int64_t a, int64_t b)
+{
+  return PLUS ? a + b : a - b;
+}
+
+// The entries of the y/z block (iy, iz), (jy, jz) and its x pairs, eight times K_ij at
+// the scale of G: K(ix, jx) = e_ix e_jx Sx + e_ix F[jx] + e_jx F'[ix] + T[c(ix, jx)].
+// t(k) is table value k.
+template <int iy, int iz, int jy, int jz, class T>
+PXG_HD void entryBlock(T const & t, int64_t (&K)[2][2])
+{
+  constexpr int cy = cls(iy, jy), cz = cls(iz, jz);
+  constexpr bool yy = iy == jy, zz = iz == jz, yz = iy == jz, zy = jy == iz; // e e > 0
+  constexpr bool diag = yy && zz;
+  int64_t X[3];
+#pragma unroll
+  for (int cx = 0; cx < 3; ++cx)
+  {
+    // e_iy e_jy Sy + e_iz e_jz Sz + e_iy e_jz U(jy, iz) + e_jy e_iz U(iy, jz)
+    int64_t const sy = t(idxS(1, cx, cz)), s = acc<zz>(yy ? sy : -sy, t(idxS(2, cx, cy)));
+    if constexpr (diag)
+      X[cx] = acc<yz>(s, 2 * t(idxU(2, jy, iz, cx)));
+    else
+      X[cx] = acc<yz>(acc<zy>(s, t(idxU(2, iy, jz, cx))), t(idxU(2, jy, iz, cx)));
+  }
+  int64_t F[2], Fp[2];
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+  {
+    int64_t const f = t(idxU(0, x, iy, cz));
+    F[x] = acc<jz == 1>(jy ? f : -f, t(idxU(1, x, iz, cy)));
+    if constexpr (diag)
+      Fp[x] = F[x];
+    else
+    {
+      int64_t const fp = t(idxU(0, x, jy, cz));
+      Fp[x] = acc<iz == 1>(iy ? fp : -fp, t(idxU(1, x, jz, cy)));
+    }
+  }
+  int64_t const sx = t(idxS(0, cy, cz));
+#pragma unroll
+  for (int ix = 0; ix < 2; ++ix)
+#pragma unroll
+    for (int jx = 0; jx < 2; ++jx)
+    {
+      if (diag && jx < ix)
+        continue;
+      int64_t k = X[cls(ix, jx)];
+      k = jx ? k + Fp[ix] : k - Fp[ix];
+      k = ix ? k + F[jx] : k - F[jx];
+      K[ix][jx] = ix == jx ? k + sx : k - sx;
+    }
+}
+
+// Mass class table, eight times Mt[cx][cy][cz] = sum_q v_q W W W at the scale of the
+// points' values v (below one at F = 58)
+PXG_HD void massTable(int64_t (&v)[8], int64_t (&M)[3][3][3])
+{
+  moments(v);
+  int64_t w[8];
+  w[0] = mulc(kAAA, v[0]);
+  w[1] = mulc(kAAB, v[1]), w[2] = mulc(kAAB, v[2]), w[4] = mulc(kAAB, v[4]);
+  w[3] = mulc(kABB, v[3]), w[5] = mulc(kABB, v[5]), w[6] = mulc(kABB, v[6]);
+  w[7] = mulc(kBBB, v[7]);
+  expand(w);
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    M[q & 1][(q >> 1) & 1][q >> 2] = w[q];
+  // one mixed axis, two mixed axes
+  int64_t const aac = mulc(kAAC, v[0]), x = mulc(kACB, v[1]), y = mulc(kACB, v[2]), z = mulc(kACB, v[4]);
+  M[2][0][0] = aac, M[2][1][0] = y, M[2][0][1] = z, M[2][1][1] = mulc(kCBB, v[6]);
+  expand2(M[2][0][0], M[2][1][0], M[2][0][1], M[2][1][1]);
+  M[0][2][0] = aac, M[1][2][0] = x, M[0][2][1] = z, M[1][2][1] = mulc(kCBB, v[5]);
+  expand2(M[0][2][0], M[1][2][0], M[0][2][1], M[1][2][1]);
+  M[0][0][2] = aac, M[1][0][2] = x, M[0][1][2] = y, M[1][1][2] = mulc(kCBB, v[3]);
+  expand2(M[0][0][2], M[1][0][2], M[0][1][2], M[1][1][2]);
+  int64_t const acc0 = mulc(kACC, v[0]);
+  M[0][2][2] = acc0, M[1][2][2] = mulc(kCCB, v[1]);
+  M[2][0][2] = acc0, M[2][1][2] = mulc(kCCB, v[2]);
+  M[2][2][0] = acc0, M[2][2][1] = mulc(kCCB, v[4]);
+  pairExpand(M[0][2][2], M[1][2][2]), pairExpand(M[2][0][2], M[2][1][2]), pairExpand(M[2][2][0], M[2][2][1]);
+  M[2][2][2] = mulc(kCCC, v[0]);
+}
+
+// ------------------------------------------------------------------ sine load
+// sin(pi (o + d)) at the points, d = J xi: with u = the signed column sums at F = 63 of
+// their quarter, pi d = 4 pi g 2^p u, and the Taylor series about o in u, Horner from
+// the top.  A step multiplies by u at F = 63 and so loses one bit: coefficient k is kept
+// at F = 62 + k, scaled by 2^-e so that it holds for p <= -3.
+struct SerC
+{
+  Cst m; // (4 pi g)^k / k! = m 2^j
+  int j;
+};
+PXG_HD constexpr SerC serC(int k)
+{
+  constexpr SerC t[15] = {
+      {cst(0x3a0aa4f6dc87a652ll), 5},
+      {cst(0x34a34cc4a60faa41ll), 7},
+      {cst(0x3fa653af99556461ll), 8},
+      {cst(0x39b951e3ef7ba41dll), 9},
+      {cst(0x53c27987d5f2ba05ll), 9},
+      {cst(0x32a41d9d01c719aell), 10},
+      {cst(0x347cbede9f4066dfll), 10},
+      {cst(0x2f99c7c1b08f6eball), 10},
+      {cst(0x4cbeb872823ea0c4ll), 9},
+      {cst(0x37ae156aab47d0ecll), 9},
+      {cst(0x4972f1a42e34445cll), 8},
+      {cst(0x58d08305dcd934c0ll), 7},
+      {cst(0x31911161a51cebd5ll), 7},
+      {cst(0x335faba26fce95fall), 6},
+      {cst(0x31b2653d29e4b398ll), 5},
+  };
+  return t[k - 1];
+}
+constexpr int kLoadMaxP = -3;       // largest p
+constexpr float kLoadMaxT = 0.5f;   // largest |pi d| of degree 15 (0.07: 9, 0.0205: 7): truncation below 8e-19
+// a bound of |pi d| for the coordinate r
+PXG_HD float offsetBound(uint32_t const (&cmax)[9], int r, int sc)
+{
+  // pi g 2^(sc - 30) sum_a cmax: the scale as a float's exponent (sc >= -300: below the
+  // smallest float it is zero)
+  float const f = (float)(cmax[r] + cmax[3 + r] + cmax[6 + r]) * (1.8138f / 1073741824.f);
+#ifdef __CUDA_ARCH__
+  return ldexpf(f, sc);
+#else
+  return __builtin_ldexpf(f, sc);
+#endif
+}
+// Series of one coordinate from S, C = sin, cos of pi o: the coefficients k[0..DEG] and
+// the shift nf that normalises the sum; returns e with sin = sum 2^-62 2^e after it
+template <int DEG>
+PXG_HD int seriesCoefs(double S, double C, int p, float bound, int64_t (&k)[DEG + 1], int & nf)
+{
+  int es = expoField(S) - 1022;
+  es = es < -400 ? -400 : es;
+#ifdef __CUDA_ARCH__
+  int const et = (__float_as_int(bound) >> 23) - 126; // bound < 2^et
+#else
+  int const et = bound > 0.f ? __builtin_ilogbf(bound) + 1 : -126;
+#endif
+  int const e = 1 + (es > p + 5 ? es : p + 5), en = 1 + (es > et ? es : et);
+  nf = e > en ? e - en : 0;
+  nf = nf < 40 ? nf : 40;
+  int64_t const s = roundToInt(scaleExp(S, 62)), c = roundToInt(scaleExp(C, 62));
+  k[0] = es <= -400 ? 0 : roundToInt(scaleExp(S, 62 - e));
+#pragma unroll
+  for (int i = 1; i <= DEG; ++i)
+  {
+    int const sr = e - serC(i).j - i * (p + 1);
+    int64_t const v = mulc(serC(i).m, (i & 1) ? c : s) >> (sr < 63 ? sr : 63);
+    k[i] = (i & 2) ? -v : v;
+  }
+  return e - nf;
+}
+// the offset of one point and coordinate: the signed sum of its shifted columns, F = 63
+// of its quarter
+PXG_HD Sp pointOffset(Sp a, Sp b, Sp d, int q, Shifts const & s)
+{
+  int64_t const x = (shl((int64_t)a.h, 32) + a.l) >> (s.n[0] - s.nmin + 1);
+  int64_t const y = (shl((int64_t)b.h, 32) + b.l) >> (s.n[1] - s.nmin + 1);
+  int64_t const z = (shl((int64_t)d.h, 32) + d.l) >> (s.n[2] - s.nmin + 1);
+  int64_t t = (q & 4) ? z : -z;
+  t = (q & 2) ? t + y : t - y;
+  t = (q & 1) ? t + x : t - x;
+  return split(t);
+}
+// |det| sin sin sin from the three normalised values: F = 59
+PXG_HD int64_t pointLoad(int64_t f0, int64_t f1, int64_t f2, int64_t det)
+{
+  int64_t const f = shl(mul(split(f0), split(f1)), 2), g = shl(mul(split(f2), split(shl(det, 2))), 2);
+  return mul(split(f), split(g)) >> 1;
+}
+// twice sum_q r_q l l l at the eight nodes (index bits x, y, z)
+PXG_HD void nodeSums(int64_t (&r)[8])
+{
+  moments(r);
+  r[0] = mulc(kL0, r[0]);
+  r[1] = mulc(kL1, r[1]), r[2] = mulc(kL1, r[2]), r[4] = mulc(kL1, r[4]);
+  r[3] = mulc(kL2, r[3]), r[5] = mulc(kL2, r[5]), r[6] = mulc(kL2, r[6]);
+  r[7] = mulc(kL3, r[7]);
+  expand(r);
+}
+
+} // namespace q1x
+} // namespace pxg
