@@ -186,7 +186,7 @@ PXG_HD int64_t mulc(Cst c, int64_t x)
 // an integer times 2^k as a double, correctly rounded (k keeps it normal)
 PXG_HD double toDouble(int64_t x, int k) { return scaleExp((double)x, k); }
 
-// 1 / d for d at F = 60 in [2^-6, 1): F = 56, relative error below 2^-55.  A float
+// 1 / d for d at F = 60 in [1/2, 1): F = 56, relative error below 2^-55.  A float
 // estimate y0 (relative error e below 2^-21), then y0 (1 + e + e^2), e = 1 - d y0.
 PXG_HD int64_t recip(int64_t d)
 {

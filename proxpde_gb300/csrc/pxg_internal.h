@@ -438,7 +438,38 @@ struct AsmArgs
   int grpRedMax;
   // launched as a programmatic dependent of the zeroing of its outputs (pdlWait)
   int pdl;
+  // what the operators come to for the kernels that fold them (foldOps)
+  struct Fold
+  {
+    // needK / needM: some operator has a stiffness / mass; foldK / foldM: exactly one has,
+    // its coefficient sK / sM (times k_e with coefK / coefM) goes into the values, for the
+    // array K / M; simple: each needed one is folded; same: both in one operator; bc: some
+    // operator has Dirichlet conditions (bcK, bcM: that of K, of M)
+    bool needK, needM, foldK, foldM, coefK, coefM, simple, same, bc, bcK, bcM, coef;
+    double sK, sM;
+    double *K, *M;
+  } fold;
 };
+
+inline void foldOps(AsmArgs & a)
+{
+  AsmArgs::Fold & f = a.fold;
+  bool k[2], m[2];
+  for (int i = 0; i < 2; ++i)
+    k[i] = a.op[i].on && a.op[i].stiff, m[i] = a.op[i].on && a.op[i].mass;
+  f.needK = k[0] || k[1], f.needM = m[0] || m[1];
+  f.foldK = k[0] != k[1], f.foldM = m[0] != m[1];
+  LhsDev const & ok = a.op[k[0] ? 0 : 1];
+  LhsDev const & om = a.op[m[0] ? 0 : 1];
+  f.sK = f.foldK ? ok.sc : 1., f.sM = f.foldM ? om.mc : 1.;
+  f.coefK = f.foldK && ok.stiff == 2, f.coefM = f.foldM && om.mass == 2;
+  f.coef = (usesCoef(a.op[0]) || usesCoef(a.op[1])) && a.kE;
+  f.K = f.needK ? ok.vals : nullptr, f.M = f.needM ? om.vals : nullptr;
+  f.simple = (f.foldK || !f.needK) && (f.foldM || !f.needM) && (f.needK || f.needM);
+  f.same = f.needK && f.needM && k[0] == m[0];
+  f.bcK = f.needK && ok.bc, f.bcM = f.needM && om.bc;
+  f.bc = (a.op[0].on && a.op[0].bc) || (a.op[1].on && a.op[1].bc);
+}
 
 // The default FP64 element kernels run as programmatic dependents of the kernel that
 // zeroes their outputs: their blocks start while the (DRAM-bound) zeroing runs, compute
@@ -511,10 +542,8 @@ __device__ __forceinline__ int64_t elemOf(AsmArgs const & a, int64_t i)
 }
 
 void launchAssembleQ1(AsmArgs const & a, cudaStream_t s, bool fp64, bool perThread, int threads);
-// the default Q1 kernels of the FP64 arithmetic (pxg_q1f64.cu)
+// the default Q1 kernel of the FP64 arithmetic (pxg_q1fx.cu)
 void launchAssembleQ1F64(AsmArgs const & a, cudaStream_t s, int threads);
-// its fixed-point kernel (pxg_q1fx.cu), for constant and sin sin sin loads
-void launchAssembleQ1Fx(AsmArgs const & a, cudaStream_t s, int threads);
 // element colouring (pxg_colour.cu); built once per mesh
 pxg_status buildColouring(pxg_ctx * c);
 

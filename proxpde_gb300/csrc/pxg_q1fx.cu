@@ -39,29 +39,32 @@ struct Q1Shared
   };
   union
   {
-    int64_t G[48][32];  // component c at point q: c * 8 + q
-    double kval[32][37]; // entries of the stiffness (an odd stride: no bank conflicts)
+    int64_t G[48][32];    // component c at point q: c * 8 + q
+    double kval[32][37];  // entries of the stiffness (an odd stride: no bank conflicts)
+    int64_t off[3][8][32]; // offsets of the points, before G
   };
   union
   {
-    int64_t rq[8][32];     // load values of the points
-    double sc[6][32];      // sine, cosine of pi times the origin
+    int64_t rq[8][32]; // load values of the points
+    double rqd[8][32]; // the same in FP64
+    int64_t sm[6][32]; // sine, cosine of pi times the origin: mantissas
   };
+  int se[6][32]; // and exponents
+  double org[3][32];
+  int64_t det[8][32];
   union
   {
-    int64_t det[8][32];
-    int32_t dmax[3][32]; // high word of the largest difference per coordinate
-  };
-  union
-  {
-    double mval[32][27]; // the mass table
+    int64_t mtab[32][27]; // the mass table, then as doubles
+    double mval[32][27];
     uint32_t psize[8][32];
+    int32_t dmax[3][32]; // high word of the largest difference per coordinate
   };
   uint32_t cmax[9][32];
   uint32_t dof[8][32];
-  int32_t rp[8][32];
-  int32_t ee[3][32], nf[3][32]; // exponents and shifts of the sine series
-  int32_t scale[32];
+  int32_t rp[32][8];
+  int32_t ee[3][32];            // exponents of the sine series
+  float bound[3][32];           // bounds of its argument
+  int32_t el[32];               // exponent of the load values
   uint32_t flags[32]; // bits 0-7 constrained nodes, 8 in the mesh, 9 fixed point holds it
 };
 
@@ -100,6 +103,79 @@ __device__ __forceinline__ void entriesOut(Q1Shared & sh, int l, int eK)
         sh.kval[l][base + (a == b ? ix + jx : 2 * ix + jx)] = q1x::toDouble(K[ix][jx], eK);
 }
 
+// an analytic function at a point, out of line
+__device__ __noinline__ double evalPoint(int fn, double x, double y, double z) { return evalFn(fn, 1.0, x, y, z); }
+// sum_n phi_n field_n at point q: one axis at a time, l_a = A on the node's side, B on the other
+__device__ __noinline__ double fieldPoint(double const * field, Q1Shared const & sh, int l, int q)
+{
+  double f[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    f[k] = field[sh.dof[q1f::node((k ^ q) & 1, ((k ^ q) >> 1) & 1, (k ^ q) >> 2)][l]];
+#pragma unroll
+  for (int t = 1; t < 8; t *= 2)
+#pragma unroll
+    for (int k = 0; k < 8; k += 2 * t)
+      f[k] = fma(q1f::A, f[k], q1f::B * f[k | t]);
+  return f[0];
+}
+
+// Dirichlet condensation (builder.hpp:76-124) of entry (i, j) of element el under the
+// operator of K (with k) and of M (with m): the diagonal of a constrained DOF, the lift
+// -K_ij h_j of a free row
+__device__ __forceinline__ void condense(AsmArgs const & a, Q1Shared const & sh, int el, int i, int j, bool k, bool m,
+                                         bool ci, int32_t pij, double kv, double mv)
+{
+  if (i == j)
+  {
+    if (k)
+      atomicAdd(a.fold.K + pij, a.bcDiag);
+    if (m)
+      atomicAdd(a.fold.M + pij, a.bcDiag);
+  }
+  else if (!ci && a.b && (k || m))
+  {
+    double const z = ((k ? kv : 0.) + (m ? mv : 0.)) * a.bcVal[sh.dof[j][el]];
+    if (z != 0.)
+      atomicAdd(a.b + sh.dof[i][el], -z);
+  }
+}
+
+// Entry (i, j) of the block's element el for any operators and with the Dirichlet
+// condensation (builder.hpp:76-124): the diagonal of a constrained DOF, the lift -K_ij h_j
+// of a free row.  kx, mx: its places in the stiffness and mass values.
+__device__ __noinline__ void scatterGeneral(AsmArgs const & a, Q1Shared const & sh, int el, int i, int j, int kx, int mx)
+{
+  int64_t const e = elemOf(a, blockIdx.x * 32ll + el);
+  int32_t const pij = sh.rp[el][i] + a.rank[e * 64 + i * 8 + j];
+  uint32_t const cons = sh.flags[el] & 0xffu;
+  bool const ci = (cons >> i) & 1u, cj = (cons >> j) & 1u;
+  double const kfac = a.fold.coef ? a.kE[e] : 1.0;
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+  {
+    LhsDev const & op = a.op[m];
+    if (!op.on)
+      continue;
+    // a single operator's coefficient is folded into the values
+    double const kf = a.fold.foldK ? 1. : (op.stiff == 2 ? op.sc * kfac : op.sc),
+                 mf = a.fold.foldM ? 1. : massCoef(op, kfac);
+    double val = op.stiff ? kf * sh.kval[el][kx] : mf * sh.mval[el][mx];
+    if (op.stiff && op.mass)
+      val = fma(mf, sh.mval[el][mx], val);
+    if (!(op.bc && (ci || cj)))
+      atomicAdd(op.vals + pij, val);
+    else if (i == j)
+      atomicAdd(op.vals + pij, a.bcDiag);
+    else if (!ci && a.b)
+    {
+      double const z = val * a.bcVal[sh.dof[j][el]];
+      if (z != 0.)
+        atomicAdd(a.b + sh.dof[i][el], -z);
+    }
+  }
+}
+
 // out of line: the few elements the fixed-point form refuses
 __device__ __noinline__ void elementF64Rare(AsmArgs const & a, int64_t e) { elementF64(a, e); }
 
@@ -114,18 +190,17 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
   int64_t const i0 = blockIdx.x * 32ll + l;
   bool const inMesh = i0 < a.nelem;
   int64_t const e = elemOf(a, inMesh ? i0 : a.nelem - 1);
-  LhsDev const & op0 = a.op[0];
-  LhsDev const & op1 = a.op[1];
-  bool const k0 = op0.on && op0.stiff, k1 = op1.on && op1.stiff;
-  bool const m0 = op0.on && op0.mass, m1 = op1.on && op1.mass;
-  bool const needK = k0 || k1, needM = m0 || m1;
-  bool const sine = a.rkind && a.fn == PXG_FN_SIN3;
+  bool const needK = a.fold.needK, needM = a.fold.needM;
+  // loads: sin sin sin by its series, a constant, and anything else (another function, the
+  // projection of a DOF field, elements too large for the series) point by point in FP64
+  bool const analytic = a.rkind == 1 && a.fn != PXG_FN_CONST, sine = a.rkind == 1 && a.fn == PXG_FN_SIN3;
 
   // ---- 0. inputs
+  double const kfac = a.fold.coef ? a.kE[e] : 1.0;
   double d[8];
   if (w < 6)
   {
-    if (w < 3 || sine)
+    if (w < 3 || analytic)
     {
       int const r = w < 3 ? w : w - 3;
       uint4 const c0 = reinterpret_cast<uint4 const *>(a.conn)[2 * e];
@@ -147,14 +222,6 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
         }
         sh.dmax[r][l] = m;
       }
-      else
-      {
-        // element origin = vertex average (geo.hpp:721-728)
-        double const o = 0.125 * (((d[0] + d[1]) + (d[2] + d[3])) + ((d[4] + d[5]) + (d[6] + d[7])));
-        double S, C;
-        sinCosPiTab(o, S, C);
-        sh.sc[r][l] = S, sh.sc[3 + r][l] = C;
-      }
     }
   }
   else if (w == 6)
@@ -167,21 +234,30 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
     for (int n = 0; n < 8; ++n)
     {
       sh.dof[n][l] = dof[n];
-      sh.rp[n][l] = a.rowPtr[dof[n]];
+      sh.rp[l][n] = a.rowPtr[dof[n]];
       if (a.bcMask && a.bcMask[dof[n]])
         cons |= 1u << n;
     }
     sh.flags[l] = cons;
   }
   __syncthreads();
+  int sc[3];
+  bool ok = q1x::coordScales(sh.dmax[0][l], sh.dmax[1][l], sh.dmax[2][l], sc);
+  int const scMin = min(sc[0], min(sc[1], sc[2]));
   if (w < 3)
   {
-    int32_t m = sh.dmax[0][l] > sh.dmax[1][l] ? sh.dmax[0][l] : sh.dmax[1][l];
-    m = m > sh.dmax[2][l] ? m : sh.dmax[2][l];
-    int const sc = q1x::coordScale(m);
+    int const scw = w == 0 ? sc[0] : (w == 1 ? sc[1] : sc[2]);
     int64_t col[3][4];
     uint32_t cm[3];
-    q1x::coordColumns(d, sc, col, cm);
+    int64_t off[8];
+    q1x::coordColumns(d, scw, col, cm, off);
+    if (analytic)
+    {
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        sh.off[w][q][l] = off[q];
+      sh.bound[w][l] = q1x::offsetBound(cm, scw);
+    }
 #pragma unroll
     for (int c = 0; c < 3; ++c)
     {
@@ -190,79 +266,73 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
         sh.col[(c * 3 + w) * 4 + p][l] = col[c][p];
       sh.cmax[c * 3 + w][l] = cm[c];
     }
-    if (w == 0)
-      sh.scale[l] = sc;
+  }
+  else if (w < 6 && analytic)
+  {
+    // element origin = vertex average (geo.hpp:721-728)
+    double const o = 0.125 * (((d[0] + d[1]) + (d[2] + d[3])) + ((d[4] + d[5]) + (d[6] + d[7])));
+    sh.org[w - 3][l] = o;
+    double t[2] = {0., 0.};
+    if (sine)
+      sinCosPiTab(o, t[0], t[1]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+    {
+      int64_t m;
+      int x;
+      q1x::sineParts(t[i], m, x);
+      sh.sm[2 * (w - 3) + i][l] = m, sh.se[2 * (w - 3) + i][l] = x;
+      if (i == 0)
+        sh.ee[w - 3][l] = q1x::seriesExponent(x, w == 3 ? sc[0] : (w == 4 ? sc[1] : sc[2]));
+    }
   }
   __syncthreads();
 
   // ---- 1. scales, and one point per warp
-  int const sc = sh.scale[l];
   q1x::Shifts s;
   int deg = 0;
-  bool ok;
+  bool series = false;
   {
     uint32_t cm[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k)
       cm[k] = sh.cmax[k][l];
-    ok = q1x::columnShifts(cm, s) && q1x::coordScaleOk(sc);
+    ok = q1x::columnShifts(cm, s) && ok;
     if (sine)
     {
-      float const b0 = q1x::offsetBound(cm, 0, sc), b1 = q1x::offsetBound(cm, 1, sc), b2 = q1x::offsetBound(cm, 2, sc);
-      float const bm = fmaxf(b0, fmaxf(b1, b2));
-      int const p = sc - s.nmin;
-      ok = ok && p <= q1x::kLoadMaxP && bm <= q1x::kLoadMaxT;
-      // one degree for the block (every warp sees the same elements)
-      uint32_t const t = __reduce_max_sync(0xffffffffu, ok ? __float_as_uint(bm) : 0u);
-      deg = t <= __float_as_uint(0.0205f) ? 7 : (t <= __float_as_uint(0.07f) ? 9 : 15);
-      if (w >= 3 && w < 6)
-      {
-        int const r = w - 3;
-        float const b = r == 0 ? b0 : (r == 1 ? b1 : b2);
-        double const S = sh.sc[r][l], C = sh.sc[3 + r][l];
-        int64_t k[16];
-        int nf, es;
-        if (deg == 7)
-          es = q1x::seriesCoefs<7>(S, C, p, b, reinterpret_cast<int64_t(&)[8]>(k), nf);
-        else if (deg == 9)
-          es = q1x::seriesCoefs<9>(S, C, p, b, reinterpret_cast<int64_t(&)[10]>(k), nf);
-        else
-          es = q1x::seriesCoefs<15>(S, C, p, b, k, nf);
+      float const bm = fmaxf(sh.bound[0][l], fmaxf(sh.bound[1][l], sh.bound[2][l]));
+      series = ok && max(sc[0], max(sc[1], sc[2])) <= q1x::kLoadMaxScale && bm <= q1x::kLoadMaxT;
+      // one degree for the block (every warp sees the same elements); a warp forms the
+      // coefficients w, w + 8 of each coordinate
+      deg = q1x::seriesDegree(__uint_as_float(__reduce_max_sync(0xffffffffu, series ? __float_as_uint(bm) : 0u)));
+      for (int i = w; i <= deg; i += 8)
 #pragma unroll
-        for (int i = 0; i < 16; ++i)
-          if (i <= deg)
-            sh.coef[r][i][l] = k[i];
-        sh.ee[r][l] = es;
-        sh.nf[r][l] = nf;
-      }
+        for (int r = 0; r < 3; ++r)
+          sh.coef[r][i][l] =
+              q1x::seriesCoef(sh.ee[r][l], sc[r], i, sh.sm[2 * r + (i & 1)][l], sh.se[2 * r + (i & 1)][l]);
     }
   }
   int64_t G[6];
   int64_t det;
-  Sp u[3];
+  int64_t u[3];
   {
     Sp c1[3], c2[3], c3[3];
     int const p1 = w >> 1, p2 = (w & 1) | ((w >> 2) << 1), p3 = w & 3;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
     {
-      c1[r] = q1x::splitOdd(q1x::shl(sh.col[r * 4 + p1][l], s.n[0]));
-      c2[r] = q1x::splitOdd(q1x::shl(sh.col[(3 + r) * 4 + p2][l], s.n[1]));
-      c3[r] = q1x::splitOdd(q1x::shl(sh.col[(6 + r) * 4 + p3][l], s.n[2]));
-      if (sine)
-        u[r] = q1x::pointOffset(c1[r], c2[r], c3[r], w, s);
+      int64_t const x = sh.col[r * 4 + p1][l], y = sh.col[(3 + r) * 4 + p2][l], z = sh.col[(6 + r) * 4 + p3][l];
+      c1[r] = q1x::splitOdd(q1x::shl(x, s.n[0]));
+      c2[r] = q1x::splitOdd(q1x::shl(y, s.n[1]));
+      c3[r] = q1x::splitOdd(q1x::shl(z, s.n[2]));
+      u[r] = analytic ? sh.off[r][w][l] : 0;
     }
-    det = q1x::pointProducts(c1, c2, c3, G);
+    int const wt[3] = {sc[0] - scMin, sc[1] - scMin, sc[2] - scMin};
+    det = q1x::pointProducts(c1, c2, c3, __any_sync(0xffffffffu, (wt[0] | wt[1] | wt[2]) != 0) != 0, wt, G);
     sh.det[w][l] = det;
     sh.psize[w][l] = q1x::productSize(G, s);
   }
   __syncthreads();
-  double const kfac = ((usesCoef(op0) || usesCoef(op1)) && a.kE) ? a.kE[e] : 1.0;
-  // the coefficient of a single stiffness (mass) operator is folded into its values
-  bool const foldK = k0 != k1, foldM = m0 != m1;
-  double const ks0 = k0 ? (op0.stiff == 2 ? op0.sc * kfac : op0.sc) : 0.;
-  double const ks1 = k1 ? (op1.stiff == 2 ? op1.sc * kfac : op1.sc) : 0.;
-  double const ms0 = m0 ? massCoef(op0, kfac) : 0., ms1 = m1 ? massCoef(op1, kfac) : 0.;
   int64_t km, mm;
   int ke, me, nd, k, eK, eD;
   {
@@ -276,13 +346,13 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
       ps = z > ps ? z : ps;
     }
     ok = q1x::detShifts(lo, hi, nd, k) && ok;
-    ok = q1x::decompose(foldK ? (k0 ? ks0 : ks1) : 1.0, km, ke) && ok;
-    ok = q1x::decompose(foldM ? (m0 ? ms0 : ms1) : 1.0, mm, me) && ok;
+    // the coefficient of a single stiffness (mass) operator is folded into its values
+    ok = q1x::decompose(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
+    ok = q1x::decompose(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
     ok = ok && abs(ke) < 300 && abs(me) < 300; // every value stays normal
     int const sg = q1x::productShift(ps);
     eD = q1x::detExponent(sc, s, nd);
-    eK = q1x::tensorExponent(sc, s, nd, k, sg) + ke - 61;
-    det = q1x::shl(det, nd);
+    eK = q1x::tensorExponent(sc, scMin, s, k, sg) + ke - 61;
     if (needK)
     {
       q1x::pointInverse(det, k, sg, q1x::split(km), s, G);
@@ -290,25 +360,47 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
       for (int c = 0; c < 6; ++c)
         sh.G[c * 8 + w][l] = G[c];
     }
+    det = q1x::shl(det, nd);
   }
-  if (sine)
+  if (series)
   {
+    Sp const u0 = q1x::split(u[0]), u1 = q1x::split(u[1]), u2 = q1x::split(u[2]);
     int64_t f0 = sh.coef[0][deg][l], f1 = sh.coef[1][deg][l], f2 = sh.coef[2][deg][l];
     for (int i = deg - 1; i >= 0; --i)
     {
-      f0 = q1x::mulAdd(q1x::split(f0), u[0], sh.coef[0][i][l]);
-      f1 = q1x::mulAdd(q1x::split(f1), u[1], sh.coef[1][i][l]);
-      f2 = q1x::mulAdd(q1x::split(f2), u[2], sh.coef[2][i][l]);
+      f0 = q1x::mulAdd(q1x::split(f0), u0, sh.coef[0][i][l]);
+      f1 = q1x::mulAdd(q1x::split(f1), u1, sh.coef[1][i][l]);
+      f2 = q1x::mulAdd(q1x::split(f2), u2, sh.coef[2][i][l]);
     }
-    sh.rq[w][l] = q1x::pointLoad(q1x::shl(f0, sh.nf[0][l]), q1x::shl(f1, sh.nf[1][l]), q1x::shl(f2, sh.nf[2][l]), det);
+    int const n0 = q1x::seriesShift(sh.ee[0][l], sh.se[0][l], sh.bound[0][l]),
+              n1 = q1x::seriesShift(sh.ee[1][l], sh.se[2][l], sh.bound[1][l]),
+              n2 = q1x::seriesShift(sh.ee[2][l], sh.se[4][l], sh.bound[2][l]);
+    sh.rq[w][l] = q1x::pointLoad(q1x::shl(f0, n0), q1x::shl(f1, n1), q1x::shl(f2, n2), det);
+    if (w == 7)
+      sh.el[l] = sh.ee[0][l] + sh.ee[1][l] + sh.ee[2][l] - (n0 + n1 + n2);
   }
-  else if (a.rkind)
+  else if (a.rkind == 1 && !analytic)
     sh.rq[w][l] = det >> 2;
+  else if (a.rkind && ok)
+  {
+    double f;
+    if (a.rkind == 1)
+    {
+      // u = J xi / g at F = 61
+      double x[3];
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+        x[r] = fma(q1f::g, q1x::toDouble(u[r], sc[r] - 61), sh.org[r][l]);
+      f = evalPoint(a.fn, x[0], x[1], x[2]);
+    }
+    else
+      f = fieldPoint(a.field, sh, l, w);
+    sh.rqd[w][l] = a.rc * (q1x::toDouble(det, eD - 60) * f);
+  }
   __syncthreads();
   pdlWait(); // the writes start below
 
   // ---- 2. tables; load vector (buildLhs' BC values and buildRhs)
-  bool const bcOps = (op0.on && op0.bc) || (op1.on && op1.bc);
   if (w < 3)
   {
     if (needK)
@@ -351,7 +443,7 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
       q1x::massTable(v, M);
 #pragma unroll
       for (int i = 0; i < 27; ++i)
-        sh.mval[l][i] = q1x::toDouble(M[i / 9][(i / 3) % 3][i % 3], eD + me - 61);
+        sh.mtab[l][i] = M[i / 9][(i / 3) % 3][i % 3];
     }
   }
   else
@@ -363,22 +455,45 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
 #pragma unroll
       for (int n = 0; n < 8; ++n)
         dof[n] = sh.dof[n][l];
-      if (a.b && cons && bcOps)
+      if (a.b && cons && a.fold.bc)
         q1f::addBcValues(a, dof, cons);
       if (a.rkind)
       {
-        int64_t r[8];
+        double fe[8];
+        if (series || (a.rkind == 1 && !analytic))
+        {
+          int64_t r[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q)
-          r[q] = sh.rq[q][l];
-        int const el = sine ? eD + sh.ee[0][l] + sh.ee[1][l] + sh.ee[2][l] - 60 : eD - 59;
-        q1x::nodeSums(r);
+          for (int q = 0; q < 8; ++q)
+            r[q] = sh.rq[q][l];
+          int const el = sine ? eD + sh.el[l] - 60 : eD - 59;
+          q1x::nodeSums(r);
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            fe[q] = a.rc * q1x::toDouble(r[q], el);
+        }
+        else
+        {
+          // sum_q r_q l l l, one axis at a time
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            fe[q] = sh.rqd[q][l];
+#pragma unroll
+          for (int t = 1; t < 8; t *= 2)
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+              if (!(q & t))
+              {
+                double const v0 = fe[q], v1 = fe[q | t];
+                fe[q] = fma(q1f::A, v0, q1f::B * v1), fe[q | t] = fma(q1f::B, v0, q1f::A * v1);
+              }
+        }
 #pragma unroll
         for (int q = 0; q < 8; ++q)
         {
           int const n = q1f::node(q & 1, (q >> 1) & 1, q >> 2);
           if (!(a.rbc && ((cons >> n) & 1u)))
-            atomicAdd(a.b + dof[n], a.rc * q1x::toDouble(r[q], el));
+            atomicAdd(a.b + dof[n], fe[q]);
         }
       }
     }
@@ -386,7 +501,26 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
   }
   __syncthreads();
 
-  // ---- 3. entries
+  // ---- 3. entries; the scatter's ranks are fetched ahead of them
+  int kx[2], mx[2];
+  uint16_t rank[8];
+  if (a.fold.simple)
+  {
+    // (row, column) of the lane in its element's 8 x 8 ranks: 32 (t & 1) + l
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+    {
+      int64_t const i = blockIdx.x * 32ll + 4 * w + (t >> 1);
+      rank[t] = a.rank[elemOf(a, i < a.nelem ? i : a.nelem - 1) * 64 + 32 * (t & 1) + l];
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+  {
+    int const li = latticeOf(4 * h + (l >> 3)), lj = latticeOf(l & 7), q = li ^ lj;
+    kx[h] = entryIndex(li, lj);
+    mx[h] = ((q & 1) ? 2 : (li & 1)) * 9 + ((q & 2) ? 2 : ((li >> 1) & 1)) * 3 + ((q & 4) ? 2 : (li >> 2));
+  }
   if (needK)
   {
     switch (w)
@@ -418,80 +552,48 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
       entriesOut<3, 3>(sh, l, eK);
     }
   }
+  if (needM)
+    for (int i = w; i < 27; i += 8)
+      sh.mval[l][i] = q1x::toDouble(sh.mtab[l][i], eD + me - 61);
   __syncthreads();
 
   // ---- 4. scatter: lane = (row i, column j) of four rows, warp w the elements 4w..4w+3
   if (needK || needM)
   {
-    int const j = l & 7;
-    int kx[2], mx[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
+    if (a.fold.simple)
     {
-      int const li = latticeOf(4 * h + (l >> 3)), lj = latticeOf(j), q = li ^ lj;
-      kx[h] = entryIndex(li, lj);
-      mx[h] = ((q & 1) ? 2 : (li & 1)) * 9 + ((q & 2) ? 2 : ((li >> 1) & 1)) * 3 + ((q & 4) ? 2 : (li >> 2));
-    }
-    // the usual pair: one operator's stiffness, the other's mass
-    bool const pair = foldK && foldM && ((k0 && !m0 && m1 && !k1) || (k1 && !m1 && m0 && !k0));
 #pragma unroll
-    for (int t = 0; t < 4; ++t)
-    {
-      int const el = 4 * w + t;
-      uint32_t const fl = sh.flags[el];
-      if ((fl & 0x300u) != 0x300u)
-        continue;
-      int64_t const ee = elemOf(a, blockIdx.x * 32ll + el);
-      uint32_t const cons = fl & 0xffu;
-      bool const anyBc = cons && bcOps;
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
+      for (int t = 0; t < 8; ++t)
       {
-        int const i = 4 * h + (l >> 3);
-        int32_t const pij = sh.rp[i][el] + a.rank[ee * 64 + i * 8 + j];
-        double const kv = needK ? sh.kval[el][kx[h]] : 0., mv = needM ? sh.mval[el][mx[h]] : 0.;
-        if (pair && !anyBc)
-        {
-          atomicAdd((k0 ? op0.vals : op1.vals) + pij, kv);
-          atomicAdd((k0 ? op1.vals : op0.vals) + pij, mv);
+        int const el = 4 * w + (t >> 1), i = 4 * (t & 1) + (l >> 3);
+        uint32_t const fl = sh.flags[el];
+        if ((fl & 0x300u) != 0x300u)
           continue;
-        }
-        double kf = 1., mf = 1., kg = 1., mg = 1.; // coefficients of op0 and op1 not folded
-        if (!foldK || !foldM)
+        int32_t const pij = sh.rp[el][i] + rank[t];
+        double kv = sh.kval[el][kx[t & 1]], mv = sh.mval[el][mx[t & 1]];
+        if (a.fold.same)
+          kv += mv;
+        bool addK = needK, addM = needM && !a.fold.same;
+        if (a.fold.bc && (fl & 0xffu))
         {
-          double const kfe = ((usesCoef(op0) || usesCoef(op1)) && a.kE) ? a.kE[ee] : 1.0;
-          if (!foldK)
-            kf = op0.stiff == 2 ? op0.sc * kfe : op0.sc, kg = op1.stiff == 2 ? op1.sc * kfe : op1.sc;
-          if (!foldM)
-            mf = massCoef(op0, kfe), mg = massCoef(op1, kfe);
+          bool const ci = (fl >> i) & 1u, cj = (fl >> (l & 7)) & 1u, c = ci || cj;
+          condense(a, sh, el, i, l & 7, c && addK && a.fold.bcK, c && addM && a.fold.bcM, ci, pij, kv, mv);
+          addK = addK && !(c && a.fold.bcK), addM = addM && !(c && a.fold.bcM);
         }
-        bool const ci = (cons >> i) & 1u, cj = (cons >> j) & 1u;
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-        {
-          LhsDev const & op = a.op[m];
-          if (!op.on)
-            continue;
-          double const ksm = m ? kg : kf, msm = m ? mg : mf;
-          double val = op.stiff ? ksm * kv : msm * mv;
-          if (op.stiff && op.mass)
-            val = fma(msm, mv, val);
-          if (anyBc && op.bc && (ci || cj))
-          {
-            // condensation (builder.hpp:76-124): the diagonal of a constrained DOF, the
-            // lift -K_ij h_j of a free row
-            if (i == j)
-              atomicAdd(op.vals + pij, a.bcDiag);
-            else if (!ci && a.b)
-            {
-              double const z = val * a.bcVal[sh.dof[j][el]];
-              if (z != 0.)
-                atomicAdd(a.b + sh.dof[i][el], -z);
-            }
-            continue;
-          }
-          atomicAdd(op.vals + pij, val);
-        }
+        if (addK)
+          atomicAdd(a.fold.K + pij, kv);
+        if (addM)
+          atomicAdd(a.fold.M + pij, mv);
+      }
+    }
+    else
+    {
+#pragma unroll 1
+      for (int t = 0; t < 8; ++t)
+      {
+        int const el = 4 * w + (t >> 1);
+        if ((sh.flags[el] & 0x300u) == 0x300u)
+          scatterGeneral(a, sh, el, 4 * (t & 1) + (l >> 3), l & 7, kx[t & 1], mx[t & 1]);
       }
     }
   }
@@ -499,13 +601,17 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
     elementF64Rare(a, e);
 }
 
-void launchAssembleQ1Fx(AsmArgs const & a, cudaStream_t s, int threads)
+void launchAssembleQ1F64(AsmArgs const & args, cudaStream_t s, int threads)
 {
+  if (args.nelem <= 0)
+    return;
+  AsmArgs a = args;
+  foldOps(a);
   unsigned const blocks = (unsigned)((a.nelem + 31) / 32);
   if (threads == 64)
-    launchElemKernel(kAssembleQ1Fx<4>, blocks, 256, 0, s, a);
-  else
     launchElemKernel(kAssembleQ1Fx<3>, blocks, 256, 0, s, a);
+  else
+    launchElemKernel(kAssembleQ1Fx<4>, blocks, 256, 0, s, a);
 }
 
 } // namespace pxg

@@ -7,14 +7,17 @@
 // sums and differences of the points' values, as additions cost little and products much.
 // Compiles for the host too, where its accuracy is tested.
 //
-// Magnitudes.  Coordinates are differences to vertex 0 in units of 2^sc, the power of
-// two above the largest; the Jacobian columns (half edges) are shifted left by n_a until
-// a bound of their 1-norm over the points is in [1/2, 1), so that cofactors, their
-// products and the determinants all stay below one.  |det| is shifted to a largest value
-// in [1/2, 1) again, 1 / |det| to at most one.  Refused are elements whose columns need
-// more than 6 bits (aspect ratios beyond about 1:16), whose determinant is below 2^-7 of
-// that scale, or varies by more than 2^5 between the points: there the format could carry
-// fewer significant bits than FP64.
+// Magnitudes.  Each coordinate is taken as differences to vertex 0 in units of a power of
+// two above the largest (one unit for the three where they differ by at most 4: only
+// elements flat along an axis need more), so that a thin extent keeps its bits; in these
+// units the Jacobian columns (half edges) are shifted left by n_a until a bound of their
+// 1-norm over the points is in [1/2, 1), and cofactors, their products and the
+// determinants all stay below one.  The determinants' reciprocals and the products are
+// normalised once more, per point and per element.  A rounding of 2^-60 of the largest
+// value thus stands where the FP64 form has one of 2^-53, at every step; the smaller
+// values lose the same bits in both.  Refused are non-finite coordinates and coefficients,
+// zeros, elements whose determinant is below 2^-28 of their edges' product at some point,
+// and sizes whose exponents the results could not hold.
 #pragma once
 
 #include "pxg_fx.h"
@@ -102,20 +105,22 @@ PXG_HD void expand2(int64_t & v0, int64_t & v1, int64_t & v2, int64_t & v3)
   pairExpand(v0, v2), pairExpand(v1, v3);
 }
 PXG_HD int64_t shl(int64_t x, int k) { return (int64_t)((uint64_t)x << k); }
+PXG_HD uint32_t shr32(uint32_t x, int k) { return k < 32 ? x >> k : 0u; }
+PXG_HD int64_t join(Sp x) { return shl((int64_t)x.h, 32) + x.l; }
 
 // ------------------------------------------------------------------- geometry
 // Columns of one coordinate r from its eight vertex values' differences to vertex 0 (d,
-// index bits x, y, z; d[0] = 0) in units of 2^sc: col[a][p] at F = 62 for the column a at
+// index bits x, y, z; d[0] = 0) in units of 2^sc: col[a][p] at F = 60 for the column a at
 // the points p = (qy, qz), (qx, qz), (qx, qy) (first bit lowest), and their largest high
-// words per column.
-PXG_HD void coordColumns(double const (&d)[8], int sc, int64_t (&col)[3][4], uint32_t (&cmax)[3])
+// words per column; and the points' offsets J xi / g, their signed sums, at F = 61.
+PXG_HD void coordColumns(double const (&d)[8], int sc, int64_t (&col)[3][4], uint32_t (&cmax)[3], int64_t (&off)[8])
 {
   int64_t H[8];
   H[0] = 0;
 #pragma unroll
   for (int v = 1; v < 8; ++v)
-    H[v] = roundToInt(scaleExp(d[v], 59 - sc));
-  // the Walsh-Hadamard transform, at most 7 2^59, is eight times the mean: F = 62
+    H[v] = roundToInt(scaleExp(d[v], 57 - sc));
+  // the Walsh-Hadamard transform, at most 7 2^57, is eight times the mean: F = 60
   moments(H);
   int64_t const a110 = 2 * mulc(kB, H[3]), a101 = 2 * mulc(kB, H[5]), a011 = 2 * mulc(kB, H[6]),
                 a111 = mulc(kGG, H[7]);
@@ -128,6 +133,14 @@ PXG_HD void coordColumns(double const (&d)[8], int sc, int64_t (&col)[3][4], uin
     col[0][p] = u1 - w1, col[0][p + 2] = u1 + w1; // (qy = p, qz)
     col[1][p] = u2 - w2, col[1][p + 2] = u2 + w2; // (qx = p, qz)
     col[2][p] = u3 - w2, col[2][p + 2] = u3 + w2; // (qx = p, qy)
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+  {
+    int64_t const x = col[0][q >> 1], y = col[1][(q & 1) + 2 * (q >> 2)], z = col[2][q & 3];
+    int64_t t = (q & 4) ? z : -z;
+    t = (q & 2) ? t + y : t - y;
+    off[q] = 2 * ((q & 1) ? t + x : t - x);
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -143,12 +156,24 @@ PXG_HD void coordColumns(double const (&d)[8], int sc, int64_t (&col)[3][4], uin
     cmax[a] = m;
   }
 }
-// exponent of the largest difference: sc, and whether the format takes it (finite, and
-// the conversions' exponents in range)
-PXG_HD int coordScale(int32_t maxHi) { return (maxHi >> 20) - 1022; }
-PXG_HD bool coordScaleOk(int sc) { return sc >= -300 && sc <= 59; }
+// exponents sc[r] of the units from the largest differences' high words; false where the
+// format does not take them (non-finite, or the conversions' exponents out of range)
+PXG_HD bool coordScales(int32_t m0, int32_t m1, int32_t m2, int (&sc)[3])
+{
+  sc[0] = (m0 >> 20) - 1022, sc[1] = (m1 >> 20) - 1022, sc[2] = (m2 >> 20) - 1022;
+  int const t = sc[0] > sc[1] ? sc[0] : sc[1], hi = t > sc[2] ? t : sc[2];
+  int lo = hi;
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+  {
+    sc[r] = sc[r] >= hi - 2 ? hi : sc[r];
+    lo = sc[r] < lo ? sc[r] : lo;
+  }
+  return lo >= -300 && hi <= 59;
+}
 
-// Column shifts from the largest high words cmax[a * 3 + r]
+// Column shifts from the largest high words cmax[a * 3 + r]: the columns at F = 62 are then
+// the half edges times 2^(n - 2) in units of 2^sc[r]
 struct Shifts
 {
   int n[3], nmin, nmax;
@@ -160,7 +185,7 @@ PXG_HD bool columnShifts(uint32_t const (&cmax)[9], Shifts & s)
   for (int a = 0; a < 3; ++a)
   {
     s.n[a] = clz32(cmax[3 * a] + cmax[3 * a + 1] + cmax[3 * a + 2]) - 2;
-    ok = ok && s.n[a] >= 0 && s.n[a] <= 6;
+    ok = ok && s.n[a] >= 0 && s.n[a] <= 40;
   }
   s.nmax = s.n[0] > s.n[1] ? s.n[0] : s.n[1];
   s.nmax = s.nmax > s.n[2] ? s.nmax : s.n[2];
@@ -170,8 +195,10 @@ PXG_HD bool columnShifts(uint32_t const (&cmax)[9], Shifts & s)
 }
 
 // One point: the cofactors A, B, C of its shifted columns a, b, d, |det| and the products
-// xx yy zz xy xz yz, all at F = 60
-PXG_HD int64_t pointProducts(Sp const (&a)[3], Sp const (&b)[3], Sp const (&d)[3], int64_t (&G)[6])
+// xx yy zz xy xz yz, all at F = 60; w[r]: the bits by which coordinate r's unit exceeds
+// the smallest one (flat: some are not zero)
+PXG_HD int64_t pointProducts(Sp const (&a)[3], Sp const (&b)[3], Sp const (&d)[3], bool flat, int const (&w)[3],
+                             int64_t (&G)[6])
 {
   Sp A[3], B[3], C[3];
 #pragma unroll
@@ -183,51 +210,63 @@ PXG_HD int64_t pointProducts(Sp const (&a)[3], Sp const (&b)[3], Sp const (&d)[3
     C[r] = split(shl(dot2(a[s], b[t], a[t], neg(b[s])), 2));
   }
   int64_t const v = dot3(a, A);
+  if (flat)
+  {
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+    {
+      int const k = w[r] < 63 ? w[r] : 63;
+      A[r] = split(join(A[r]) >> k), B[r] = split(join(B[r]) >> k), C[r] = split(join(C[r]) >> k);
+    }
+  }
   G[0] = dot3(A, A), G[1] = dot3(B, B), G[2] = dot3(C, C);
   G[3] = dot3(A, B), G[4] = dot3(A, C), G[5] = dot3(B, C);
   return v < 0 ? -v : v;
 }
 
-// Shifts of the determinants from the high words of |det| at the eight points: nd to the
-// left (the largest in [1/2, 1) at F = 60), then 2^-k for the inverses (at most one)
+// Shifts from the high words of |det| at the eight points, the smallest lo and the largest
+// hi: nd and k take the largest and the smallest to [1/2, 1) at F = 60
 PXG_HD bool detShifts(uint32_t lo, uint32_t hi, int & nd, int & k)
 {
-  nd = clz32(hi) - 4;
-  bool const ok = nd >= 0 && nd <= 6 && (lo << (nd & 7)) > (1u << 22);
-  k = clz32(lo) - 4 - nd + 1; // lo 2^nd >= 2^(28 - k)
-  return ok;
+  nd = clz32(hi) - 4, k = clz32(lo) - 4;
+  return lo != 0 && nd >= 0;
 }
 // The largest diagonal product of a point, aligned to the common exponent (high word),
 // and the shift to the left its maximum over the points leaves
 PXG_HD uint32_t productSize(int64_t const (&G)[6], Shifts const & s)
 {
-  uint32_t const a = (uint32_t)hi32(G[0]) >> (2 * (s.nmax - s.n[0])), b = (uint32_t)hi32(G[1]) >> (2 * (s.nmax - s.n[1])),
-                 c = (uint32_t)hi32(G[2]) >> (2 * (s.nmax - s.n[2]));
+  uint32_t const a = shr32((uint32_t)hi32(G[0]), 2 * (s.nmax - s.n[0])),
+                 b = shr32((uint32_t)hi32(G[1]), 2 * (s.nmax - s.n[1])),
+                 c = shr32((uint32_t)hi32(G[2]), 2 * (s.nmax - s.n[2]));
   uint32_t const m = a > b ? a : b;
   return m > c ? m : c;
 }
 PXG_HD int productShift(uint32_t size)
 {
   int const k = clz32(size) - 4;
-  return k < 0 ? 0 : (k > 12 ? 12 : k);
+  return k < 0 ? 0 : k;
 }
 // exponents: det = det' 2^-60 2^eD (after the shift nd), G = G' 2^-58 2^eG
-PXG_HD int detExponent(int sc, Shifts const & s, int nd) { return 3 * sc - (s.n[0] + s.n[1] + s.n[2]) - nd; }
-PXG_HD int tensorExponent(int sc, Shifts const & s, int nd, int k, int sg)
+PXG_HD int detExponent(int const (&sc)[3], Shifts const & s, int nd)
 {
-  return k + nd + sc - (s.n[0] + s.n[1] + s.n[2]) + 2 * s.nmax - sg;
+  return sc[0] + sc[1] + sc[2] + 6 - (s.n[0] + s.n[1] + s.n[2]) - nd;
 }
-// G = km |J| (J^T J)^-1 at one point (F = 58) from its products and shifted det: times
-// 2^-k km / |det|, the components aligned to one exponent
+PXG_HD int tensorExponent(int const (&sc)[3], int scMin, Shifts const & s, int k, int sg)
+{
+  return k + 3 + sc[0] + sc[1] + sc[2] - 2 * scMin - (s.n[0] + s.n[1] + s.n[2]) + 2 * s.nmax - sg;
+}
+// G = km |J| (J^T J)^-1 at one point (F = 58) from its products and unshifted |det|: times
+// 2^-(k+1) km / |det|, the components aligned to one exponent
 PXG_HD void pointInverse(int64_t det, int k, int sg, Sp km, Shifts const & s, int64_t (&G)[6])
 {
-  Sp const y = split(shl(mul(split(shl(recip(det), 6 - k)), km), 2));
+  int const n = clz32((uint32_t)hi32(det)) - 4;
+  Sp const y = split(shl(mul(split(shl(recip(shl(det, n)), 5) >> (k - n)), km), 2));
 #pragma unroll
   for (int c = 0; c < 6; ++c)
   {
     int const a = c < 3 ? c : (c == 5 ? 1 : 0), b = c < 3 ? c : (c == 3 ? 1 : 2);
     int const t = sg - (2 * s.nmax - s.n[a] - s.n[b]);
-    G[c] = mul(split(shl(G[c], t > 0 ? t : 0)), y) >> (t > 0 ? 0 : -t);
+    G[c] = mul(split(shl(G[c], t > 0 ? t : 0)), y) >> (t > 0 ? 0 : (t > -63 ? -t : 63));
   }
 }
 
@@ -356,18 +395,20 @@ PXG_HD void massTable(int64_t (&v)[8], int64_t (&M)[3][3][3])
 }
 
 // ------------------------------------------------------------------ sine load
-// sin(pi (o + d)) at the points, d = J xi: with u = the signed column sums at F = 63 of
-// their quarter, pi d = 4 pi g 2^p u, and the Taylor series about o in u, Horner from
-// the top.  A step multiplies by u at F = 63 and so loses one bit: coefficient k is kept
-// at F = 62 + k, scaled by 2^-e so that it holds for p <= -3.
+// sin(pi (o + d)) at the points, d = J xi: with u the signed column sums at F = 63 of
+// their quarter (coordColumns), pi d = 4 pi g 2^sc u, and the Taylor series about o in u,
+// Horner from the top.  A step multiplies by u at F = 63 and so loses one bit:
+// coefficient k is kept at F = 62 + k, scaled by 2^-e so that it holds for sc <= -2.
 struct SerC
 {
-  Cst m; // (4 pi g)^k / k! = m 2^j
+  Cst m; // (4 pi g)^k / k! = m 2^j, k = 1..15
   int j;
 };
-PXG_HD constexpr SerC serC(int k)
-{
-  constexpr SerC t[15] = {
+#ifdef __CUDACC__
+__constant__
+#endif
+  SerC const kSeries[16] = {
+      {cst(0), 0}, // coefficient 0 is S itself
       {cst(0x3a0aa4f6dc87a652ll), 5},
       {cst(0x34a34cc4a60faa41ll), 7},
       {cst(0x3fa653af99556461ll), 8},
@@ -383,61 +424,58 @@ PXG_HD constexpr SerC serC(int k)
       {cst(0x31911161a51cebd5ll), 7},
       {cst(0x335faba26fce95fall), 6},
       {cst(0x31b2653d29e4b398ll), 5},
-  };
-  return t[k - 1];
-}
-constexpr int kLoadMaxP = -3;       // largest p
-constexpr float kLoadMaxT = 0.5f;   // largest |pi d| of degree 15 (0.07: 9, 0.0205: 7): truncation below 8e-19
-// a bound of |pi d| for the coordinate r
-PXG_HD float offsetBound(uint32_t const (&cmax)[9], int r, int sc)
+};
+constexpr int kLoadMaxScale = -2;   // largest sc
+constexpr float kLoadMaxT = 0.5f; // largest |pi d|
+// a bound of |pi d| for one coordinate from its columns' largest high words (zero for
+// elements below 2^-90, where it does not matter)
+PXG_HD float offsetBound(uint32_t const (&cmax)[3], int sc)
 {
-  // pi g 2^(sc - 30) sum_a cmax: the scale as a float's exponent (sc >= -300: below the
-  // smallest float it is zero)
-  float const f = (float)(cmax[r] + cmax[3 + r] + cmax[6 + r]) * (1.8138f / 1073741824.f);
+  // pi g 2^(sc - 28) sum_a cmax
+  float const f = (float)(cmax[0] + cmax[1] + cmax[2] + 1u) * (1.8138f / 268435456.f);
+  if (sc < -90)
+    return 0.f;
 #ifdef __CUDA_ARCH__
-  return ldexpf(f, sc);
+  return __int_as_float(__float_as_int(f) + (sc << 23));
 #else
   return __builtin_ldexpf(f, sc);
 #endif
 }
-// Series of one coordinate from S, C = sin, cos of pi o: the coefficients k[0..DEG] and
-// the shift nf that normalises the sum; returns e with sin = sum 2^-62 2^e after it
-template <int DEG>
-PXG_HD int seriesCoefs(double S, double C, int p, float bound, int64_t (&k)[DEG + 1], int & nf)
+// mantissa (F = 62, signed) and exponent (at most 0) of a sine or cosine; zero: 0, -400
+PXG_HD void sineParts(double x, int64_t & m, int & e)
 {
-  int es = expoField(S) - 1022;
-  es = es < -400 ? -400 : es;
+  if (!decompose(x, m, e))
+    m = 0, e = -400;
+  if (e > 0) // +-1
+    m *= 2, e = 0;
+  e = e < -400 ? -400 : e;
+}
+// exponent of the coefficients of a series about o with sin(pi o) = m 2^es
+PXG_HD int seriesExponent(int es, int sc)
+{
+  int const k = sc + (sc == -2 ? 6 : 5); // 2 (4 pi g 2^sc)^i / i! 2^-e below 0.72 for every i
+  return 1 + (es > k ? es : k);
+}
+// the shift that normalises the series' sum: sin = sum 2^-62 2^(e - shift) after it
+PXG_HD int seriesShift(int e, int es, float bound)
+{
 #ifdef __CUDA_ARCH__
   int const et = (__float_as_int(bound) >> 23) - 126; // bound < 2^et
 #else
   int const et = bound > 0.f ? __builtin_ilogbf(bound) + 1 : -126;
 #endif
-  int const e = 1 + (es > p + 5 ? es : p + 5), en = 1 + (es > et ? es : et);
-  nf = e > en ? e - en : 0;
-  nf = nf < 40 ? nf : 40;
-  int64_t const s = roundToInt(scaleExp(S, 62)), c = roundToInt(scaleExp(C, 62));
-  k[0] = es <= -400 ? 0 : roundToInt(scaleExp(S, 62 - e));
-#pragma unroll
-  for (int i = 1; i <= DEG; ++i)
-  {
-    int const sr = e - serC(i).j - i * (p + 1);
-    int64_t const v = mulc(serC(i).m, (i & 1) ? c : s) >> (sr < 63 ? sr : 63);
-    k[i] = (i & 2) ? -v : v;
-  }
-  return e - nf;
+  int const n = e - 1 - (es > et ? es : et);
+  return n < 0 ? 0 : (n > 40 ? 40 : n);
 }
-// the offset of one point and coordinate: the signed sum of its shifted columns, F = 63
-// of its quarter
-PXG_HD Sp pointOffset(Sp a, Sp b, Sp d, int q, Shifts const & s)
+// coefficient i at F = 62 + i; m 2^em = S (i even) or C (odd)
+PXG_HD int64_t seriesCoef(int e, int sc, int i, int64_t m, int em)
 {
-  int64_t const x = (shl((int64_t)a.h, 32) + a.l) >> (s.n[0] - s.nmin + 1);
-  int64_t const y = (shl((int64_t)b.h, 32) + b.l) >> (s.n[1] - s.nmin + 1);
-  int64_t const z = (shl((int64_t)d.h, 32) + d.l) >> (s.n[2] - s.nmin + 1);
-  int64_t t = (q & 4) ? z : -z;
-  t = (q & 2) ? t + y : t - y;
-  t = (q & 1) ? t + x : t - x;
-  return split(t);
+  int const sr = e - em - kSeries[i].j - i * (sc + 1);
+  int64_t const v = (i ? mulc(kSeries[i].m, m) : m) >> (sr < 63 ? sr : 63);
+  return (i & 2) ? -v : v;
 }
+// degree for a bound of |pi d|: truncation below 8e-19
+PXG_HD int seriesDegree(float bound) { return bound <= 0.0205f ? 7 : (bound <= 0.07f ? 9 : 15); }
 // |det| sin sin sin from the three normalised values: F = 59
 PXG_HD int64_t pointLoad(int64_t f0, int64_t f1, int64_t f2, int64_t det)
 {
