@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
 #pragma unroll
         for (int r = 0; r < 3; ++r)
           sh.coef[r][i][l] =
-              q1x::seriesCoef(sh.ee[r][l], sc[r], i, sh.sm[2 * r + (i & 1)][l], sh.se[2 * r + (i & 1)][l]);
+              q1x::seriesCoef(q1x::kSeries[i], sh.ee[r][l], sc[r], i, sh.sm[2 * r + (i & 1)][l], sh.se[2 * r + (i & 1)][l]);
     }
   }
   int64_t G[6];

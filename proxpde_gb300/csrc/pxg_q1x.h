@@ -450,10 +450,13 @@ PXG_HD void sineParts(double x, int64_t & m, int & e)
     m *= 2, e = 0;
   e = e < -400 ? -400 : e;
 }
-// exponent of the coefficients of a series about o with sin(pi o) = m 2^es
+// exponent of the coefficients of a series about o with sin(pi o) = m 2^es: they stay
+// below 0.72 at F = 62 + i, that is (8 pi t 2^sc)^i / i! 2^-e < 0.72 for every i, t = g
+// (Q2: the larger t of the three-point rule)
+template <bool Q2 = false>
 PXG_HD int seriesExponent(int es, int sc)
 {
-  int const k = sc + (sc == -2 ? 6 : 5); // 2 (4 pi g 2^sc)^i / i! 2^-e below 0.72 for every i
+  int const k = sc + (Q2 ? (sc == -2 ? 8 : (sc == -3 ? 6 : 5)) : (sc == -2 ? 6 : 5));
   return 1 + (es > k ? es : k);
 }
 // the shift that normalises the series' sum: sin = sum 2^-62 2^(e - shift) after it
@@ -467,11 +470,11 @@ PXG_HD int seriesShift(int e, int es, float bound)
   int const n = e - 1 - (es > et ? es : et);
   return n < 0 ? 0 : (n > 40 ? 40 : n);
 }
-// coefficient i at F = 62 + i; m 2^em = S (i even) or C (odd)
-PXG_HD int64_t seriesCoef(int e, int sc, int i, int64_t m, int em)
+// coefficient i at F = 62 + i (t: entry i of the constants); m 2^em = S (i even) or C (odd)
+PXG_HD int64_t seriesCoef(SerC const & t, int e, int sc, int i, int64_t m, int em)
 {
-  int const sr = e - em - kSeries[i].j - i * (sc + 1);
-  int64_t const v = (i ? mulc(kSeries[i].m, m) : m) >> (sr < 63 ? sr : 63);
+  int const sr = e - em - t.j - i * (sc + 1);
+  int64_t const v = (i ? mulc(t.m, m) : m) >> (sr < 63 ? sr : 63);
   return (i & 2) ? -v : v;
 }
 // degree for a bound of |pi d|: truncation below 8e-19

@@ -1,5 +1,6 @@
-// Q2 hexahedron element kernel in FP64 arithmetic with sum factorisation: one warp per
-// element.  It computes what proxpde's element loop computes for a Q2 hexahedron with
+// Q2 hexahedron elements with sum factorisation, in 64-bit fixed point (the kernel, at the
+// end) and, for the few elements that format refuses, in FP64 by one warp.  An element
+// computes what proxpde's element loop computes for a Q2 hexahedron with
 // the 3x3x3 Gauss rule (include/builder.hpp:53-153): CurFE::reinit (include/curfe.hpp:
 // 50-103), AssemblyStiffness(FE) / AssemblyScalarMass / AssemblyMassFE
 // (include/assembly_lhs.hpp:52-109, 207-221, 262-277), AssemblyRhsAnalytic and
@@ -37,6 +38,7 @@
 #include <vector>
 
 #include "pxg_internal.h"
+#include "pxg_q2x.h"
 #include "pxg_sinpi.h"
 
 namespace pxg
@@ -69,6 +71,9 @@ __device__ uint16_t gPairsF[NP];   // (i << 8 | j), i <= j
 // (one padding)
 __device__ uint16_t gPairIdx[NP * 8];
 constexpr int kPairsPerLane = (NP + 31) / 32; // 12
+// for the fixed-point kernel: the pairs (q2x::Pair) and the weights at F = 62, lattice order
+__device__ uint32_t gPairsX[NP];
+__device__ int64_t gWx[NQ];
 
 
 __host__ __device__ constexpr int symCls(int a, int b)
@@ -176,11 +181,11 @@ struct Smem
 };
 } // namespace q2f
 
-__global__ void __launch_bounds__(32) kAssembleQ2F64(AsmArgs a)
+// One element in FP64 by a warp
+__device__ __noinline__ void elementQ2F64(AsmArgs const & a, int64_t e, q2f::Smem & S)
 {
   using namespace q2f;
-  __shared__ Smem S;
-  int const lane = threadIdx.x;
+  int const lane = threadIdx.x & 31;
   for (int k = lane; k < 72; k += 32)
     S.coef[k] = gCoef[k], S.coefN[k] = gCoefN[k];
   if (lane < NQ)
@@ -190,7 +195,6 @@ __global__ void __launch_bounds__(32) kAssembleQ2F64(AsmArgs a)
     S.nodeOfLat[lane] = gNodeOfLat[lane];
     S.ruleOfLat[lane] = gRuleOfLat[lane];
   }
-  int64_t const e = elemOf(a, blockIdx.x);
   // ---- inputs
   if (lane < 24)
   {
@@ -292,8 +296,7 @@ __global__ void __launch_bounds__(32) kAssembleQ2F64(AsmArgs a)
   double const * const cL = S.coef;
   double const * const cP = S.coef + 9;
 
-  // ---- load vector (buildLhs' BC values, buildRhs); the writes start here
-  pdlWait();
+  // ---- load vector (buildLhs' BC values, buildRhs)
   bool const bcOps = (op0.on && op0.bc) || (op1.on && op1.bc);
   if (a.b && cons && bcOps && lane < N && ((cons >> lane) & 1u))
   {
@@ -453,6 +456,583 @@ __global__ void __launch_bounds__(32) kAssembleQ2F64(AsmArgs a)
         atomicAdd(op.vals + pji, val);
     }
   }
+}
+
+// ------------------------------------------------------------ the fixed-point kernel
+// A block of four warps computes four elements in 64-bit fixed point (pxg_q2x.h); a thread
+// works for element tid & 3 throughout:
+//  0. coordinates, differences and Walsh-Hadamard transform by groups of eight lanes (one
+//     coordinate of one element), units, shifts, and the sine series of the load;
+//  1. one quadrature point per thread: columns, cofactors, |det|, products, then G and the
+//     weighted determinant, and the load value;
+//  2. the P axis that every table contracts first: 63 lines per element;
+//  3. the two remaining axes of a table for one class of the first, nine values in, 36 out,
+//     in registers: first S_x, S_y, S_z and the mass (while a warp sums the load to the
+//     nodes), then the symmetric and antisymmetric tables of the mixed components; after
+//     each of the two rounds every thread adds its pairs' terms into registers;
+//  4. the scatter: a warp adds the 27 x 27 entries of one element row by row, so that lanes
+//     read consecutive ranks and neighbouring columns share sectors.
+// The FP64 form issues 509 FP64 instructions per element and warp, at 64 cycles each on
+// this part; this one has none but the conversions of the results (26 per element).
+namespace q2f
+{
+constexpr int E = 4;        // elements per block
+constexpr int NT = 32 * E;  // threads per block
+using q1x::Sp;
+
+struct Shared
+{
+  int64_t H[E][3][8]; // H100, H010, H001, tH110, tH101, tH011, ttH111 at F = 60
+  union
+  {
+    int64_t G[7][NQ][E];     // xx yy zz xy xz yz, w |det|
+    int64_t tab[4 * 216][E]; // tables of a round
+    struct
+    {
+      double kd[E][NP + 1], md[E][NP + 1]; // entries
+    };
+  };
+  int64_t s1[7][54][E]; // after the first axis
+  int64_t rq[NQ][E]; // load values (rqd: in FP64)
+  int64_t coef[3][16][E];
+  int64_t sm[6][E];
+  double org[3][E];
+  uint32_t cmax[E][9];
+  int32_t dmax[3][E];
+  int32_t se[6][E], ee[3][E];
+  float bound[3][E];
+  uint32_t lo[E], hi[E], ps[E], cons[E], ok[E];
+  int32_t el[E];
+  uint32_t dof[E][N];
+  int32_t rp[E][N];
+};
+static_assert(sizeof(Smem) * E <= sizeof(Shared), "the refused elements' buffers fit the block's");
+
+// x times s - 1, s in {0, 1, 2}
+__device__ __forceinline__ int64_t times(int64_t x, int s) { return s == 1 ? 0 : (s == 0 ? -x : x); }
+
+// contraction of a plane v[qs][ql] (first axis done) over its two axes
+template <int KIND> // 0: P, D   1: P, P   2: S, S
+__device__ __forceinline__ void plane(int64_t const (*in)[E], int64_t (*out)[E], int el)
+{
+  int64_t m[3][6]; // [ql][cs]
+#pragma unroll
+  for (int l = 0; l < 3; ++l)
+  {
+    if constexpr (KIND == 2)
+      q2x::lineS(in[l][el], in[3 + l][el], in[6 + l][el], m[l]);
+    else
+      q2x::lineP(in[l][el], in[3 + l][el], in[6 + l][el], m[l]);
+  }
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+  {
+    int64_t o[6];
+    if constexpr (KIND == 0)
+      q2x::lineD(m[0][c], m[1][c], m[2][c], o);
+    else if constexpr (KIND == 1)
+      q2x::lineP(m[0][c], m[1][c], m[2][c], o);
+    else
+      q2x::lineS(m[0][c], m[1][c], m[2][c], o);
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      out[c * 6 + k][el] = o[k];
+  }
+}
+__device__ __forceinline__ void planeA(int64_t const (*in)[E], int64_t (*out)[E], int el)
+{
+  int64_t m[3][3];
+#pragma unroll
+  for (int l = 0; l < 3; ++l)
+    q2x::lineA(in[l][el], in[3 + l][el], in[6 + l][el], m[l]);
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+  {
+    int64_t o[3];
+    q2x::lineA(m[0][c], m[1][c], m[2][c], o);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      out[c * 3 + k][el] = o[k];
+  }
+}
+// l_a of three doubles
+__device__ __forceinline__ void lineLd(double v0, double v1, double v2, double (&o)[3])
+{
+  constexpr double t = 0.774596669241483;
+  double const a = 0.5 * t * t * (v0 + v2), b = 0.5 * t * (v2 - v0);
+  o[0] = a - b, o[1] = a + b, o[2] = fma(1. - t * t, v0 + v2, v1);
+}
+
+// the load's value at a point that is not a series or a constant: another function, a DOF
+// field, a large element
+__device__ __noinline__ double pointValue(AsmArgs const & a, Shared const & sh, int el, int q, double x, double y,
+                                          double z)
+{
+  if (a.rkind == 1)
+    return evalFn(a.fn, 1.0, x, y, z);
+  int const qx = q / 9, qy = (q / 3) % 3, qz = q % 3;
+  double s = 0.;
+  for (int n = 0; n < N; ++n)
+  {
+    int const L = gLatOfNode[n];
+    s = fma(gCoef[3 * (L / 9) + qx] * gCoef[3 * ((L / 3) % 3) + qy] * gCoef[3 * (L % 3) + qz],
+            a.field[sh.dof[el][n]], s);
+  }
+  return s;
+}
+
+// entry (i, j) of element el for any operators and with the Dirichlet condensation
+// (builder.hpp:76-124)
+__device__ __noinline__ void scatterGeneral(AsmArgs const & a, Shared const & sh, int el, int64_t e, int i, int j,
+                                            int p, int32_t pij)
+{
+  uint32_t const cons = sh.cons[el];
+  bool const ci = (cons >> i) & 1u, cj = (cons >> j) & 1u;
+  double const kfac = a.fold.coef ? a.kE[e] : 1.0;
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+  {
+    LhsDev const & op = a.op[m];
+    if (!op.on)
+      continue;
+    // a single operator's coefficient is folded into the values
+    double const kf = a.fold.foldK ? 1. : (op.stiff == 2 ? op.sc * kfac : op.sc),
+                 mf = a.fold.foldM ? 1. : massCoef(op, kfac);
+    double val = op.stiff ? kf * sh.kd[el][p] : mf * sh.md[el][p];
+    if (op.stiff && op.mass)
+      val = fma(mf, sh.md[el][p], val);
+    if (!(op.bc && (ci || cj)))
+      atomicAdd(op.vals + pij, val);
+    else if (i == j)
+      atomicAdd(op.vals + pij, a.bcDiag);
+    else if (!ci && a.b)
+    {
+      double const z = val * a.bcVal[sh.dof[el][j]];
+      if (z != 0.)
+        atomicAdd(a.b + sh.dof[el][i], -z);
+    }
+  }
+}
+} // namespace q2f
+
+__global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid_constant__ a)
+{
+  using namespace q2f;
+  __shared__ Shared sh;
+  int const tid = threadIdx.x, w = tid >> 5, l = tid & 31, el = tid & 3, x = tid >> 2;
+  int64_t const i0 = blockIdx.x * (int64_t)E;
+  auto element = [&](int k) { return elemOf(a, i0 + k < a.nelem ? i0 + k : a.nelem - 1); };
+  int64_t const e = element(el);
+  bool const needK = a.fold.needK, needM = a.fold.needM;
+  // loads: sin sin sin by its series, a constant, and anything else point by point in FP64
+  bool const analytic = a.rkind == 1 && a.fn != PXG_FN_CONST, sine = a.rkind == 1 && a.fn == PXG_FN_SIN3;
+  double const kfac = a.fold.coef ? a.kE[e] : 1.0;
+
+  // ---- 0. inputs
+  if (tid < E)
+    sh.lo[tid] = 0xffffffffu, sh.hi[tid] = 0, sh.ps[tid] = 0, sh.cons[tid] = 0;
+  // group of eight lanes g = 3 element + coordinate, lane v = lattice vertex
+  int const g = tid >> 3, v = tid & 7, ge = g / 3, gr = g - 3 * ge;
+  double d = 0.;
+  if (tid < 8 * 3 * E)
+  {
+    // lattice order of the nodes: 0 1 3 2 4 5 7 6
+    int const node = v ^ ((v >> 1) & 1);
+    double const X = a.xyz[3 * (int64_t)a.conn[element(ge) * 8 + node] + gr];
+    d = X - __shfl_sync(0xffffffffu, X, l & 24);
+    int32_t m = q1x::hi32(q1x::doubleBits(d)) & 0x7fffffff;
+    double o = X;
+#pragma unroll
+    for (int t = 1; t < 8; t *= 2)
+    {
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, t));
+      if (analytic)
+        o += __shfl_xor_sync(0xffffffffu, o, t);
+    }
+    if (v == 0)
+      sh.dmax[gr][ge] = m, sh.org[gr][ge] = 0.125 * o; // origin = vertex average (geo.hpp:721-728)
+  }
+  else
+  {
+    for (int k = tid - 8 * 3 * E; k < E * N; k += NT - 8 * 3 * E)
+    {
+      int const ke = k / N, n = k - ke * N;
+      uint32_t const dof = a.emap[element(ke) * N + n];
+      sh.dof[ke][n] = dof;
+      sh.rp[ke][n] = a.rowPtr[dof];
+    }
+  }
+  __syncthreads();
+  int sc[3];
+  bool ok = q1x::coordScales(sh.dmax[0][el], sh.dmax[1][el], sh.dmax[2][el], sc);
+  int const scMin = min(sc[0], min(sc[1], sc[2]));
+  if (tid < 8 * 3 * E)
+  {
+    int gs[3];
+    q1x::coordScales(sh.dmax[0][ge], sh.dmax[1][ge], sh.dmax[2][ge], gs);
+    int const sr = gr == 0 ? gs[0] : (gr == 1 ? gs[1] : gs[2]);
+    int64_t h = q1x::roundToInt(q1x::scaleExp(d, 57 - sr));
+#pragma unroll
+    for (int t = 1; t < 8; t *= 2)
+    {
+      int64_t const o = __shfl_xor_sync(0xffffffffu, h, t);
+      h = (v & t) ? h - o : h + o;
+    }
+    // lane v holds H_v (a set bit: difference), eight times the mean: F = 60.  times t per
+    // axis beyond the first
+    if (v == 3 || v == 5 || v == 6)
+      h = 2 * q1x::mulc(q2x::kTh, h);
+    if (v == 7)
+      h = 2 * q1x::mulc(q2x::kT2h, h);
+    if (v)
+      sh.H[ge][gr][v] = h;
+    // bounds of the columns: sums of their terms
+    uint32_t const z = (uint32_t)abs(q1x::hi32(h)) + 1u;
+    uint32_t const z1 = __shfl_sync(0xffffffffu, z, (l & 24) + 1), z2 = __shfl_sync(0xffffffffu, z, (l & 24) + 2),
+                   z3 = __shfl_sync(0xffffffffu, z, (l & 24) + 3), z4 = __shfl_sync(0xffffffffu, z, (l & 24) + 4),
+                   z5 = __shfl_sync(0xffffffffu, z, (l & 24) + 5), z6 = __shfl_sync(0xffffffffu, z, (l & 24) + 6),
+                   z7 = __shfl_sync(0xffffffffu, z, (l & 24) + 7);
+    if (v == 0)
+    {
+      uint32_t const c[3] = {z1 + z3 + z5 + z7, z2 + z3 + z6 + z7, z4 + z5 + z6 + z7};
+      sh.cmax[ge][gr] = c[0], sh.cmax[ge][3 + gr] = c[1], sh.cmax[ge][6 + gr] = c[2];
+      float const b = q2x::kBoundRatio * q1x::offsetBound(c, sr);
+      // the offsets hold at F = 61 below 4
+      sh.bound[gr][ge] = c[0] + c[1] + c[2] < (1u << 30) ? b : 1e30f;
+      if (sine)
+      {
+        double t[2];
+        sinCosPiTab(sh.org[gr][ge], t[0], t[1]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+        {
+          int64_t mt;
+          int xt;
+          q1x::sineParts(t[i], mt, xt);
+          sh.sm[2 * gr + i][ge] = mt, sh.se[2 * gr + i][ge] = xt;
+          if (i == 0)
+            sh.ee[gr][ge] = q1x::seriesExponent<true>(xt, sr);
+        }
+      }
+    }
+  }
+  else if (a.bcMask)
+  {
+    for (int k = tid - 8 * 3 * E; k < E * N; k += NT - 8 * 3 * E)
+    {
+      int const ke = k / N, n = k - ke * N;
+      if (a.bcMask[sh.dof[ke][n]])
+        atomicOr(&sh.cons[ke], 1u << n);
+    }
+  }
+  __syncthreads();
+
+  // ---- 1. scales, and one point per thread
+  q1x::Shifts s;
+  {
+    uint32_t cm[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+      cm[k] = sh.cmax[el][k];
+    ok = q1x::columnShifts(cm, s) && ok;
+  }
+  bool series = false;
+  int deg = 0;
+  if (sine)
+  {
+    float const bm = fmaxf(sh.bound[0][el], fmaxf(sh.bound[1][el], sh.bound[2][el]));
+    series = ok && max(sc[0], max(sc[1], sc[2])) <= q1x::kLoadMaxScale && bm <= q1x::kLoadMaxT;
+    // one degree for the block (every warp sees its four elements)
+    deg = q1x::seriesDegree(__uint_as_float(__reduce_max_sync(0xffffffffu, series ? __float_as_uint(bm) : 0u)));
+    for (int k = x; k < 3 * (deg + 1); k += 32)
+    {
+      int const r = k / (deg + 1), i = k - r * (deg + 1);
+      sh.coef[r][i][el] = q1x::seriesCoef(q2x::kSeries[i], sh.ee[r][el], r == 0 ? sc[0] : (r == 1 ? sc[1] : sc[2]), i,
+                                          sh.sm[2 * r + (i & 1)][el], sh.se[2 * r + (i & 1)][el]);
+    }
+  }
+  int const q = x < NQ ? x : 0, qx = q / 9, qy = (q / 3) % 3, qz = q % 3;
+  int64_t G[6], det, u[3];
+  {
+    Sp c1[3], c2[3], c3[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+    {
+      int64_t const * const H = sh.H[el][r];
+      int64_t const yz = times(times(H[7], qz), qy), xz = times(times(H[7], qz), qx), xy = times(times(H[7], qy), qx);
+      int64_t const t1 = H[1] + times(H[3], qy) + times(H[5], qz) + yz;
+      int64_t const t2 = H[2] + times(H[3], qx) + times(H[6], qz) + xz;
+      int64_t const t3 = H[4] + times(H[5], qx) + times(H[6], qy) + xy;
+      u[r] = 2 * (times(t1, qx) + times(t2, qy) + times(t3, qz)); // J xi / t at F = 61
+      c1[r] = q1x::splitOdd(q1x::shl(t1, s.n[0]));
+      c2[r] = q1x::splitOdd(q1x::shl(t2, s.n[1]));
+      c3[r] = q1x::splitOdd(q1x::shl(t3, s.n[2]));
+    }
+    int const wt[3] = {sc[0] - scMin, sc[1] - scMin, sc[2] - scMin};
+    det = q1x::pointProducts(c1, c2, c3, __any_sync(0xffffffffu, (wt[0] | wt[1] | wt[2]) != 0) != 0, wt, G);
+    uint32_t lo = (uint32_t)q1x::hi32(det), hi = lo, ps = q1x::productSize(G, s);
+#pragma unroll
+    for (int t = 4; t < 32; t *= 2)
+    {
+      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, t));
+      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, t));
+      ps = max(ps, __shfl_xor_sync(0xffffffffu, ps, t));
+    }
+    if (l < E)
+      atomicMin(&sh.lo[l], lo), atomicMax(&sh.hi[l], hi), atomicMax(&sh.ps[l], ps);
+  }
+  __syncthreads();
+  int64_t km, mm;
+  int ke, me, nd, k;
+  ok = q1x::detShifts(sh.lo[el], sh.hi[el], nd, k) && ok;
+  // the coefficient of a single stiffness (mass) operator is folded into its values
+  ok = q1x::decompose(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
+  ok = q1x::decompose(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
+  ok = ok && abs(ke) < 300 && abs(me) < 300; // every value stays normal
+  int const sg = q1x::productShift(sh.ps[el]);
+  int const eD = q1x::detExponent(sc, s, nd);
+  int const eK = q1x::tensorExponent(sc, scMin, s, k, sg) + ke - 57, eM = eD + me - 60;
+  if (x < NQ)
+  {
+    Sp const wq = q1x::split(gWx[q]);
+    if (needK)
+    {
+      q1x::pointInverse(det, k, sg, q1x::split(q1x::shl(q1x::mul(q1x::split(km), wq), 2)), s, G);
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+        sh.G[c][q][el] = G[c] >> 1; // F = 57: the entries reach 25 times the largest value
+    }
+    int64_t const dw = q1x::mul(q1x::split(q1x::shl(q1x::shl(det, nd), 2)), wq); // F = 60
+    if (needM)
+      sh.G[6][q][el] = q1x::mul(q1x::split(q1x::shl(dw, 2)), q1x::split(mm));
+    if (series)
+    {
+      Sp const u0 = q1x::split(u[0]), u1 = q1x::split(u[1]), u2 = q1x::split(u[2]);
+      int64_t f0 = sh.coef[0][deg][el], f1 = sh.coef[1][deg][el], f2 = sh.coef[2][deg][el];
+      for (int i = deg - 1; i >= 0; --i)
+      {
+        f0 = q1x::mulAdd(q1x::split(f0), u0, sh.coef[0][i][el]);
+        f1 = q1x::mulAdd(q1x::split(f1), u1, sh.coef[1][i][el]);
+        f2 = q1x::mulAdd(q1x::split(f2), u2, sh.coef[2][i][el]);
+      }
+      int const n0 = q1x::seriesShift(sh.ee[0][el], sh.se[0][el], sh.bound[0][el]),
+                n1 = q1x::seriesShift(sh.ee[1][el], sh.se[2][el], sh.bound[1][el]),
+                n2 = q1x::seriesShift(sh.ee[2][el], sh.se[4][el], sh.bound[2][el]);
+      sh.rq[q][el] = q1x::pointLoad(q1x::shl(f0, n0), q1x::shl(f1, n1), q1x::shl(f2, n2), dw);
+      if (q == 0)
+        sh.el[el] = sh.ee[0][el] + sh.ee[1][el] + sh.ee[2][el] - (n0 + n1 + n2);
+    }
+    else if (a.rkind == 1 && !analytic)
+      sh.rq[q][el] = dw >> 1;
+    else if (a.rkind && ok)
+    {
+      double p[3] = {0., 0., 0.};
+      if (a.rkind == 1)
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+          p[r] = fma(0.774596669241483, q1x::toDouble(u[r], sc[r] - 61), sh.org[r][el]);
+      sh.rq[q][el] =
+          __double_as_longlong(a.rc * (q1x::toDouble(dw, eD - 60) * pointValue(a, sh, el, q, p[0], p[1], p[2])));
+    }
+  }
+  if (tid < E)
+    sh.ok[tid] = (ok ? 1u : 0u) | (i0 + tid < a.nelem ? 2u : 0u);
+  __syncthreads();
+
+  // ---- 2. the first axis (stride f; s, l the other two): P
+  // S_x: y, z, x   S_y: x, z, y   S_z, mass: x, y, z   xy: z, x, y   xz: y, x, z   yz: x, y, z
+  for (int k2 = x; k2 < 63; k2 += 32)
+  {
+    int const T = k2 / 9, r = k2 - 9 * T, q1 = r / 3, q2 = r - 3 * q1;
+    if (T == 3 ? !needM : !needK)
+      continue;
+    int const f = (T == 0 || T == 5) ? 3 : (T == 4 ? 1 : 9), st = T <= 1 ? 1 : ((T == 4 || T == 5) ? 9 : 3),
+              lt = T == 0 ? 9 : ((T == 1 || T == 4) ? 3 : 1);
+    int64_t const(*in)[E] = sh.G[T < 3 ? T : (T == 3 ? 6 : T - 1)] + q1 * st + q2 * lt;
+    int64_t o[6];
+    q2x::lineP(in[0][el], in[f][el], in[2 * f][el], o);
+#pragma unroll
+    for (int c = 0; c < 6; ++c)
+      sh.s1[T][c * 9 + r][el] = o[c];
+  }
+  __syncthreads();
+  pdlWait(); // the writes start below
+
+  // ---- 3. the tables S_x, S_y, S_z and mass; the load on the last warp
+  if (x < 24)
+  {
+    int const T = x / 6, c = x - 6 * T;
+    if (T < 3)
+    {
+      if (needK)
+        plane<0>(sh.s1[T] + c * 9, sh.tab + x * 36, el);
+    }
+    else if (needM)
+      plane<1>(sh.s1[3] + c * 9, sh.tab + x * 36, el);
+  }
+  else
+  {
+    // one line per lane pass: nine lines of four elements, three axes in place; the value
+    // index is qx 9 + qy 3 + qz
+    bool const mine = sh.ok[el] == 3u, fixedLoad = series || (a.rkind == 1 && !analytic);
+    int64_t(*rq)[E] = sh.rq;
+    if (a.rkind)
+    {
+#pragma unroll 1
+      for (int ax = 0; ax < 3; ++ax)
+      {
+        int const f = ax == 0 ? 9 : (ax == 1 ? 3 : 1), g1 = ax == 0 ? 3 : 9, g2 = ax == 2 ? 3 : 1;
+        for (int n = x - 24; n < 9; n += 8)
+        {
+          int const o0 = (n / 3) * g1 + (n % 3) * g2;
+          int64_t const v0 = rq[o0][el], v1 = rq[o0 + f][el], v2 = rq[o0 + 2 * f][el];
+          if (fixedLoad)
+          {
+            int64_t o[3];
+            q2x::lineL(v0, v1, v2, o);
+            rq[o0][el] = o[0], rq[o0 + f][el] = o[1], rq[o0 + 2 * f][el] = o[2];
+          }
+          else
+          {
+            double o[3];
+            lineLd(__longlong_as_double(v0), __longlong_as_double(v1), __longlong_as_double(v2), o);
+            rq[o0][el] = __double_as_longlong(o[0]), rq[o0 + f][el] = __double_as_longlong(o[1]),
+            rq[o0 + 2 * f][el] = __double_as_longlong(o[2]);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    if (mine && a.b && (a.rkind || a.fold.bc))
+    {
+      uint32_t const cons = sh.cons[el];
+      int const ex = sine ? eD + sh.el[el] - 59 : eD - 59;
+      for (int L = x - 24; L < N; L += 8)
+      {
+        int const n = gNodeOfLat[L];
+        bool const c = (cons >> n) & 1u;
+        uint32_t const dof = sh.dof[el][n];
+        if (a.rkind && !(a.rbc && c))
+          atomicAdd(a.b + dof,
+                    fixedLoad ? a.rc * q1x::toDouble(rq[L][el], ex) : __longlong_as_double(rq[L][el]));
+        if (c)
+        {
+          // buildLhs' Dirichlet values, once per operator with BCs (builder.hpp:119)
+          double const h = a.bcVal[dof];
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+            if (a.op[m].on && a.op[m].bc && h != 0.)
+              atomicAdd(a.b + dof, h);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  int64_t kv[kPairsPerLane], mv[kPairsPerLane];
+#pragma unroll
+  for (int t = 0; t < kPairsPerLane; ++t)
+  {
+    int const p = x + 32 * t;
+    kv[t] = 0, mv[t] = 0;
+    if (p < NP)
+    {
+      q2x::Pair const pr{gPairsX[p]};
+      int const cx = pr.sym(0), cy = pr.sym(1), cz = pr.sym(2);
+      if (needK)
+        kv[t] = sh.tab[cy * 36 + cz * 6 + cx][el] + sh.tab[216 + cx * 36 + cz * 6 + cy][el] +
+                sh.tab[432 + cx * 36 + cy * 6 + cz][el];
+      if (needM)
+        mv[t] = sh.tab[648 + cx * 36 + cy * 6 + cz][el];
+    }
+  }
+  __syncthreads();
+  // the mixed components: SS at m 216 + lead 36 + s1 6 + s2, AA at 648 + m 54 + lead 9 + a1 3 + a2
+  if (needK)
+  {
+    if (x < 18)
+      plane<2>(sh.s1[4 + x / 6] + (x % 6) * 9, sh.tab + x * 36, el);
+    if (x >= 14)
+    {
+      int const z = x - 14;
+      planeA(sh.s1[4 + z / 6] + (z % 6) * 9, sh.tab + 648 + z * 9, el);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kPairsPerLane; ++t)
+    {
+      int const p = x + 32 * t;
+      if (p < NP)
+      {
+        q2x::Pair const pr{gPairsX[p]};
+        int const cx = pr.sym(0), cy = pr.sym(1), cz = pr.sym(2), ax = pr.anti(0), ay = pr.anti(1), az = pr.anti(2);
+        int64_t z = sh.tab[cz * 36 + cx * 6 + cy][el] + sh.tab[216 + cy * 36 + cx * 6 + cz][el] +
+                    sh.tab[432 + cx * 36 + cy * 6 + cz][el];
+        if (ax != 3 && ay != 3)
+        {
+          int64_t const y = sh.tab[648 + cz * 9 + ax * 3 + ay][el];
+          z = pr.up(0) == pr.up(1) ? z - y : z + y;
+        }
+        if (ax != 3 && az != 3)
+        {
+          int64_t const y = sh.tab[702 + cy * 9 + ax * 3 + az][el];
+          z = pr.up(0) == pr.up(2) ? z - y : z + y;
+        }
+        if (ay != 3 && az != 3)
+        {
+          int64_t const y = sh.tab[756 + cx * 9 + ay * 3 + az][el];
+          z = pr.up(1) == pr.up(2) ? z - y : z + y;
+        }
+        kv[t] += 2 * z;
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int t = 0; t < kPairsPerLane; ++t)
+  {
+    int const p = x + 32 * t;
+    if (p < NP)
+    {
+      if (needK)
+        sh.kd[el][p] = q1x::toDouble(kv[t], eK);
+      if (needM)
+        sh.md[el][p] = q1x::toDouble(mv[t], eM);
+    }
+  }
+  __syncthreads();
+
+  // ---- 4. scatter: warp w adds element w
+  int64_t const ew = element(w);
+  uint32_t const okw = sh.ok[w];
+  if (okw == 3u && (needK || needM))
+  {
+    uint16_t const * const rk = a.rank + ew * (N * N);
+    bool const plain = a.fold.simple && !(a.fold.bc && sh.cons[w]);
+#pragma unroll 6
+    for (int f = l; f < N * N; f += 32)
+    {
+      int const i = f / N, j = f - i * N, lo = min(i, j), hi = max(i, j), p = lo * (53 - lo) / 2 + hi;
+      int32_t const pij = sh.rp[w][i] + rk[f];
+      if (plain)
+      {
+        if (a.fold.same)
+          atomicAdd(a.fold.K + pij, sh.kd[w][p] + sh.md[w][p]);
+        else
+        {
+          if (needK)
+            atomicAdd(a.fold.K + pij, sh.kd[w][p]);
+          if (needM)
+            atomicAdd(a.fold.M + pij, sh.md[w][p]);
+        }
+      }
+      else
+        scatterGeneral(a, sh, w, ew, i, j, p, pij);
+    }
+  }
+  // refused elements, each by its warp in FP64
+  if (__syncthreads_or(okw == 2u))
+    if (okw == 2u)
+      elementQ2F64(a, ew, reinterpret_cast<Smem *>(&sh)[w]);
 }
 
 // The 1D tables, the lattice maps and the pair list, from the reference's rule and
@@ -615,13 +1195,35 @@ pxg_status initQ2F64Tables(pxg_ctx * c)
     o[6] = aaIdx(px, iy, jy, iz, jz);
   }
   PXG_CUDA(c, cudaMemcpyToSymbol(gPairIdx, pidx.data(), pidx.size() * 2));
+  std::vector<uint32_t> px(pairs.size());
+  for (size_t q = 0; q < pairs.size(); ++q)
+  {
+    int const i = pairs[q] >> 8, j = pairs[q] & 0xff;
+    int const L[2] = {latOfNode[i], latOfNode[j]}, div[3] = {9, 3, 1};
+    uint32_t v = (uint32_t)i << 18 | (uint32_t)j << 23;
+    for (int ax = 0; ax < 3; ++ax)
+    {
+      int const p = (L[0] / div[ax]) % 3, r = (L[1] / div[ax]) % 3;
+      v |= (uint32_t)symCls(p, r) << (3 * ax) | (uint32_t)(p == r ? 3 : p + r - 1) << (9 + 2 * ax) |
+           (uint32_t)(p < r) << (15 + ax);
+    }
+    px[q] = v;
+  }
+  PXG_CUDA(c, cudaMemcpyToSymbol(gPairsX, px.data(), px.size() * 4));
+  int64_t wx[NQ];
+  for (int q = 0; q < NQ; ++q)
+    wx[q] = (int64_t)(wl[q] * 4611686018427387904.0); // exact
+  PXG_CUDA(c, cudaMemcpyToSymbol(gWx, wx, sizeof(wx)));
   return PXG_OK;
 }
 
-void launchAssembleQ2F64(AsmArgs const & a, cudaStream_t s)
+void launchAssembleQ2F64(AsmArgs const & args, cudaStream_t s)
 {
-  if (a.nelem > 0)
-    launchElemKernel(kAssembleQ2F64, (unsigned)a.nelem, 32, 0, s, a);
+  if (args.nelem <= 0)
+    return;
+  AsmArgs a = args;
+  foldOps(a);
+  launchElemKernel(kAssembleQ2Fx, (unsigned)((a.nelem + q2f::E - 1) / q2f::E), q2f::NT, 0, s, a);
 }
 
 } // namespace pxg
