@@ -57,8 +57,8 @@ __device__ double gCoefN[72];      // P, D, S, A classes divided by their first 
 // (216) and its AA table (128: index a for a positive orientation, 64 + a for a
 // negative one, 54 for the pairs without an AA term, whose scale is 0)
 constexpr int kAA = 128;
-constexpr int kTab = 3 * 216 + 3 * (216 + kAA);
-__device__ double gScale[kTab];
+constexpr int kScales = 3 * 216 + 3 * (216 + kAA);
+__device__ double gScale[kScales];
 __device__ double gT[3];           // t_k
 __device__ double gWl[NQ];         // weights in lattice order qx * 9 + qy * 3 + qz
 __device__ uint8_t gRuleOfLat[NQ]; // the rule's point index of each lattice point
@@ -71,9 +71,22 @@ __device__ uint16_t gPairsF[NP];   // (i << 8 | j), i <= j
 // (one padding)
 __device__ uint16_t gPairIdx[NP * 8];
 constexpr int kPairsPerLane = (NP + 31) / 32; // 12
-// for the fixed-point kernel: the pairs (q2x::Pair) and the weights at F = 62, lattice order
-__device__ uint32_t gPairsX[NP];
+// for the fixed-point kernel: the weights at F = 62 in lattice order; the places of each
+// pair's terms in the tables of the two rounds (S_x, S_y, S_z, mass; SS and AA of xy, xz,
+// yz, 16 bits each), and of each entry (row, column) its row and pair (i | pair << 8)
 __device__ int64_t gWx[NQ];
+__device__ ushort4 gPairA[NP];
+__device__ uint4 gPairB[NP];
+__device__ uint32_t gEntry[N * N];
+// The tables' rows, one array: 7 x 54 after the first axis, then 4 x 6 x 36 of a round, a
+// plane of 36 every 37 rows (a row is 32 bytes: eight planes written at once at a stride
+// of 36 would share their banks).  In
+// the second round AA and -AA (54 each) of xy and xz take the first-axis rows of the
+// first four tables, those of yz and a zero follow SS.
+constexpr int kPlane = 37, kTab = 7 * 54, kRows = kTab + 24 * kPlane, kZero = kTab + 18 * kPlane + 108;
+__host__ __device__ constexpr int rowAA(int m) { return m < 2 ? 108 * m : kTab + 18 * kPlane; }
+// table T of a round, classes a (of its first axis), b and c
+__host__ __device__ constexpr int rowOf(int T, int a, int b, int c) { return kTab + (T * 6 + a) * kPlane + b * 6 + c; }
 
 
 __host__ __device__ constexpr int symCls(int a, int b)
@@ -485,14 +498,17 @@ struct Shared
   int64_t H[E][3][8]; // H100, H010, H001, tH110, tH101, tH011, ttH111 at F = 60
   union
   {
-    int64_t G[7][NQ][E];     // xx yy zz xy xz yz, w |det|
-    int64_t tab[4 * 216][E]; // tables of a round
+    int64_t row[kRows][E];
+    struct
+    {
+      int64_t s1[7][54][E];  // after the first axis
+      int64_t G[7][NQ][E];   // xx yy zz xy xz yz, w |det| (before the tables)
+    };
     struct
     {
       double kd[E][NP + 1], md[E][NP + 1]; // entries
     };
   };
-  int64_t s1[7][54][E]; // after the first axis
   int64_t rq[NQ][E]; // load values (rqd: in FP64)
   int64_t coef[3][16][E];
   int64_t sm[6][E];
@@ -509,7 +525,7 @@ struct Shared
 static_assert(sizeof(Smem) * E <= sizeof(Shared), "the refused elements' buffers fit the block's");
 
 // x times s - 1, s in {0, 1, 2}
-__device__ __forceinline__ int64_t times(int64_t x, int s) { return s == 1 ? 0 : (s == 0 ? -x : x); }
+__device__ __forceinline__ int64_t times(int64_t x, int s) { return x * (int64_t)(s - 1); }
 
 // contraction of a plane v[qs][ql] (first axis done) over its two axes
 template <int KIND> // 0: P, D   1: P, P   2: S, S
@@ -539,6 +555,7 @@ __device__ __forceinline__ void plane(int64_t const (*in)[E], int64_t (*out)[E],
       out[c * 6 + k][el] = o[k];
   }
 }
+// the antisymmetric table of a component, and its negative 54 rows on
 __device__ __forceinline__ void planeA(int64_t const (*in)[E], int64_t (*out)[E], int el)
 {
   int64_t m[3][3];
@@ -552,7 +569,7 @@ __device__ __forceinline__ void planeA(int64_t const (*in)[E], int64_t (*out)[E]
     q2x::lineA(m[0][c], m[1][c], m[2][c], o);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
-      out[c * 3 + k][el] = o[k];
+      out[c * 3 + k][el] = o[k], out[54 + c * 3 + k][el] = -o[k];
   }
 }
 // l_a of three doubles
@@ -629,6 +646,10 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
   double const kfac = a.fold.coef ? a.kE[e] : 1.0;
 
   // ---- 0. inputs
+  // the ranks the warp's scatter will read
+  if (l < (N * N * 2 + 255) / 128)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<char const *>(a.rank + element(w) * (N * N)) +
+                                                  min(128 * l, N * N * 2 - 2)));
   if (tid < E)
     sh.lo[tid] = 0xffffffffu, sh.hi[tid] = 0, sh.ps[tid] = 0, sh.cons[tid] = 0;
   // group of eight lanes g = 3 element + coordinate, lane v = lattice vertex
@@ -865,10 +886,10 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
     if (T < 3)
     {
       if (needK)
-        plane<0>(sh.s1[T] + c * 9, sh.tab + x * 36, el);
+        plane<0>(sh.s1[T] + c * 9, sh.row + rowOf(0, x, 0, 0), el);
     }
     else if (needM)
-      plane<1>(sh.s1[3] + c * 9, sh.tab + x * 36, el);
+      plane<1>(sh.s1[3] + c * 9, sh.row + rowOf(0, x, 0, 0), el);
   }
   else
   {
@@ -936,26 +957,26 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
     kv[t] = 0, mv[t] = 0;
     if (p < NP)
     {
-      q2x::Pair const pr{gPairsX[p]};
-      int const cx = pr.sym(0), cy = pr.sym(1), cz = pr.sym(2);
+      ushort4 const r = gPairA[p];
       if (needK)
-        kv[t] = sh.tab[cy * 36 + cz * 6 + cx][el] + sh.tab[216 + cx * 36 + cz * 6 + cy][el] +
-                sh.tab[432 + cx * 36 + cy * 6 + cz][el];
+        kv[t] = sh.row[r.x][el] + sh.row[r.y][el] + sh.row[r.z][el];
       if (needM)
-        mv[t] = sh.tab[648 + cx * 36 + cy * 6 + cz][el];
+        mv[t] = sh.row[r.w][el];
     }
   }
   __syncthreads();
-  // the mixed components: SS at m 216 + lead 36 + s1 6 + s2, AA at 648 + m 54 + lead 9 + a1 3 + a2
+  // the mixed components
   if (needK)
   {
     if (x < 18)
-      plane<2>(sh.s1[4 + x / 6] + (x % 6) * 9, sh.tab + x * 36, el);
+      plane<2>(sh.s1[4 + x / 6] + (x % 6) * 9, sh.row + rowOf(0, x, 0, 0), el);
     if (x >= 14)
     {
       int const z = x - 14;
-      planeA(sh.s1[4 + z / 6] + (z % 6) * 9, sh.tab + 648 + z * 9, el);
+      planeA(sh.s1[4 + z / 6] + (z % 6) * 9, sh.row + rowAA(z / 6) + (z % 6) * 9, el);
     }
+    if (x == 31)
+      sh.row[kZero][el] = 0;
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < kPairsPerLane; ++t)
@@ -963,26 +984,9 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
       int const p = x + 32 * t;
       if (p < NP)
       {
-        q2x::Pair const pr{gPairsX[p]};
-        int const cx = pr.sym(0), cy = pr.sym(1), cz = pr.sym(2), ax = pr.anti(0), ay = pr.anti(1), az = pr.anti(2);
-        int64_t z = sh.tab[cz * 36 + cx * 6 + cy][el] + sh.tab[216 + cy * 36 + cx * 6 + cz][el] +
-                    sh.tab[432 + cx * 36 + cy * 6 + cz][el];
-        if (ax != 3 && ay != 3)
-        {
-          int64_t const y = sh.tab[648 + cz * 9 + ax * 3 + ay][el];
-          z = pr.up(0) == pr.up(1) ? z - y : z + y;
-        }
-        if (ax != 3 && az != 3)
-        {
-          int64_t const y = sh.tab[702 + cy * 9 + ax * 3 + az][el];
-          z = pr.up(0) == pr.up(2) ? z - y : z + y;
-        }
-        if (ay != 3 && az != 3)
-        {
-          int64_t const y = sh.tab[756 + cx * 9 + ay * 3 + az][el];
-          z = pr.up(1) == pr.up(2) ? z - y : z + y;
-        }
-        kv[t] += 2 * z;
+        uint4 const r = gPairB[p];
+        kv[t] += 2 * (sh.row[r.x & 0xffffu][el] + sh.row[r.x >> 16][el] + sh.row[r.y & 0xffffu][el] +
+                      sh.row[r.y >> 16][el] + sh.row[r.z & 0xffffu][el] + sh.row[r.z >> 16][el]);
       }
     }
     __syncthreads();
@@ -1007,14 +1011,15 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
   if (okw == 3u && (needK || needM))
   {
     uint16_t const * const rk = a.rank + ew * (N * N);
-    bool const plain = a.fold.simple && !(a.fold.bc && sh.cons[w]);
-#pragma unroll 6
-    for (int f = l; f < N * N; f += 32)
+    uint32_t const cons = a.fold.bc ? sh.cons[w] : 0u;
+    if (a.fold.simple && !cons)
     {
-      int const i = f / N, j = f - i * N, lo = min(i, j), hi = max(i, j), p = lo * (53 - lo) / 2 + hi;
-      int32_t const pij = sh.rp[w][i] + rk[f];
-      if (plain)
+#pragma unroll 12
+      for (int f = l; f < N * N; f += 32)
       {
+        uint32_t const ip = gEntry[f];
+        int const p = ip >> 8;
+        int32_t const pij = sh.rp[w][ip & 0xffu] + rk[f];
         if (a.fold.same)
           atomicAdd(a.fold.K + pij, sh.kd[w][p] + sh.md[w][p]);
         else
@@ -1025,8 +1030,47 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
             atomicAdd(a.fold.M + pij, sh.md[w][p]);
         }
       }
-      else
-        scatterGeneral(a, sh, w, ew, i, j, p, pij);
+    }
+    else if (a.fold.simple)
+    {
+      // with the Dirichlet condensation (builder.hpp:76-124): the diagonal of a
+      // constrained DOF, the lift -K_ij h_j of a free row
+      bool const one = needK && needM && !a.fold.same; // a second operator
+#pragma unroll 4
+      for (int f = l; f < N * N; f += 32)
+      {
+        uint32_t const ip = gEntry[f];
+        int const i = ip & 0xffu, j = f - i * N, p = ip >> 8;
+        int32_t const pij = sh.rp[w][i] + rk[f];
+        bool const ci = (cons >> i) & 1u, c = ci || ((cons >> j) & 1u);
+        // first operator: K, or K + M in one, or M alone; second: M
+        double v0 = needK ? sh.kd[w][p] : sh.md[w][p], v1 = one ? sh.md[w][p] : 0.;
+        if (a.fold.same)
+          v0 += sh.md[w][p];
+        double * const d0 = needK ? a.fold.K : a.fold.M;
+        bool const c0 = c && (needK ? a.fold.bcK : a.fold.bcM), c1 = one && c && a.fold.bcM;
+        if (!ci && (c0 || c1) && i != j && a.b)
+        {
+          double const z = ((c0 ? v0 : 0.) + (c1 ? v1 : 0.)) * a.bcVal[sh.dof[w][j]];
+          if (z != 0.)
+            atomicAdd(a.b + sh.dof[w][i], -z);
+        }
+        v0 = c0 ? a.bcDiag : v0, v1 = c1 ? a.bcDiag : v1;
+        if (!c0 || i == j)
+          atomicAdd(d0 + pij, v0);
+        if (one && (!c1 || i == j))
+          atomicAdd(a.fold.M + pij, v1);
+      }
+    }
+    else
+    {
+#pragma unroll 1
+      for (int f = l; f < N * N; f += 32)
+      {
+        uint32_t const ip = gEntry[f];
+        int const i = ip & 0xffu;
+        scatterGeneral(a, sh, w, ew, i, f - i * N, ip >> 8, sh.rp[w][i] + rk[f]);
+      }
     }
   }
   // refused elements, each by its warp in FP64
@@ -1124,7 +1168,7 @@ pxg_status initQ2F64Tables(pxg_ctx * c)
   for (int cc = 0; cc < 3; ++cc)
     for (int k = 0; k < 3; ++k)
       coefN[63 + 3 * cc + k] = coef[63 + 3 * cc + k] / first(63, cc);
-  std::vector<double> scale(kTab, 0.);
+  std::vector<double> scale(kScales, 0.);
   auto sP = [&](int cc) { return first(9, cc); };
   auto sD = [&](int cc) { return first(27, cc); };
   auto sS = [&](int cc) { return first(45, cc); };
@@ -1195,21 +1239,33 @@ pxg_status initQ2F64Tables(pxg_ctx * c)
     o[6] = aaIdx(px, iy, jy, iz, jz);
   }
   PXG_CUDA(c, cudaMemcpyToSymbol(gPairIdx, pidx.data(), pidx.size() * 2));
-  std::vector<uint32_t> px(pairs.size());
+  std::vector<ushort4> pa(pairs.size());
+  std::vector<uint4> pb(pairs.size());
+  std::vector<uint32_t> entry(N * N);
   for (size_t q = 0; q < pairs.size(); ++q)
   {
     int const i = pairs[q] >> 8, j = pairs[q] & 0xff;
-    int const L[2] = {latOfNode[i], latOfNode[j]}, div[3] = {9, 3, 1};
-    uint32_t v = (uint32_t)i << 18 | (uint32_t)j << 23;
-    for (int ax = 0; ax < 3; ++ax)
-    {
-      int const p = (L[0] / div[ax]) % 3, r = (L[1] / div[ax]) % 3;
-      v |= (uint32_t)symCls(p, r) << (3 * ax) | (uint32_t)(p == r ? 3 : p + r - 1) << (9 + 2 * ax) |
-           (uint32_t)(p < r) << (15 + ax);
-    }
-    px[q] = v;
+    int const Li = latOfNode[i], Lj = latOfNode[j];
+    int const I[3] = {Li / 9, (Li / 3) % 3, Li % 3}, J[3] = {Lj / 9, (Lj / 3) % 3, Lj % 3};
+    int const x = symCls(I[0], J[0]), y = symCls(I[1], J[1]), z = symCls(I[2], J[2]);
+    pa[q] = make_ushort4((unsigned short)rowOf(0, y, z, x), (unsigned short)rowOf(1, x, z, y),
+                         (unsigned short)rowOf(2, x, y, z), (unsigned short)rowOf(3, x, y, z));
+    // the term is 2 SS - 2 s s' AA, s the sign of j - i on an axis
+    auto anti = [&](int m, int lead, int u, int v) {
+      if (I[u] == J[u] || I[v] == J[v])
+        return kZero;
+      bool const minus = (I[u] < J[u]) == (I[v] < J[v]);
+      return rowAA(m) + (minus ? 54 : 0) + lead * 9 + (I[u] + J[u] - 1) * 3 + (I[v] + J[v] - 1);
+    };
+    auto two = [](int lo, int hi) { return (unsigned)lo | (unsigned)hi << 16; };
+    pb[q] = make_uint4(two(rowOf(0, z, x, y), anti(0, z, 0, 1)), two(rowOf(1, y, x, z), anti(1, y, 0, 2)),
+                       two(rowOf(2, x, y, z), anti(2, x, 1, 2)), 0u);
+    entry[i * N + j] = (uint32_t)i | (uint32_t)q << 8;
+    entry[j * N + i] = (uint32_t)j | (uint32_t)q << 8;
   }
-  PXG_CUDA(c, cudaMemcpyToSymbol(gPairsX, px.data(), px.size() * 4));
+  PXG_CUDA(c, cudaMemcpyToSymbol(gPairA, pa.data(), pa.size() * sizeof(ushort4)));
+  PXG_CUDA(c, cudaMemcpyToSymbol(gPairB, pb.data(), pb.size() * sizeof(uint4)));
+  PXG_CUDA(c, cudaMemcpyToSymbol(gEntry, entry.data(), entry.size() * 4));
   int64_t wx[NQ];
   for (int q = 0; q < NQ; ++q)
     wx[q] = (int64_t)(wl[q] * 4611686018427387904.0); // exact

@@ -102,17 +102,5 @@ __constant__
 // pi t / (pi g), rounded up: the bound of the offsets against q1x::offsetBound's
 constexpr float kBoundRatio = 1.3417f;
 
-// a pair (i, j), i <= j, of the element's nodes, packed: per axis the symmetric class of
-// (i, j) (3 bits), the antisymmetric one (2 bits; 3: i and j agree there) and whether
-// i < j (1 bit), then i and j (5 bits each)
-struct Pair
-{
-  uint32_t v;
-  PXG_HD int sym(int axis) const { return (v >> (3 * axis)) & 7; }
-  PXG_HD int anti(int axis) const { return (v >> (9 + 2 * axis)) & 3; }
-  PXG_HD bool up(int axis) const { return (v >> (15 + axis)) & 1; }
-  PXG_HD int i() const { return (v >> 18) & 31; }
-  PXG_HD int j() const { return (v >> 23) & 31; }
-};
 } // namespace q2x
 } // namespace pxg
