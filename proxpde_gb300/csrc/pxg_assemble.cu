@@ -25,6 +25,7 @@
 
 #include "pxg_dfl.h"
 #include "pxg_internal.h"
+#include "pxg_p2bary.h"
 
 namespace pxg
 {
@@ -331,6 +332,12 @@ pxg_status initTables(pxg_ctx * c)
       PXG_CUDA(c, cudaMemcpyToSymbol(cQ2xi, xi.data(), xi.size() * 8));
     }
   }
+  pxg_status const pg = initP2Group(c);
+  if (pg != PXG_OK)
+    return pg;
+  pxg_status const tl = initTetLoad(c);
+  if (tl != PXG_OK)
+    return tl;
   pxg_status const q2 = initQ2Tables(c);
   if (q2 != PXG_OK)
     return q2;
@@ -340,32 +347,6 @@ pxg_status initTables(pxg_ctx * c)
 }
 
 // ------------------------------------------------------------------ kernels
-// adjugate and determinant of a 3x3 matrix
-__device__ __forceinline__ double adj3(double const (&J)[3][3], double (&A)[3][3])
-{
-  A[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
-  A[0][1] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
-  A[0][2] = J[0][1] * J[1][2] - J[0][2] * J[1][1];
-  A[1][0] = J[1][2] * J[2][0] - J[1][0] * J[2][2];
-  A[1][1] = J[0][0] * J[2][2] - J[0][2] * J[2][0];
-  A[1][2] = J[0][2] * J[1][0] - J[0][0] * J[1][2];
-  A[2][0] = J[1][0] * J[2][1] - J[1][1] * J[2][0];
-  A[2][1] = J[0][1] * J[2][0] - J[0][0] * J[2][1];
-  A[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
-  return J[0][0] * A[0][0] + J[0][1] * A[1][0] + J[0][2] * A[2][0];
-}
-
-// G = s * A A^T (symmetric, packed 00 11 22 01 02 12)
-__device__ __forceinline__ void gram(double const (&A)[3][3], double s, double * G)
-{
-  G[0] = s * (A[0][0] * A[0][0] + A[0][1] * A[0][1] + A[0][2] * A[0][2]);
-  G[1] = s * (A[1][0] * A[1][0] + A[1][1] * A[1][1] + A[1][2] * A[1][2]);
-  G[2] = s * (A[2][0] * A[2][0] + A[2][1] * A[2][1] + A[2][2] * A[2][2]);
-  G[3] = s * (A[0][0] * A[1][0] + A[0][1] * A[1][1] + A[0][2] * A[1][2]);
-  G[4] = s * (A[0][0] * A[2][0] + A[0][1] * A[2][1] + A[0][2] * A[2][2]);
-  G[5] = s * (A[1][0] * A[2][0] + A[1][1] * A[2][1] + A[1][2] * A[2][2]);
-}
-
 __device__ __forceinline__ void red(double * p, double v) { atomicAdd(p, v); }
 
 template <int T, int NT>
@@ -988,89 +969,15 @@ __global__ void __launch_bounds__(NT) kAssembleTet(AsmArgs a)
 // kAssembleTet64 (the default for P1/P2) in IEEE binary64 throughout.  Per element:
 // J from the vertex differences, adj(J), |det J|, G = adj adj^T / |det J| (with a
 // single stiffness operator's coefficient folded in).  P1 reads its entries from G
-// directly; P2 with the usual stiffness + mass pair uses the barycentric form below,
+// directly; P2 with at most one stiffness and one mass uses the barycentric form below,
 // and otherwise the six-term products of G with the reference tensor (FP64 constant
 // memory).  A mass entry is |det J| Mhat_ij (a single mass operator's coefficient
 // folded into |det J|).  P2 tetrahedron: src/reffe.cpp:542-642, vertices then the
 // edges 01 12 20 03 13 23.
 
-// P2 in barycentric form.  With lambda_0 = 1 - x - y - z, lambda_1..3 = x, y, z, the
-// vertex and edge functions are phi_i = lambda_i (2 lambda_i - 1) and
-// phi_(ab) = 4 lambda_a lambda_b, whose gradients are linear in the lambdas, so with
-// s_kl = k |T| grad lambda_k . grad lambda_l and the exact moments
-// (1/|T|) int lambda_k lambda_l = (1 + delta_kl) / 20 the stiffness entries are short
-// integer combinations of s' = s / 5:
-//   vertex-vertex        K_ii = 3 s'_ii,  K_ij = -s'_ij
-//   vertex i, edge (ab)  i = a: 3 s'_ib - s'_ii;  i not in (ab): -(s'_ia + s'_ib)
-//   edge-edge            the same edge: 8 (s'_aa + s'_bb + s'_ab); sharing vertex v with
-//                        other ends p, q: 4 (s'_vv + s'_vq + s'_pv + 2 s'_pq); disjoint
-//                        (ab), (cd): 4 (s'_ac + s'_ad + s'_bc + s'_bd)
-// The gradients of the lambdas sum to zero, so every row of s sums to zero and so does
-// all of s.  With E_ab = s'_aa + s'_bb + s'_ab and r the vertex outside v, p, q the
-// edge-edge entries become 8 E_ab, 4 (2 s'_pq - s'_vr) (six distinct values over the
-// twelve pairs: the pairs sharing r with the same p, q give the same) and
-// -4 (E_ab + s'_ab): 36 FP64 operations for the 21 entries instead of 78.
-// The reference's 11-point rule integrates these degree-2 integrands exactly, so the
-// values agree with its per-quadrature-point sums to round-off (64 FP64 operations per
-// element for the 55 entries, instead of 177 for the reference-tensor products without
-// their zero terms).
-// exact negation: the sign bit flipped on the integer pipe
-__device__ __forceinline__ double negx(double x)
-{
-  return __hiloint2double(__double2hiint(x) ^ (int)0x80000000, __double2loint(x));
-}
-template <int I, int J>
-__device__ __forceinline__ double p2Stiff(double const (&s)[4][4], double const (&E)[6])
-{
-  if constexpr (J < 4)
-    return I == J ? 3.0 * s[I][I] : negx(s[I][J]);
-  else
-  {
-    constexpr int c = p2EdgeEnd(J, 0), d = p2EdgeEnd(J, 1);
-    if constexpr (I < 4)
-    {
-      if constexpr (I == c)
-        return fma(3.0, s[I][d], -s[I][I]);
-      else if constexpr (I == d)
-        return fma(3.0, s[I][c], -s[I][I]);
-      else
-        return -s[I][c] - s[I][d];
-    }
-    else
-    {
-      constexpr int a = p2EdgeEnd(I, 0), b = p2EdgeEnd(I, 1);
-      if constexpr (I == J)
-        return 8.0 * E[I - 4];
-      else if constexpr (a == c || a == d || b == c || b == d)
-      {
-        constexpr int v = (a == c || a == d) ? a : b, p = v == a ? b : a, q = c == v ? d : c;
-        constexpr int r = 6 - v - p - q;
-        return 4.0 * fma(2.0, s[p < q ? p : q][p < q ? q : p], -s[v < r ? v : r][v < r ? r : v]);
-      }
-      else
-        return -4.0 * (E[I - 4] + s[a][b]);
-    }
-  }
-}
-// a representative entry of each P2 mass class
-__host__ __device__ constexpr int p2MassRepI(int c) { return c < 4 ? 0 : 4; }
-__host__ __device__ constexpr int p2MassRepJ(int c)
-{
-  return c == 0 ? 0 : c == 1 ? 1 : c == 2 ? 4 : c == 3 ? 5 : c == 4 ? 4 : c == 5 ? 5 : 9;
-}
-// f(I, J) for the 55 pairs I <= J of the P2 element, as compile-time constants
-template <int I, int J, class F>
-__device__ __forceinline__ void p2ForPairs(F && f)
-{
-  f(std::integral_constant<int, I>{}, std::integral_constant<int, J>{});
-  if constexpr (J + 1 < 10)
-    p2ForPairs<I, J + 1>(f);
-  else if constexpr (I + 1 < 10)
-    p2ForPairs<I + 1, I + 1>(f);
-}
-
-template <int T, int NT>
-__global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
+// PLAIN: one operator's stiffness and the other's mass, no Dirichlet conditions
+template <int T, int NT, bool PLAIN>
+__global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_constant__ a)
 {
   constexpr int N = Elem<T>::N, NQ = Elem<T>::NQ;
   int64_t const i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1092,7 +999,7 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
   for (int i = 0; i < N; ++i)
     dof[i] = a.emap[e * N + i];
   uint32_t cons = 0;
-  if (a.bcMask)
+  if (!PLAIN && a.bcMask)
   {
 #pragma unroll
     for (int i = 0; i < N; ++i)
@@ -1103,7 +1010,7 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
   LhsDev const & op1 = a.op[1];
   bool const k0 = op0.on && op0.stiff, k1 = op1.on && op1.stiff;
   bool const m0 = op0.on && op0.mass, m1 = op1.on && op1.mass;
-  bool const needK = k0 || k1, needM = m0 || m1;
+  bool const needK = PLAIN || k0 || k1, needM = PLAIN || m0 || m1;
   bool const kE = usesCoef(op0) || usesCoef(op1);
   double const kfac = (kE && a.kE) ? a.kE[e] : 1.0;
 
@@ -1115,7 +1022,7 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
       J[r][cc] = X[cc + 1][r] - X[0][r];
   double A[3][3];
   double const adet = fabs(adj3(J, A));
-  bool const foldK = k0 != k1, foldM = m0 != m1;
+  bool const foldK = PLAIN || k0 != k1, foldM = PLAIN || m0 != m1;
   double const ks0 = k0 ? (op0.stiff == 2 ? op0.sc * kfac : op0.sc) : 0.;
   double const ks1 = k1 ? (op1.stiff == 2 ? op1.sc * kfac : op1.sc) : 0.;
   double const ms0 = m0 ? massCoef(op0, kfac) : 0., ms1 = m1 ? massCoef(op1, kfac) : 0.;
@@ -1128,10 +1035,11 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
     ra = fma(ra, fma(e, e, e), ra);
   }
   bool const anyBc = cons && ((op0.on && op0.bc) || (op1.on && op1.bc));
-  bool const kmPair = op0.on && op0.stiff && !op0.mass && op1.on && !op1.stiff && op1.mass;
-  // the usual operator pair (stiffness-only, then mass-only, both folded) in a warp
-  // without constrained entries: a loop without per-entry operator branches
-  bool const fast = kmPair && !__any_sync(__activemask(), anyBc);
+  // bcWarp: some lane has constrained entries.  fast: at most one stiffness and one mass
+  // (P2: both), their coefficients folded in, no per-entry operator branches
+  bool const bcWarp = !PLAIN && __any_sync(__activemask(), anyBc);
+  bool const both = PLAIN || (needK && needM && !a.fold.same);
+  bool const fast = PLAIN || (a.fold.simple && !bcWarp && (T == P1TET || both));
   double G[6];
   {
     double gs = (foldK ? (k0 ? ks0 : ks1) : 1.0) * ra;
@@ -1163,12 +1071,10 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
     K1[0][0] = cs[0] + (cs[1] + cs[2]);
   }
 
-  // the warp-group scatter of P2 finds its positions in its own map
-  bool const grouped = T == P2TET && fast && a.grpOff;
   int32_t rpn[N];
 #pragma unroll
   for (int n = 0; n < N; ++n)
-    rpn[n] = grouped ? 0 : a.rowPtr[dof[n]];
+    rpn[n] = a.rowPtr[dof[n]];
   uint16_t const * rk = a.rank + e * (int64_t)(N * N);
   constexpr int kRowUnroll = N <= 4 ? N : 1;
   if constexpr (T == P2TET)
@@ -1199,133 +1105,18 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
 #pragma unroll
       for (int c = 0; c < 7; ++c)
         mc[c] = am * MHAT<T>(p2MassRepI(c), p2MassRepJ(c));
-      if (!grouped)
-        pdlWait(); // the writes start here (the grouped path waits before its flush)
-      if (a.grpOff)
-      {
-        // warp-group scatter: the lane's values and the group's contribution codes to
-        // shared memory, then one reduction per distinct position of the warp's 32
-        // elements, in ascending order
-        extern __shared__ double gsm[];
-        int const lane = threadIdx.x & 31;
-        unsigned char * const wbase = reinterpret_cast<unsigned char *>(gsm) + (threadIdx.x >> 5) * kP2GroupSmemPerWarp;
-        double * const sw = reinterpret_cast<double *>(wbase);
-        uint16_t * const si = reinterpret_cast<uint16_t *>(wbase + kP2GroupValues * 32 * sizeof(double));
-        // value v of lane l at v * 32 + (l ^ (v & 15)): the flush reads, in one
-        // instruction, values of the same few elements (lanes) for different entries,
-        // which this swizzle spreads over the banks
-        auto swAt = [sw](uint32_t v, uint32_t l) -> double & { return sw[v * 32 + (l ^ (v & 15u))]; };
-        p2ForPairs<0, 0>([&](auto I, auto J) {
-          constexpr int i = decltype(I)::value, j = decltype(J)::value;
-          swAt(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
-        });
-#pragma unroll
-        for (int c = 0; c < 7; ++c)
-          swAt(55 + c, lane) = mc[c];
-        unsigned const mask = __activemask();
-        int const W = __popc(mask); // the active lanes are 0 .. W - 1
-        int64_t const g = e >> 5;
-        int const nItems = W * 100;
-        int32_t const dEnd = a.grpOff[g + 1];
-        constexpr int U = 4;
-        // the map of the next batch of positions is loaded while this one is summed and
-        // reduced; the first batch's loads are issued before the codes are staged
-        int32_t npos[U];
-        int nb0[U], nb1[U];
-        auto loadBatch = [&](int32_t d0) {
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-          {
-            int32_t const d = d0 + u * W + lane;
-            npos[u] = d < dEnd ? a.grpPos[d] : 0;
-            nb0[u] = d < dEnd ? a.grpBeg[d] : 0;
-            nb1[u] = d + 1 < dEnd ? a.grpBeg[d + 1] : nItems;
-          }
-        };
-        loadBatch(a.grpOff[g]);
-        // the group's codes: W * 100 of them, 16 bytes (8 codes) per load; the map pads
-        // the last group's codes to a multiple of 8
-        uint4 const * const gi = reinterpret_cast<uint4 const *>(a.grpItem + g * kP2GroupItems);
-        // every load of a batch in flight before the first store: at most 13 per lane
-        // for any warp width (ceil(12.5 W) / W < 13.5), in two batches of seven
-        int const n8 = (nItems + 7) / 8;
-        uint4 * const si4 = reinterpret_cast<uint4 *>(si);
-        static_assert(kP2GroupItems / 8 <= 32 * 14, "code staging batches");
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-        {
-          uint4 tmp[7];
-#pragma unroll
-          for (int r = 0; r < 7; ++r)
-          {
-            int const k = lane + (7 * h + r) * W;
-            if (k < n8)
-              tmp[r] = gi[k];
-          }
-#pragma unroll
-          for (int r = 0; r < 7; ++r)
-          {
-            int const k = lane + (7 * h + r) * W;
-            if (k < n8)
-              si4[k] = tmp[r];
-          }
-        }
-        __syncwarp(mask);
-        pdlWait(); // the writes start here
-        for (int32_t d0 = a.grpOff[g]; d0 < dEnd; d0 += U * W)
-        {
-          int32_t pos[U];
-          int b0[U], b1[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-            pos[u] = npos[u], b0[u] = nb0[u], b1[u] = nb1[u];
-          loadBatch(d0 + U * W);
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-          {
-            if (d0 + u * W + lane >= dEnd)
-              break;
-            // the position's contributions in element order: no addition for the
-            // first (the FP64 pipe is the scarce one)
-            // a position with few contributions: one reduction each (the L2 atomic unit
-            // has room, the FP64 pipe has not); more: sum them here, reduce once
-            if (b1[u] - b0[u] <= a.grpRedMax)
-            {
-              for (int k = b0[u]; k < b1[u]; ++k)
-              {
-                uint32_t const code = si[k];
-                red(op0.vals + pos[u], swAt((code >> 5) & 63u, code & 31u));
-                red(op1.vals + pos[u], swAt(55 + (code >> 11), code & 31u));
-              }
-              continue;
-            }
-            uint32_t code = si[b0[u]];
-            double kk = swAt((code >> 5) & 63u, code & 31u);
-            double mm = swAt(55 + (code >> 11), code & 31u);
-            for (int k = b0[u] + 1; k < b1[u]; ++k)
-            {
-              code = si[k];
-              kk += swAt((code >> 5) & 63u, code & 31u);
-              mm += swAt(55 + (code >> 11), code & 31u);
-            }
-            red(op0.vals + pos[u], kk);
-            red(op1.vals + pos[u], mm);
-          }
-        }
-        goto entriesDone;
-      }
+      pdlWait(); // the writes start here
       p2ForPairs<0, 0>([&](auto I, auto J) {
         constexpr int i = decltype(I)::value, j = decltype(J)::value;
         double const kv = p2Stiff<i, j>(s, E);
         double const mv = mc[p2MassClass(i, j)];
-        int32_t const pij = rpn[i] + rk[i * N + j];
-        red(op0.vals + pij, kv);
-        red(op1.vals + pij, mv);
+        int32_t const pij = rpn[i] + rk[i * N + j], pji = i == j ? pij : rpn[j] + rk[j * N + i];
+        red(a.fold.K + pij, kv);
+        red(a.fold.M + pij, mv);
         if constexpr (j != i)
         {
-          int32_t const pji = rpn[j] + rk[j * N + i];
-          red(op0.vals + pji, kv);
-          red(op1.vals + pji, mv);
+          red(a.fold.K + pji, kv);
+          red(a.fold.M + pji, mv);
         }
       });
       goto entriesDone;
@@ -1358,14 +1149,32 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs a)
         mv = am * MHAT<T>(i, j);
       int32_t const pij = rpi + rk[i * N + j];
       int32_t const pji = pickN(rpn, j) + rk[j * N + i];
-      if (fast)
+      if (PLAIN)
       {
-        red(op0.vals + pij, kv);
-        red(op1.vals + pij, mv);
+        red(a.fold.K + pij, kv);
+        red(a.fold.M + pij, mv);
         if (j != i)
         {
-          red(op0.vals + pji, kv);
-          red(op1.vals + pji, mv);
+          red(a.fold.K + pji, kv);
+          red(a.fold.M + pji, mv);
+        }
+        continue;
+      }
+      if (fast)
+      {
+        if (a.fold.same)
+          kv += mv;
+        if (needK)
+        {
+          red(a.fold.K + pij, kv);
+          if (j != i)
+            red(a.fold.K + pji, kv);
+        }
+        if (needM && !a.fold.same)
+        {
+          red(a.fold.M + pij, mv);
+          if (j != i)
+            red(a.fold.M + pji, mv);
         }
         continue;
       }
@@ -2012,25 +1821,23 @@ void launchAssembleTet(AsmArgs const & a, cudaStream_t s, int threads)
 }
 
 template <int T>
-void launchAssembleTet64(AsmArgs const & a, cudaStream_t s, int threads)
+void launchAssembleTet64(AsmArgs const & args, cudaStream_t s, int threads)
 {
+  AsmArgs a = args;
+  foldOps(a);
   auto go = [&](auto kern, int nt) {
     unsigned const blocks = (unsigned)((a.nelem + nt - 1) / nt);
-    size_t smem = 0;
-    if (T == P2TET && a.grpOff)
-    {
-      // the warp-group scatter's values and codes
-      smem = (size_t)(nt / 32) * kP2GroupSmemPerWarp;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    }
     if (blocks > 0)
-      launchElemKernel(kern, blocks, nt, smem, s, a);
+      launchElemKernel(kern, blocks, nt, 0, s, a);
   };
+  // the usual pair without Dirichlet conditions has its own instance: the others' branches
+  // cost its registers (64^3 x 6, K + M: 1.05 ms against 1.12)
+  bool const plain = a.fold.simple && a.fold.needK && a.fold.needM && !a.fold.same && !(a.bcMask && a.fold.bc);
   if (threads == 64)
-    return go(kAssembleTet64<T, 64>, 64);
+    return plain ? go(kAssembleTet64<T, 64, true>, 64) : go(kAssembleTet64<T, 64, false>, 64);
   if (threads == 256)
-    return go(kAssembleTet64<T, 256>, 256);
-  go(kAssembleTet64<T, 128>, 128);
+    return plain ? go(kAssembleTet64<T, 256, true>, 256) : go(kAssembleTet64<T, 256, false>, 256);
+  plain ? go(kAssembleTet64<T, 128, true>, 128) : go(kAssembleTet64<T, 128, false>, 128);
 }
 
 template <int T>
@@ -2317,17 +2124,29 @@ pxg_status pxg_assemble(pxg_ctx * c, pxg_lhs_op const * op0, double * vals0, pxg
       else if (fp64)
       {
         AsmArgs lg = la;
-        if (!la.perm && c->groups.built && c->groupScatter)
+        foldOps(lg);
+        if (!la.perm && c->groups.built && c->groupScatter && lg.fold.simple)
         {
           lg.grpOff = c->groups.off.p;
           lg.grpPos = c->groups.pos.p;
           lg.grpBeg = c->groups.beg.p;
           lg.grpItem = c->groups.item.p;
           lg.grpRedMax = c->groupRedMax;
+          // its loads: none or a constant; others in the one-thread kernel
+          bool const other = la.rkind && !(la.rkind == 1 && la.fn == PXG_FN_CONST);
+          if (other)
+            lg.rkind = 0;
+          launchAssembleP2Group(lg, s, c->threads);
+          if (other)
+          {
+            AsmArgs l2 = la;
+            l2.op[0].on = l2.op[1].on = 0;
+            l2.pdl = 0;
+            launchAssembleTet64<P2TET>(l2, s, c->threads);
+          }
         }
-        // the warp-group scatter's shared memory favours small blocks (64 threads: ten
-        // warps per SM), so that is its default
-        launchAssembleTet64<P2TET>(lg, s, c->threads ? c->threads : (lg.grpOff ? 64 : 128));
+        else
+          launchAssembleTet64<P2TET>(la, s, c->threads);
       }
       else
         launchAssembleTet<P2TET>(la, s, c->threads);
@@ -2351,6 +2170,22 @@ pxg_status pxg_assemble(pxg_ctx * c, pxg_lhs_op const * op0, double * vals0, pxg
     }
   };
   auto launch = [&](AsmArgs const & la) {
+    // sin sin sin on tetrahedra in the FP64 arithmetic: its own fixed-point kernel (P2
+    // 30^3 x 6 with K and M: in one FP64 kernel 0.53 ms, in the two 0.20; P1 16^3 x 6 38 and
+    // 32 us, 6^3 x 6 23 and 30: a second launch costs more than P1's twelve sines on few
+    // elements)
+    if (la.rkind == 1 && la.fn == PXG_FN_SIN3 && c->arith == PXG_ARITH_FP64 && !c->tetGeneric &&
+        (c->etype == P2TET || (c->etype == P1TET && la.nelem >= 12000)))
+    {
+      AsmArgs l1 = la, l2 = la;
+      if (la.op[0].on || la.op[1].on)
+      {
+        l1.rkind = 0;
+        launchElem(l1);
+        l2.pdl = 0; // the outputs are zeroed once the element kernel is done
+      }
+      return launchTetSineLoad(c->etype, l2, s);
+    }
     if (la.rkind != 3)
       return launchElem(la);
     if (la.op[0].on || la.op[1].on)

@@ -523,13 +523,11 @@ __host__ __device__ constexpr int p2UpperIdx(int i, int j)
 {
   return j < i ? p2UpperIdx(j, i) : i * 10 - i * (i - 1) / 2 + (j - i);
 }
-// warp-group scatter of the P2 kernel: per warp, the 55 stiffness entries and the 7 mass
-// values of each lane's element in shared memory, value-major (value v of lane l at
-// v * 32 + l), then the group's 3,200 contribution codes; a code is
-// lane | pair index << 5 | mass class << 11
+// warp-group scatter of the P2 kernel: the 55 stiffness entries and the 7 mass values of
+// each of a group's 32 elements in shared memory, and its 3,200 contribution codes; a code
+// is lane | pair index << 5 | mass class << 11
 constexpr int kP2GroupValues = 55 + 7;
 constexpr int kP2GroupItems = 32 * 100;
-constexpr size_t kP2GroupSmemPerWarp = kP2GroupValues * 32 * sizeof(double) + kP2GroupItems * sizeof(uint16_t);
 __host__ __device__ constexpr uint16_t p2GroupCode(int lane, int i, int j)
 {
   return (uint16_t)(lane | (p2UpperIdx(i, j) << 5) | (p2MassClass(i, j) << 11));
@@ -661,6 +659,13 @@ pxg_status initTables(pxg_ctx * c);
 void hostRule(int t, std::vector<double> & xi, std::vector<double> & w);
 pxg_status initQ2Tables(pxg_ctx * c);                      // pxg_q2.cu
 void launchAssembleQ2(AsmArgs const & a, cudaStream_t s, int sms); // pxg_q2.cu
+pxg_status initP2Group(pxg_ctx * c);                              // pxg_p2group.cu
+// P2 tetrahedra with the warp-group map (at most one stiffness and one mass; no load or a
+// constant)
+void launchAssembleP2Group(AsmArgs const & a, cudaStream_t s, int threads);
+pxg_status initTetLoad(pxg_ctx * c);                              // pxg_tetload.cu
+// the sin sin sin load of P1 / P2 tetrahedra (rhs kind 1)
+void launchTetSineLoad(int etype, AsmArgs const & a, cudaStream_t s);
 pxg_status initQ2F64Tables(pxg_ctx * c);                          // pxg_q2f64.cu
 void launchAssembleQ2F64(AsmArgs const & a, cudaStream_t s);      // pxg_q2f64.cu
 pxg_status buildScatterGroups(pxg_ctx * c);                       // pxg_group.cu

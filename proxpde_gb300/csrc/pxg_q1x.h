@@ -478,7 +478,7 @@ PXG_HD int64_t seriesCoef(SerC const & t, int e, int sc, int i, int64_t m, int e
   return (i & 2) ? -v : v;
 }
 // degree for a bound of |pi d|: truncation below 8e-19
-PXG_HD int seriesDegree(float bound) { return bound <= 0.0205f ? 7 : (bound <= 0.07f ? 9 : 15); }
+PXG_HD int seriesDegree(float bound) { return bound <= 0.0205f ? 7 : (bound <= 0.07f ? 9 : (bound <= 0.16f ? 11 : 15)); }
 // |det| sin sin sin from the three normalised values: F = 59
 PXG_HD int64_t pointLoad(int64_t f0, int64_t f1, int64_t f2, int64_t det)
 {
