@@ -26,6 +26,7 @@
 #include "pxg_dfl.h"
 #include "pxg_internal.h"
 #include "pxg_p2bary.h"
+#include "pxg_q1x.h"
 
 namespace pxg
 {
@@ -975,6 +976,74 @@ __global__ void __launch_bounds__(NT) kAssembleTet(AsmArgs a)
 // folded into |det J|).  P2 tetrahedron: src/reffe.cpp:542-642, vertices then the
 // edges 01 12 20 03 13 23.
 
+// P1 stiffness K_ij = ks C_i . C_j / |det J| (C_1..3 the cofactor vectors, C_0 minus their
+// sum) and |det J| in 64-bit fixed point (pxg_q1x.h, whose point functions take the edge
+// vectors J as columns): 33 FP64 instructions, nearly all conversions, where the FP64 form
+// has about 90.  False for an element the format refuses.
+__device__ __forceinline__ bool p1Fixed(double const (&J)[3][3], double ks, double (&K)[4][4], double & adet)
+{
+  using q1x::Sp;
+  int32_t m[3];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+  {
+    m[r] = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      m[r] = max(m[r], fx::hi32(fx::doubleBits(J[r][k])) & 0x7fffffff);
+  }
+  int sc[3];
+  bool ok = q1x::coordScales(m[0], m[1], m[2], sc);
+  int const scMin = min(sc[0], min(sc[1], sc[2]));
+  int64_t D[3][3]; // [column][coordinate] at F = 60
+  uint32_t cm[9];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+      D[k][r] = fx::roundToInt(fx::scaleExp(J[r][k], 60 - sc[r]));
+      cm[3 * k + r] = (uint32_t)abs(fx::hi32(D[k][r])) + 1u;
+    }
+  q1x::Shifts s;
+  ok = q1x::columnShifts(cm, s) && ok;
+  Sp c[3][3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+      c[k][r] = fx::splitOdd(q1x::shl(D[k][r], s.n[k]));
+  int const wt[3] = {sc[0] - scMin, sc[1] - scMin, sc[2] - scMin};
+  int64_t G[6];
+  int64_t const det =
+      q1x::pointProducts(c[0], c[1], c[2], __any_sync(__activemask(), (wt[0] | wt[1] | wt[2]) != 0) != 0, wt, G);
+  uint32_t const h = (uint32_t)fx::hi32(det);
+  int nd, k, ke;
+  int64_t km;
+  ok = q1x::detShifts(h, h, nd, k) && ok;
+  ok = fx::decompose(ks, km, ke) && ok;
+  ok = ok && abs(ke) < 300; // every value stays normal
+  if (!ok)
+    return false;
+  int const sg = q1x::productShift(q1x::productSize(G, s));
+  q1x::pointInverse(det, k, sg, fx::split(km), s, G);
+  int const eK = q1x::tensorExponent(sc, scMin, s, k, sg) + ke - 58;
+  adet = fx::toDouble(q1x::shl(det, nd), q1x::detExponent(sc, s, nd) - 60);
+  int64_t const Gs[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
+  int64_t cs[3];
+#pragma unroll
+  for (int b = 0; b < 3; ++b)
+  {
+    cs[b] = Gs[0][b] + Gs[1][b] + Gs[2][b];
+    K[0][b + 1] = fx::toDouble(-cs[b], eK);
+#pragma unroll
+    for (int a = 0; a <= b; ++a)
+      K[a + 1][b + 1] = fx::toDouble(Gs[a][b], eK);
+  }
+  K[0][0] = fx::toDouble(cs[0] + cs[1] + cs[2], eK);
+  return true;
+}
+
 // PLAIN: one operator's stiffness and the other's mass, no Dirichlet conditions
 template <int T, int NT, bool PLAIN>
 __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_constant__ a)
@@ -1020,56 +1089,58 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_consta
 #pragma unroll
     for (int cc = 0; cc < 3; ++cc)
       J[r][cc] = X[cc + 1][r] - X[0][r];
-  double A[3][3];
-  double const adet = fabs(adj3(J, A));
   bool const foldK = PLAIN || k0 != k1, foldM = PLAIN || m0 != m1;
   double const ks0 = k0 ? (op0.stiff == 2 ? op0.sc * kfac : op0.sc) : 0.;
   double const ks1 = k1 ? (op1.stiff == 2 ? op1.sc * kfac : op1.sc) : 0.;
   double const ms0 = m0 ? massCoef(op0, kfac) : 0., ms1 = m1 ? massCoef(op1, kfac) : 0.;
-  // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + e + e^2),
-  // e = 1 - x y), instead of a full-precision division with its special cases
-  double ra;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
-  {
-    double const e = fma(-adet, ra, 1.0);
-    ra = fma(ra, fma(e, e, e), ra);
-  }
   bool const anyBc = cons && ((op0.on && op0.bc) || (op1.on && op1.bc));
   // bcWarp: some lane has constrained entries.  fast: at most one stiffness and one mass
   // (P2: both), their coefficients folded in, no per-entry operator branches
   bool const bcWarp = !PLAIN && __any_sync(__activemask(), anyBc);
   bool const both = PLAIN || (needK && needM && !a.fold.same);
   bool const fast = PLAIN || (a.fold.simple && !bcWarp && (T == P1TET || both));
-  double G[6];
+  double const ksf = foldK ? (k0 ? ks0 : ks1) : 1.0;
+  double G[6], K1[4][4], adet;
+  // P1: with G carrying the sum of the Tet4 weights (the reference volume 1/6)
+  bool const fixed = T == P1TET && p1Fixed(J, ksf * cP1Ws, K1, adet);
+  if (!fixed)
   {
-    double gs = (foldK ? (k0 ? ks0 : ks1) : 1.0) * ra;
+    double A[3][3];
+    adet = fabs(adj3(J, A));
+    // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + e + e^2),
+    // e = 1 - x y), instead of a full-precision division with its special cases
+    double ra;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
+    {
+      double const e = fma(-adet, ra, 1.0);
+      ra = fma(ra, fma(e, e, e), ra);
+    }
+    double gs = ksf * ra;
     if constexpr (T == P1TET)
       gs *= cP1Ws;
     else if (fast)
       gs *= 1.0 / 30.0; // s'_(a+1)(b+1) = G_ab of the barycentric form
     gram(A, gs, G);
+    // P1: grad phi_i |det J| are the adjugate rows (i = 1..3) and minus their sum (i = 0),
+    // so K_ij = k / (6 |det J|) A_i . A_j reads the Gram entries of the adjugate directly:
+    // K_(a+1)(b+1) = G_ab, K_0(b+1) = -sum_a G_ab, K_00 = sum_ab G_ab
+    if constexpr (T == P1TET)
+    {
+      double const Gs[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
+      double cs[3];
+#pragma unroll
+      for (int b = 0; b < 3; ++b)
+      {
+        cs[b] = Gs[0][b] + (Gs[1][b] + Gs[2][b]);
+        K1[0][b + 1] = -cs[b];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          K1[a + 1][b + 1] = Gs[a][b];
+      }
+      K1[0][0] = cs[0] + (cs[1] + cs[2]);
+    }
   }
   double const am = foldM ? (m0 ? ms0 : ms1) * adet : adet;
-  // P1: grad phi_i |det J| are the adjugate rows (i = 1..3) and minus their sum (i = 0),
-  // so K_ij = k / (6 |det J|) A_i . A_j reads the Gram entries of the adjugate directly:
-  // K_(a+1)(b+1) = G_ab, K_0(b+1) = -sum_a G_ab, K_00 = sum_ab G_ab, with G carrying
-  // the sum of the Tet4 weights (the reference volume 1/6)
-  double K1[4][4];
-  if constexpr (T == P1TET)
-  {
-    double const Gs[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
-    double cs[3];
-#pragma unroll
-    for (int b = 0; b < 3; ++b)
-    {
-      cs[b] = Gs[0][b] + (Gs[1][b] + Gs[2][b]);
-      K1[0][b + 1] = -cs[b];
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-        K1[a + 1][b + 1] = Gs[a][b];
-    }
-    K1[0][0] = cs[0] + (cs[1] + cs[2]);
-  }
 
   int32_t rpn[N];
 #pragma unroll
@@ -2114,7 +2185,7 @@ pxg_status pxg_assemble(pxg_ctx * c, pxg_lhs_op const * op0, double * vals0, pxg
       if (c->tetGeneric)
         launchAssemble<P1TET>(la, s, c->threads);
       else if (fp64)
-        launchAssembleTet64<P1TET>(la, s, c->threads);
+        launchAssembleTet64<P1TET>(la, s, c->threads ? c->threads : 64); // 96^3 x 6: 0.79 ms, 128 threads 0.80
       else
         launchAssembleTet<P1TET>(la, s, c->threads);
       break;

@@ -63,7 +63,8 @@ struct Q1Shared
   uint32_t dof[8][32];
   int32_t rp[32][8];
   int32_t ee[3][32];            // exponents of the sine series
-  float bound[3][32];           // bounds of its argument
+  float bound[3][32];           // bounds of its argument, and their exponents
+  int32_t et[3][32];
   int32_t el[32];               // exponent of the load values
   uint32_t flags[32]; // bits 0-7 constrained nodes, 8 in the mesh, 9 fixed point holds it
 };
@@ -256,7 +257,8 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         sh.off[w][q][l] = off[q];
-      sh.bound[w][l] = q1x::offsetBound(cm, scw);
+      q1x::Bound const b = q1x::offsetBound(cm, scw);
+      sh.bound[w][l] = b.f, sh.et[w][l] = b.e;
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c)
@@ -372,9 +374,9 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
       f1 = q1x::mulAdd(q1x::split(f1), u1, sh.coef[1][i][l]);
       f2 = q1x::mulAdd(q1x::split(f2), u2, sh.coef[2][i][l]);
     }
-    int const n0 = q1x::seriesShift(sh.ee[0][l], sh.se[0][l], sh.bound[0][l]),
-              n1 = q1x::seriesShift(sh.ee[1][l], sh.se[2][l], sh.bound[1][l]),
-              n2 = q1x::seriesShift(sh.ee[2][l], sh.se[4][l], sh.bound[2][l]);
+    int const n0 = q1x::seriesShift(sh.ee[0][l], sh.se[0][l], sh.et[0][l]),
+              n1 = q1x::seriesShift(sh.ee[1][l], sh.se[2][l], sh.et[1][l]),
+              n2 = q1x::seriesShift(sh.ee[2][l], sh.se[4][l], sh.et[2][l]);
     sh.rq[w][l] = q1x::pointLoad(q1x::shl(f0, n0), q1x::shl(f1, n1), q1x::shl(f2, n2), det);
     if (w == 7)
       sh.el[l] = sh.ee[0][l] + sh.ee[1][l] + sh.ee[2][l] - (n0 + n1 + n2);

@@ -427,19 +427,29 @@ __constant__
 };
 constexpr int kLoadMaxScale = -2;   // largest sc
 constexpr float kLoadMaxT = 0.5f; // largest |pi d|
-// a bound of |pi d| for one coordinate from its columns' largest high words (zero for
-// elements below 2^-90, where it does not matter)
-PXG_HD float offsetBound(uint32_t const (&cmax)[3], int sc)
+// a bound x 2^k of |pi d| as a float (zero below 2^-100: for the degree) and its exponent
+struct Bound
 {
-  // pi g 2^(sc - 28) sum_a cmax
-  float const f = (float)(cmax[0] + cmax[1] + cmax[2] + 1u) * (1.8138f / 268435456.f);
-  if (sc < -90)
-    return 0.f;
+  float f;
+  int e; // below 2^e
+};
+PXG_HD Bound makeBound(float x, int k)
+{
+  Bound b;
 #ifdef __CUDA_ARCH__
-  return __int_as_float(__float_as_int(f) + (sc << 23));
+  int const i = __float_as_int(x);
+  b.e = (i >> 23) - 126 + k;
+  b.f = b.e < -100 ? 0.f : __int_as_float(i + (k << 23));
 #else
-  return __builtin_ldexpf(f, sc);
+  b.e = __builtin_ilogbf(x) + 1 + k;
+  b.f = b.e < -100 ? 0.f : __builtin_ldexpf(x, k);
 #endif
+  return b;
+}
+// the bound for one coordinate from its columns' largest high words: pi g 2^(sc - 28) sum cmax
+PXG_HD Bound offsetBound(uint32_t const (&cmax)[3], int sc, float ratio = 1.f)
+{
+  return makeBound((float)(cmax[0] + cmax[1] + cmax[2] + 1u) * (ratio * 1.8138f), sc - 28);
 }
 // mantissa (F = 62, signed) and exponent (at most 0) of a sine or cosine; zero: 0, -400
 PXG_HD void sineParts(double x, int64_t & m, int & e)
@@ -459,14 +469,10 @@ PXG_HD int seriesExponent(int es, int sc)
   int const k = sc + (Q2 ? (sc == -2 ? 8 : (sc == -3 ? 6 : 5)) : (sc == -2 ? 6 : 5));
   return 1 + (es > k ? es : k);
 }
-// the shift that normalises the series' sum: sin = sum 2^-62 2^(e - shift) after it
-PXG_HD int seriesShift(int e, int es, float bound)
+// the shift that normalises the series' sum, |pi d| below 2^et: sin = sum 2^-62
+// 2^(e - shift) after it
+PXG_HD int seriesShift(int e, int es, int et)
 {
-#ifdef __CUDA_ARCH__
-  int const et = (__float_as_int(bound) >> 23) - 126; // bound < 2^et
-#else
-  int const et = bound > 0.f ? __builtin_ilogbf(bound) + 1 : -126;
-#endif
   int const n = e - 1 - (es > et ? es : et);
   return n < 0 ? 0 : (n > 40 ? 40 : n);
 }

@@ -517,6 +517,7 @@ struct Shared
   int32_t dmax[3][E];
   int32_t se[6][E], ee[3][E];
   float bound[3][E];
+  int32_t et[3][E];
   uint32_t lo[E], hi[E], ps[E], cons[E], ok[E];
   int32_t el[E];
   uint32_t dof[E][N];
@@ -717,9 +718,10 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
     {
       uint32_t const c[3] = {z1 + z3 + z5 + z7, z2 + z3 + z6 + z7, z4 + z5 + z6 + z7};
       sh.cmax[ge][gr] = c[0], sh.cmax[ge][3 + gr] = c[1], sh.cmax[ge][6 + gr] = c[2];
-      float const b = q2x::kBoundRatio * q1x::offsetBound(c, sr);
+      q1x::Bound const b = q1x::offsetBound(c, sr, q2x::kBoundRatio);
       // the offsets hold at F = 61 below 4
-      sh.bound[gr][ge] = c[0] + c[1] + c[2] < (1u << 30) ? b : 1e30f;
+      sh.bound[gr][ge] = c[0] + c[1] + c[2] < (1u << 30) ? b.f : 1e30f;
+      sh.et[gr][ge] = b.e;
       if (sine)
       {
         double t[2];
@@ -836,9 +838,9 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
         f1 = q1x::mulAdd(q1x::split(f1), u1, sh.coef[1][i][el]);
         f2 = q1x::mulAdd(q1x::split(f2), u2, sh.coef[2][i][el]);
       }
-      int const n0 = q1x::seriesShift(sh.ee[0][el], sh.se[0][el], sh.bound[0][el]),
-                n1 = q1x::seriesShift(sh.ee[1][el], sh.se[2][el], sh.bound[1][el]),
-                n2 = q1x::seriesShift(sh.ee[2][el], sh.se[4][el], sh.bound[2][el]);
+      int const n0 = q1x::seriesShift(sh.ee[0][el], sh.se[0][el], sh.et[0][el]),
+                n1 = q1x::seriesShift(sh.ee[1][el], sh.se[2][el], sh.et[1][el]),
+                n2 = q1x::seriesShift(sh.ee[2][el], sh.se[4][el], sh.et[2][el]);
       sh.rq[q][el] = q1x::pointLoad(q1x::shl(f0, n0), q1x::shl(f1, n1), q1x::shl(f2, n2), dw);
       if (q == 0)
         sh.el[el] = sh.ee[0][el] + sh.ee[1][el] + sh.ee[2][el] - (n0 + n1 + n2);

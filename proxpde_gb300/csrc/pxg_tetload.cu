@@ -64,7 +64,8 @@ __global__ void __launch_bounds__(64) kTetSineLoad(AsmArgs const __grid_constant
   int sc[3];
   bool ok = q1x::coordScales(m[0], m[1], m[2], sc);
   Sp d[3][3];
-  float bound[3], bm = 0.f;
+  float bm = 0.f;
+  int et[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r)
   {
@@ -77,8 +78,9 @@ __global__ void __launch_bounds__(64) kTetSineLoad(AsmArgs const __grid_constant
       d[r][k] = fx::split(x);
     }
     // |pi sum xi_a d_a| <= pi 2^(sc - 30) max |d|
-    bound[r] = sc[r] < -90 ? 0.f : __int_as_float(__float_as_int((float)t * (3.1416f / 1073741824.f)) + (sc[r] << 23));
-    bm = fmaxf(bm, bound[r]);
+    q1x::Bound const b = q1x::makeBound((float)t * 3.1416f, sc[r] - 30);
+    et[r] = b.e;
+    bm = fmaxf(bm, b.f);
   }
   ok = ok && max(sc[0], max(sc[1], sc[2])) <= q1x::kLoadMaxScale && bm <= q1x::kLoadMaxT;
   uint32_t dof[N];
@@ -105,7 +107,7 @@ __global__ void __launch_bounds__(64) kTetSineLoad(AsmArgs const __grid_constant
 #pragma unroll
     for (int r = 0; r < 3; ++r)
       sinCosPiTab(X[0][r], S[r], C[r]);
-    int const ex = tetx::factors<NQ>(d, sc, bound, deg, S, C, xi, f);
+    int const ex = tetx::factors<NQ>(d, sc, et, deg, S, C, xi, f);
     Sp r[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; ++q)

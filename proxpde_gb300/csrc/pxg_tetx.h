@@ -43,9 +43,9 @@ PXG_HD int seriesExponent(int es, int sc)
 // The three factors at the points, interleaved (their chains of products hide each other's
 // latency): d[r][a] = differences of coordinate r of vertices 1..3 to vertex 0 (units
 // 2^sc[r], F = 62), xi(q, a) the points (F = 62), S[r], C[r] = sin, cos of pi times vertex
-// 0's coordinate; f[r] at F = 62; returns the sum of their exponents
+// 0's coordinate, |pi offset| below 2^et[r]; f[r] at F = 62; returns the sum of their exponents
 template <int NQ, class XI>
-PXG_HD int factors(Sp const (&d)[3][3], int const (&sc)[3], float const (&bound)[3], int deg, double const (&S)[3],
+PXG_HD int factors(Sp const (&d)[3][3], int const (&sc)[3], int const (&et)[3], int deg, double const (&S)[3],
                    double const (&C)[3], XI const & xi, int64_t (&f)[3][NQ])
 {
   int64_t ms[3], mc[3];
@@ -83,7 +83,7 @@ PXG_HD int factors(Sp const (&d)[3][3], int const (&sc)[3], float const (&bound)
 #pragma unroll
   for (int r = 0; r < 3; ++r)
   {
-    int const n = q1x::seriesShift(e[r], es[r], bound[r]);
+    int const n = q1x::seriesShift(e[r], es[r], et[r]);
     ex += e[r] - n;
 #pragma unroll
     for (int q = 0; q < NQ; ++q)
