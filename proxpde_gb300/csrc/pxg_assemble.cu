@@ -26,7 +26,7 @@
 #include "pxg_dfl.h"
 #include "pxg_internal.h"
 #include "pxg_p2bary.h"
-#include "pxg_q1x.h"
+#include "pxg_tetfx.h"
 
 namespace pxg
 {
@@ -977,58 +977,15 @@ __global__ void __launch_bounds__(NT) kAssembleTet(AsmArgs a)
 // edges 01 12 20 03 13 23.
 
 // P1 stiffness K_ij = ks C_i . C_j / |det J| (C_1..3 the cofactor vectors, C_0 minus their
-// sum) and |det J| in 64-bit fixed point (pxg_q1x.h, whose point functions take the edge
-// vectors J as columns): 33 FP64 instructions, nearly all conversions, where the FP64 form
-// has about 90.  False for an element the format refuses.
+// sum) and |det J| in 64-bit fixed point: 33 FP64 instructions, nearly all conversions, where
+// the FP64 form has about 90.  False for an element the format refuses.
 __device__ __forceinline__ bool p1Fixed(double const (&J)[3][3], double ks, double (&K)[4][4], double & adet)
 {
-  using q1x::Sp;
-  int32_t m[3];
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-  {
-    m[r] = 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      m[r] = max(m[r], fx::hi32(fx::doubleBits(J[r][k])) & 0x7fffffff);
-  }
-  int sc[3];
-  bool ok = q1x::coordScales(m[0], m[1], m[2], sc);
-  int const scMin = min(sc[0], min(sc[1], sc[2]));
-  int64_t D[3][3]; // [column][coordinate] at F = 60
-  uint32_t cm[9];
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-    {
-      D[k][r] = fx::roundToInt(fx::scaleExp(J[r][k], 60 - sc[r]));
-      cm[3 * k + r] = (uint32_t)abs(fx::hi32(D[k][r])) + 1u;
-    }
-  q1x::Shifts s;
-  ok = q1x::columnShifts(cm, s) && ok;
-  Sp c[3][3];
-#pragma unroll
-  for (int k = 0; k < 3; ++k)
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-      c[k][r] = fx::splitOdd(q1x::shl(D[k][r], s.n[k]));
-  int const wt[3] = {sc[0] - scMin, sc[1] - scMin, sc[2] - scMin};
-  int64_t G[6];
-  int64_t const det =
-      q1x::pointProducts(c[0], c[1], c[2], __any_sync(__activemask(), (wt[0] | wt[1] | wt[2]) != 0) != 0, wt, G);
-  uint32_t const h = (uint32_t)fx::hi32(det);
-  int nd, k, ke;
-  int64_t km;
-  ok = q1x::detShifts(h, h, nd, k) && ok;
-  ok = fx::decompose(ks, km, ke) && ok;
-  ok = ok && abs(ke) < 300; // every value stays normal
-  if (!ok)
+  int64_t km, G[6];
+  int ke, eK;
+  bool const okK = fx::decompose(ks, km, ke);
+  if (!tetTensor(J, okK && abs(ke) < 300, km, ke, G, eK, adet))
     return false;
-  int const sg = q1x::productShift(q1x::productSize(G, s));
-  q1x::pointInverse(det, k, sg, fx::split(km), s, G);
-  int const eK = q1x::tensorExponent(sc, scMin, s, k, sg) + ke - 58;
-  adet = fx::toDouble(q1x::shl(det, nd), q1x::detExponent(sc, s, nd) - 60);
   int64_t const Gs[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
   int64_t cs[3];
 #pragma unroll

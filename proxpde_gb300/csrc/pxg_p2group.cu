@@ -11,6 +11,7 @@
 
 #include "pxg_internal.h"
 #include "pxg_p2bary.h"
+#include "pxg_tetfx.h"
 
 namespace pxg
 {
@@ -29,9 +30,29 @@ struct GroupShared
 
 __device__ __forceinline__ void red(double * p, double v) { atomicAdd(p, v); }
 
+// s (4 x 4, zero row sums) and E_ab = s_aa + s_bb + s_ab of the six edges from the Gram
+// entries of vertices 1..3
+template <class V>
+__device__ __forceinline__ void gramRows(V const (&G)[6], V (&s)[4][4], V (&E)[6])
+{
+  s[1][1] = G[0], s[2][2] = G[1], s[3][3] = G[2];
+  s[1][2] = s[2][1] = G[3];
+  s[1][3] = s[3][1] = G[4];
+  s[2][3] = s[3][2] = G[5];
+  V const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
+  s[0][1] = s[1][0] = -c1;
+  s[0][2] = s[2][0] = -c2;
+  s[0][3] = s[3][0] = -c3;
+  s[0][0] = c1 + (c2 + c3);
+#pragma unroll
+  for (int n = 0; n < 6; ++n)
+    E[n] = (s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 0)] + s[p2EdgeEnd(4 + n, 1)][p2EdgeEnd(4 + n, 1)]) +
+           s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 1)];
+}
+
 // PLAIN: one operator's stiffness and the other's mass, no Dirichlet conditions
 template <bool PLAIN>
-__global__ void __launch_bounds__(64) kAssembleP2Group(AsmArgs const __grid_constant__ a)
+__global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs const __grid_constant__ a)
 {
   __shared__ GroupShared sh;
   int const lane = threadIdx.x & 31;
@@ -100,45 +121,52 @@ __global__ void __launch_bounds__(64) kAssembleP2Group(AsmArgs const __grid_cons
           }
         }
       }
-      double J[3][3], A[3][3];
+      double J[3][3];
 #pragma unroll
       for (int r = 0; r < 3; ++r)
 #pragma unroll
         for (int k = 0; k < 3; ++k)
           J[r][k] = X[k + 1][r] - X[0][r];
-      adet = fabs(adj3(J, A));
-      // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + t + t^2),
-      // t = 1 - x y), instead of a full-precision division with its special cases
-      double ra;
-      asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
-      double const t = fma(-adet, ra, 1.0);
-      ra = fma(ra, fma(t, t, t), ra);
-      // s'_(a+1)(b+1) = G_ab, the adjugate's Gram matrix times k / (30 |det J|)
-      double G[6];
-      gram(A, (a.fold.coefK ? a.fold.sK * kfac : a.fold.sK) * ra * (1.0 / 30.0), G);
-      if (needK)
+      double const ks = a.fold.coefK ? a.fold.sK * kfac : a.fold.sK;
+      // the entries are integer combinations of s'_(a+1)(b+1) = G_ab, the Gram matrix of the
+      // cofactors times k / (30 |det J|): km carries 16 / 30
+      int64_t km, Gx[6];
+      int ke, eG;
+      bool const okK = fx::decompose(ks, km, ke);
+      km = q1x::shl(fx::mulc(fx::cst(0x4444444444444444ll), km), 1);
+      if (tetTensor(J, okK && abs(ke) < 300, km, ke - 4, Gx, eG, adet))
       {
-        double s[4][4];
-        s[1][1] = G[0];
-        s[2][2] = G[1];
-        s[3][3] = G[2];
-        s[1][2] = s[2][1] = G[3];
-        s[1][3] = s[3][1] = G[4];
-        s[2][3] = s[3][2] = G[5];
-        double const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
-        s[0][1] = s[1][0] = negx(c1);
-        s[0][2] = s[2][0] = negx(c2);
-        s[0][3] = s[3][0] = negx(c3);
-        s[0][0] = c1 + (c2 + c3);
-        double E[6]; // E_ab = s'_aa + s'_bb + s'_ab of the six edges
-#pragma unroll
-        for (int n = 0; n < 6; ++n)
-          E[n] = (s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 0)] + s[p2EdgeEnd(4 + n, 1)][p2EdgeEnd(4 + n, 1)]) +
-                 s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 1)];
-        p2ForPairs<0, 0>([&](auto I, auto Jj) {
-          constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-          at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
-        });
+        if (needK)
+        {
+          int64_t s[4][4], E[6];
+          gramRows(Gx, s, E);
+          p2ForPairs<0, 0>([&](auto I, auto Jj) {
+            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+            at(p2UpperIdx(i, j), lane) = fx::toDouble(p2StiffFixed<i, j>(s, E), eG);
+          });
+        }
+      }
+      else
+      {
+        double A[3][3];
+        adet = fabs(adj3(J, A));
+        // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + t + t^2),
+        // t = 1 - x y), instead of a full-precision division with its special cases
+        double ra;
+        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
+        double const t = fma(-adet, ra, 1.0);
+        ra = fma(ra, fma(t, t, t), ra);
+        double G[6];
+        gram(A, ks * ra * (1.0 / 30.0), G);
+        if (needK)
+        {
+          double s[4][4], E[6];
+          gramRows(G, s, E);
+          p2ForPairs<0, 0>([&](auto I, auto Jj) {
+            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+            at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
+          });
+        }
       }
       if (needM)
       {
