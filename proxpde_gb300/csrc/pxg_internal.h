@@ -187,7 +187,7 @@ struct DevBuf
 struct CgWork
 {
   int64_t n = 0;
-  pxg::DevBuf<double> r, z, p, q, dinv, part, scal;
+  pxg::DevBuf<double> r, z, p, dinv, part, scal;
   cudaStream_t stream = nullptr;
   cudaEvent_t evIn = nullptr, evOut = nullptr;
   ~CgWork()
