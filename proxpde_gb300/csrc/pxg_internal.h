@@ -216,11 +216,9 @@ struct BatchState
 {
   bool ready = false;
   int64_t nprob = 0;
-  int probBase = 0; // global id of this batch's first problem in the last solve
   pxg::DevBuf<int64_t> elemOff, dofOff;
   std::vector<int64_t> dofOffHost;
-  pxg::DevBuf<int32_t> rowProb;
-  pxg::DevBuf<double> K, M, b, u, lam, r, z, p, q, dinv, w, Mw;
+  pxg::DevBuf<double> K, M, b, u, lam, r, z, p, dinv, w, Mw;
 };
 
 // arguments a captured batch graph was built for
@@ -233,13 +231,14 @@ struct GraphKey
   pxg_rhs_op rhs{};
   double rtol = 0.;
   int maxIter = 0;
+  int smem = 0;
   int scatter[2] = {0, 0}, threads[2] = {0, 0}; // the element kernels captured in the graph
   int arith[2] = {0, 0};
   bool operator==(GraphKey const & o) const
   {
     return nctx == o.nctx && ctx[0] == o.ctx[0] && ctx[1] == o.ctx[1] && ut[0] == o.ut[0] && ut[1] == o.ut[1] &&
            grad[0] == o.grad[0] && grad[1] == o.grad[1] && rhs.kind == o.rhs.kind && rhs.fn == o.rhs.fn &&
-           rhs.coef == o.rhs.coef && rhs.field == o.rhs.field && rtol == o.rtol && maxIter == o.maxIter &&
+           rhs.coef == o.rhs.coef && rhs.field == o.rhs.field && rtol == o.rtol && maxIter == o.maxIter && smem == o.smem &&
            scatter[0] == o.scatter[0] && scatter[1] == o.scatter[1] && threads[0] == o.threads[0] &&
            threads[1] == o.threads[1] && arith[0] == o.arith[0] && arith[1] == o.arith[1];
   }
@@ -249,16 +248,9 @@ struct GraphKey
 struct BatchShared
 {
   int nprob = 0;
-  pxg::DevBuf<double> acc;
-  pxg::DevBuf<int> done, itF, itA, err;
-  pxg::DevBuf<unsigned> bar;
-  // problem table (global problem id -> system, first row, rows) and the per-iteration
-  // row chunks of the running problems, two tables used by alternate iterations
-  pxg::DevBuf<int> probSys;
-  pxg::DevBuf<int64_t> probRow0, probRows;
-  int64_t capChunks = 0;
-  pxg::DevBuf<int> chunkProb[2], chunkRows[2], nchunk;
-  pxg::DevBuf<int64_t> chunkRow0[2];
+  pxg::DevBuf<unsigned char> res, prob, group; // results, problem list, the blocks' groups
+  pxg::DevBuf<double> part;                    // the blocks' sums
+  pxg::DevBuf<unsigned> bar;                   // the groups' arrivals, the error flag
   cudaGraphExec_t exec = nullptr;
   GraphKey key;
   ~BatchShared()
