@@ -95,13 +95,14 @@ __device__ __forceinline__ int64_t position(int32_t const * rp, int32_t const * 
 }
 
 // Entry (I, J) = (row DOF i, component d1; column DOF j, component d2) of element e:
-// the call's Dirichlet condensation, or the FP64 reduction at its CSR position
-__device__ __forceinline__ void sysEmit(SysArgs const & a, int64_t e, int I, int J, double v,
-                                       unsigned char const * consR, unsigned char const * consC, double const * h)
+// the call's Dirichlet condensation, or the FP64 reduction at its CSR position pos(row)
+template <class Pos>
+__device__ __forceinline__ void sysEmit(SysArgs const & a, int64_t e, int i, int d1, int j, int d2, double v,
+                                       unsigned char const * consR, unsigned char const * consC, double const * h,
+                                       Pos && pos)
 {
-  int const i = I % a.Nr, d1 = I / a.Nr, j = J % a.Nc, d2 = J / a.Nc;
+  int const I = d1 * a.Nr + i, J = d2 * a.Nc + j;
   int64_t const gI = a.offr + a.emr[e * a.Nr + i] + (int64_t)d1 * a.ndr;
-  int64_t const gJ = a.offc + a.emc[e * a.Nc + j] + (int64_t)d2 * a.ndc;
   bool const cI = consR[I], cJ = consC[J];
   if (cI || cJ)
   {
@@ -116,7 +117,7 @@ __device__ __forceinline__ void sysEmit(SysArgs const & a, int64_t e, int I, int
     }
     return;
   }
-  atomicAdd(a.vals + position(a.rowPtr, a.colIdx, gI, (int32_t)gJ), v);
+  atomicAdd(a.vals + pos(gI), v);
 }
 
 __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
@@ -132,6 +133,7 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
   double * wph = h + Lc;            // nq * Nr: JxW phi (block path)
   auto * consR = reinterpret_cast<unsigned char *>(wph + nq * Nr);
   unsigned char * consC = consR + Lr;
+  __shared__ int32_t perComp[27]; // columns of a component in the rows of a node (block path)
   double const * W = a.tab;
   double const * dV = W + nq;
   double const * phr = dV + nq * nv * 3;
@@ -209,6 +211,17 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
         dRc[3 * k + 2] = w * dRr[3 * k + 2];
         wph[k] = w * phr[k];
       }
+      // The pattern couples all components of two nodes or none, so a node's rows have the same
+      // columns and each component's follow the one before: one search per ordered pair of nodes
+      // gives its nine positions (a search per entry was most of the kernel's time: 18 of nine
+      // dependent loads per pair, @@)
+      if (a.dr > 1)
+        for (int i = threadIdx.x; i < Nr; i += blockDim.x)
+        {
+          int64_t const row = a.offr + a.emr[e * Nr + i];
+          perComp[i] = (int32_t)(position(a.rowPtr, a.colIdx, row, (int32_t)(row + a.ndr)) -
+                                 position(a.rowPtr, a.colIdx, row, (int32_t)row));
+        }
       __syncthreads();
       bool needM = false;
       for (int k = 0; k < a.nops; ++k)
@@ -236,9 +249,16 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
             M = fma(phr[q * Nr + i], wph[q * Nr + j], M);
         }
         double const K = B[0][0] + B[1][1] + B[2][2];
-        for (int d1 = 0; d1 < a.dr; ++d1)
-          for (int d2 = 0; d2 < a.dr; ++d2)
+        int64_t const gi = a.offr + a.emr[e * Nr + i], gj = a.offr + a.emr[e * Nr + j];
+        int64_t const rij = position(a.rowPtr, a.colIdx, gi, (int32_t)gj) - a.rowPtr[gi];
+        int64_t const rji = position(a.rowPtr, a.colIdx, gj, (int32_t)gi) - a.rowPtr[gj];
+#pragma unroll
+        for (int d1 = 0; d1 < 3; ++d1)
+#pragma unroll
+          for (int d2 = 0; d2 < 3; ++d2)
           {
+            if (d1 >= a.dr || d2 >= a.dr)
+              continue;
             double v = 0., vt = 0.; // entries (i d1, j d2) and (j d1, i d2)
             for (int k = 0; k < a.nops; ++k)
             {
@@ -268,13 +288,28 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
                 break;
               }
             }
-            sysEmit(a, e, d1 * Nr + i, d2 * Nr + j, v, consR, consC, h);
+            sysEmit(a, e, i, d1, j, d2, v, consR, consC, h,
+                    [&](int64_t row) { return a.rowPtr[row] + rij + d2 * perComp[i]; });
             if (i != j)
-              sysEmit(a, e, d1 * Nr + j, d2 * Nr + i, vt, consR, consC, h);
+              sysEmit(a, e, j, d1, i, d2, vt, consR, consC, h,
+                      [&](int64_t row) { return a.rowPtr[row] + rji + d2 * perComp[j]; });
           }
       }
       continue;
     }
+    // JxW into the row functions once, where no operator needs the gradients without it
+    bool plain = false;
+    for (int k = 0; k < a.nops; ++k)
+      plain = plain || a.kind[k] == PXG_OP_STIFFNESS || a.kind[k] == PXG_OP_TENSOR_STIFFNESS;
+    for (int k = threadIdx.x; k < nq * Nr; k += blockDim.x)
+    {
+      double const w = JxW[k / Nr];
+      wph[k] = w * phr[k];
+      if (!plain)
+        for (int c = 0; c < 3; ++c)
+          dRr[3 * k + c] *= w;
+    }
+    __syncthreads();
     for (int p = threadIdx.x; p < Lr * Lc; p += blockDim.x)
     {
       int const I = p / Lc, J = p % Lc;
@@ -300,20 +335,22 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
         case PXG_OP_MASS:
           if (d1 == d2)
             for (int q = 0; q < nq; ++q)
-              s += JxW[q] * phr[q * Nr + i] * phc[q * Nc + j];
+              s += wph[q * Nr + i] * phc[q * Nc + j];
           break;
         case PXG_OP_GRAD:
           for (int q = 0; q < nq; ++q)
-            s += JxW[q] * dRr[3 * (q * Nr + i) + d1] * phc[q * Nc + j];
+            s += (plain ? JxW[q] * dRr[3 * (q * Nr + i) + d1] : dRr[3 * (q * Nr + i) + d1]) * phc[q * Nc + j];
           break;
         case PXG_OP_DIV:
           for (int q = 0; q < nq; ++q)
-            s += JxW[q] * phr[q * Nr + i] * dRc[3 * (q * Nc + j) + d2];
+            s += wph[q * Nr + i] * dRc[3 * (q * Nc + j) + d2];
           break;
         }
         v += a.coef[k] * s;
       }
-      sysEmit(a, e, I, J, v, consR, consC, h);
+      int64_t const gJ = a.offc + a.emc[e * Nc + j] + (int64_t)d2 * a.ndc;
+      sysEmit(a, e, i, d1, j, d2, v, consR, consC, h,
+              [&](int64_t row) { return position(a.rowPtr, a.colIdx, row, (int32_t)gJ); });
     }
   }
 }
