@@ -22,6 +22,7 @@
 #include <memory>
 #include <vector>
 
+#include "pxg_fx.h"
 #include "pxg_internal.h"
 
 struct pxg_sys
@@ -94,6 +95,13 @@ __device__ __forceinline__ int64_t position(int32_t const * rp, int32_t const * 
   return lo;
 }
 
+// x 2^k, rounded to an integer and split into two words, in x's place (below 2^-700: zero)
+__device__ __forceinline__ void toFixed(double & x, int k)
+{
+  int const ex = fx::expoField(x) + k;
+  *reinterpret_cast<fx::Sp *>(&x) = fx::split(ex > 0 ? fx::roundToInt(fx::scaleExp(x, k)) : 0);
+}
+
 // Entry (I, J) = (row DOF i, component d1; column DOF j, component d2) of element e:
 // the call's Dirichlet condensation, or the FP64 reduction at its CSR position pos(row)
 template <class Pos>
@@ -120,6 +128,8 @@ __device__ __forceinline__ void sysEmit(SysArgs const & a, int64_t e, int i, int
   atomicAdd(a.vals + pos(gI), v);
 }
 
+// FIXED: the block path's sums over the quadrature points in 64-bit fixed point
+template <bool FIXED>
 __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
 {
   extern __shared__ double sm[];
@@ -134,6 +144,7 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
   auto * consR = reinterpret_cast<unsigned char *>(wph + nq * Nr);
   unsigned char * consC = consR + Lr;
   __shared__ int32_t perComp[27]; // columns of a component in the rows of a node (block path)
+  __shared__ int top[6];          // upper words of the largest gradient components, plain and weighted
   double const * W = a.tab;
   double const * dV = W + nq;
   double const * phr = dV + nq * nv * 3;
@@ -145,6 +156,8 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
     __syncthreads(); // the previous element's entries are done with the shared data
     for (int k = threadIdx.x; k < nv * 3; k += blockDim.x)
       X[k] = a.xyz[3 * (int64_t)a.conn[e * nv + k / 3] + k % 3];
+    if (threadIdx.x < 6)
+      top[threadIdx.x] = 0;
     __syncthreads();
     for (int q = threadIdx.x; q < nq; q += blockDim.x)
     {
@@ -203,6 +216,7 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
       // one space: B_d1d2(i, j) = sum_q JxW grad_d1 phi_i grad_d2 phi_j for the pairs
       // i <= j gives all nine component blocks of (i, j) and, transposed, of (j, i); the
       // stiffness is the trace of B
+      int big[6] = {0, 0, 0, 0, 0, 0};
       for (int k = threadIdx.x; k < nq * Nr; k += blockDim.x)
       {
         double const w = JxW[k / Nr];
@@ -210,11 +224,26 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
         dRc[3 * k + 1] = w * dRr[3 * k + 1];
         dRc[3 * k + 2] = w * dRr[3 * k + 2];
         wph[k] = w * phr[k];
+        if (FIXED)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+        {
+          big[c] = max(big[c], fx::hi32(fx::doubleBits(dRr[3 * k + c])) & 0x7fffffff);
+          big[3 + c] = max(big[3 + c], fx::hi32(fx::doubleBits(dRc[3 * k + c])) & 0x7fffffff);
+        }
+      }
+      if (FIXED)
+#pragma unroll
+      for (int c = 0; c < 6; ++c)
+      {
+        big[c] = (int)__reduce_max_sync(0xffffffffu, (unsigned)big[c]);
+        if ((threadIdx.x & 31) == 0)
+          atomicMax(top + c, big[c]);
       }
       // The pattern couples all components of two nodes or none, so a node's rows have the same
       // columns and each component's follow the one before: one search per ordered pair of nodes
-      // gives its nine positions (a search per entry was most of the kernel's time: 18 of nine
-      // dependent loads per pair, @@)
+      // gives its nine positions (a search per entry, 18 of nine dependent loads per pair:
+      // 2.33 ms for the three blocks of 16^3 Q2-Q1, now 1.73 ms)
       if (a.dr > 1)
         for (int i = threadIdx.x; i < Nr; i += blockDim.x)
         {
@@ -223,6 +252,27 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
                                  position(a.rowPtr, a.colIdx, row, (int32_t)row));
         }
       __syncthreads();
+      // the gradients to 64-bit fixed point, each component with its largest magnitude's exponent
+      // (F: |x| <= 2^58), in place as pairs of words
+      int sh[6];
+      bool fixed = FIXED;
+#pragma unroll
+      for (int c = 0; c < 6 && FIXED; ++c)
+      {
+        int const ex = top[c] >> 20;
+        fixed = fixed && ex > 700 && ex < 1350;
+        sh[c] = 58 - (ex - 1022);
+      }
+      if (fixed)
+      {
+        for (int k = threadIdx.x; k < 3 * nq * Nr; k += blockDim.x)
+        {
+          int const c = k % 3;
+          toFixed(dRr[k], c == 0 ? sh[0] : c == 1 ? sh[1] : sh[2]);
+          toFixed(dRc[k], c == 0 ? sh[3] : c == 1 ? sh[4] : sh[5]);
+        }
+        __syncthreads();
+      }
       bool needM = false;
       for (int k = 0; k < a.nops; ++k)
         needM = needM || a.kind[k] == PXG_OP_MASS;
@@ -236,7 +286,37 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
         }
         int const j = i + rem;
         double B[3][3] = {{0., 0., 0.}, {0., 0., 0.}, {0., 0., 0.}}, M = 0.;
-        for (int q = 0; q < nq; ++q)
+        if (fixed)
+        {
+          // four 32-bit multiply-adds a term; the 27 terms' sums of each kind stay below 2^63.
+          // Error of 27 terms, rms against 128 bits: 4.7e-17 of the sum, 6.8e-17 where the pair's
+          // gradients are up to 2^-8 of the element's largest (FP64: 1.7e-16)
+          fx::Sp const * const gs = reinterpret_cast<fx::Sp const *>(dRr), * const ws = reinterpret_cast<fx::Sp const *>(dRc);
+          int64_t hh[9] = {}, hl[9] = {}, ll[9] = {};
+          for (int q = 0; q < nq; ++q)
+          {
+            fx::Sp const * const gi = gs + 3 * (q * Nr + i), * const wj = ws + 3 * (q * Nr + j);
+#pragma unroll
+            for (int d1 = 0; d1 < 3; ++d1)
+#pragma unroll
+              for (int d2 = 0; d2 < 3; ++d2)
+              {
+                hh[3 * d1 + d2] = fx::madw(gi[d1].h, wj[d2].h, hh[3 * d1 + d2]);
+                hl[3 * d1 + d2] = fx::madw(gi[d1].h, wj[d2].l, hl[3 * d1 + d2]);
+                hl[3 * d1 + d2] = fx::madw(gi[d1].l, wj[d2].h, hl[3 * d1 + d2]);
+                ll[3 * d1 + d2] = fx::madw(gi[d1].l, wj[d2].l >> 5, ll[3 * d1 + d2]);
+              }
+            if (needM)
+              M = fma(phr[q * Nr + i], wph[q * Nr + j], M);
+          }
+#pragma unroll
+          for (int k = 0; k < 9; ++k)
+          {
+            int64_t const mid = hl[k] + (ll[k] >> 27) + (1ll << 26);
+            B[k / 3][k % 3] = fx::toDouble((hh[k] << 5) + (mid >> 27), 59 - sh[k / 3] - sh[3 + k % 3]);
+          }
+        }
+        for (int q = 0; q < nq && !fixed; ++q)
         {
           double const * gi = dRr + 3 * (q * Nr + i);
           double const * wj = dRc + 3 * (q * Nr + j);
@@ -683,7 +763,14 @@ pxg_status pxg_sys_assemble(pxg_sys * s, int row, int col, int const * kinds, do
   size_t const smem =
       (24 + 10 * (size_t)a.nq + 3 * (size_t)a.nq * (Nr + Nc) + Lc + (size_t)a.nq * Nr) * 8 + Lr + Lc;
   unsigned const grid = (unsigned)std::min<int64_t>(a.nelem, 152 * 8);
-  kSysAssemble<<<grid, kSysThreads, smem, st0>>>(a);
+  // The block path is bound by the FP64 pipe where a thread has several pairs of nodes (Q2: 378, 27
+  // points; velocity block of 16^3: fixed point saves 0.40 of 1.73 ms); the smaller elements'
+  // (P2: 55 pairs, 11 points) wait for memory, and the more registers cost more (16^3 x 6: 1.54 ms in
+  // FP64, 2.10 ms in fixed point).
+  if (a.pairPath && Nr * (Nr + 1) / 2 > kSysThreads)
+    kSysAssemble<true><<<grid, kSysThreads, smem, st0>>>(a);
+  else
+    kSysAssemble<false><<<grid, kSysThreads, smem, st0>>>(a);
   PXG_CUDA(cr, cudaGetLastError());
   return PXG_OK;
 }
