@@ -11,13 +11,14 @@
 // to the problems in groups: for every problem a group runs Jacobi-CG (pxg_cg.h) on
 // K u = b, forms J_p = 1/2 (u - u_t)^T M (u - u_t) and M (u - u_t), and runs the adjoint
 // CG K lambda = M (u - u_t).  Only a group's blocks wait for one another, each problem
-// stops at its own tolerance, and large problems get several blocks while small ones
-// share one, so that all groups end about together (planBatch).  Waits are bounded: when
+// stops at its own tolerance, and the groups are sized and fed so that they end about
+// together (planBatch).  Waits are bounded: when
 // one exceeds its limit the kernel sets an error flag and every block returns
 // (PXG_ERR_TIMEOUT on the host).
 // Before, all blocks went through all problems' rows with three grid barriers per
 // iteration: 70 us each, whatever the batch's size (12 + 12 cubes of 8 .. 28: 16.7 ms,
-// now 7.9 ms; 64 + 64 cubes of 8 .. 40: 108 ms, now 100 ms).
+// now 7.9 ms; 64 + 64 cubes of 8 .. 40: 108 ms, now 77 ms; 128 + 128 of 8 .. 48: 333 ms,
+// now 286 ms, and 424 ms with a group for every problem that one block is too slow for).
 // pxg_batch_adjoint captures the assembly, the persistent solve and the gradient
 // kernels in one CUDA graph and replays it.
 #include <algorithm>
@@ -25,6 +26,8 @@
 #include <cstdlib>
 #include <cmath>
 #include <cstring>
+#include <functional>
+#include <queue>
 #include <vector>
 
 #include "pxg_cg.h"
@@ -60,11 +63,13 @@ struct Problem
   int out; // place of its results
 };
 
-// a block's group (first block and size) and the group's share of the problem list
+// a block's group (first block and size) and its problems: list entries beg .. end, taken one by
+// one where queue < 0, or by the next free group of those that share the queue
 struct Group
 {
   int first, blocks;
   int beg, end;
+  int queue;
 };
 
 struct BatchResult
@@ -82,6 +87,7 @@ struct BatchDev
   ulonglong2 * part; // [3 * blocks]
   unsigned * bar;    // [blocks]
   unsigned * err;
+  int * next;     // [0] entries of the shared queue taken; [1 + block] the entry its group takes
   unsigned extra; // arrivals expected beyond a group (0; > 0 only to test the timeout path)
   double tol2;
   int maxIter;
@@ -141,11 +147,22 @@ __global__ void __launch_bounds__(kCgT, 1) kBatchSolve(BatchDev const __grid_con
   double * const vec = reinterpret_cast<double *>(dyn + kCgWarps * sizeof(CgTile));
   Group const grp = d.group[blockIdx.x];
   CgCount count;
-  for (int i = grp.beg; i < grp.end; ++i)
+  // the entry that the group takes next; the other blocks learn it past the barrier, which also
+  // keeps the next problem's sums from the words of this one's last
+  auto take = [&](int i) {
+    CgArgs g{};
+    g.bar = d.bar + grp.first, g.err = d.err, g.block0 = grp.first, g.blocks = grp.blocks, g.extra = d.extra;
+    if (grp.queue >= 0 && g.rank() == 0 && threadIdx.x == 0)
+      __stcg(d.next + 1 + grp.first, grp.beg + atomicAdd(d.next, 1));
+    if (!cgBarrier(g, sh, ++count.epoch))
+      return grp.end;
+    return grp.queue >= 0 ? __ldcg(d.next + 1 + grp.first) : i;
+  };
+  for (int i = take(grp.beg); i < grp.end; i = take(i + 1))
   {
     Problem const pr = d.prob[i];
     SysDev const & s = d.sys[pr.sys];
-    bool const traced = d.trace && grp.first == 0 && i == grp.beg;
+    bool const traced = d.trace && grp.first == 0 && i == 0;
     CgArgs g{s.rp, s.ci, s.K, s.b, s.u, s.p, s.r, s.z, s.dinv, d.part + 3 * grp.first, d.bar + grp.first, d.err,
              pr.row0, pr.rows, (unsigned)grp.first, (unsigned)grp.blocks, d.extra, d.tol2, d.maxIter, d.cap, 1,
              traced ? d.trace : nullptr, d.traceCap / 2};
@@ -156,18 +173,20 @@ __global__ void __launch_bounds__(kCgT, 1) kBatchSolve(BatchDev const __grid_con
     cgLanes(nr, mean, [&](auto lanes) {
       ok = batchProblem<decltype(lanes)::value>(d, s, d.res[pr.out], g, sh, tiles, vec, r0, nr, count);
     });
-    // the next problem's sums reuse the words of this one's last
-    if (!ok || (i + 1 < grp.end && !cgBarrier(g, sh, ++count.epoch)))
+    if (!ok)
       return;
   }
 }
 
-// Deals `blocks` blocks to the problems so that the groups end together, by the time an iteration
-// takes: a block's FP64 operations (0.33 ns per entry of its rows, eight more per row) and the
-// exchanges (11 us in a group of several blocks, 4 us in one block; both measured here), and
-// iterations in proportion to the cube root of the rows.  The least end time for which the blocks
-// suffice is found by bisection: a problem that one block cannot solve in that time gets a group
-// of its own; the others go, longest first, to the single block with the least work so far.
+// Deals `blocks` blocks to the problems so that all end together, by the time an iteration takes: a
+// block's FP64 operations (0.33 ns per entry of its rows, eight more per row) and the exchanges (4
+// us in one block, 8 us in a few, 12 us in all), and iterations in proportion to the cube root of
+// the rows.  Two kinds of plan, the shorter one is taken:
+//  - few problems: the least end time for which the blocks suffice (bisection); a problem that
+//    one block cannot solve in that time gets a group of its own, the others go, longest first,
+//    to single blocks as these become free;
+//  - many problems: groups of one size, which take the problems, longest first, as they become
+//    free (groups of whole blocks per problem waste up to half of the last block each).
 // Returns the largest share of rows.
 int64_t planBatch(std::vector<Problem> & prob, std::vector<double> const & entries, int blocks,
                   std::vector<Group> & group)
@@ -175,6 +194,7 @@ int64_t planBatch(std::vector<Problem> & prob, std::vector<double> const & entri
   size_t const n = prob.size();
   std::vector<double> its(n), work(n);
   double lo = 0., hi = 0.;
+  auto exchange = [](int b) { return b == 1 ? 4. : 7.5 + 0.6 * std::log2((double)b); };
   for (size_t p = 0; p < n; ++p)
   {
     its[p] = std::cbrt((double)prob[p].rows);
@@ -204,43 +224,59 @@ int64_t planBatch(std::vector<Problem> & prob, std::vector<double> const & entri
     }
     (many + (int64_t)std::ceil(single / t) <= blocks ? hi : lo) = t;
   }
-  std::vector<size_t> order, alone;
-  int used = 0;
+  std::vector<size_t> order(n);
   for (size_t p = 0; p < n; ++p)
-    if (need(p, hi) == 1)
-      alone.push_back(p);
-  std::sort(alone.begin(), alone.end(),
-            [&](size_t a, size_t b) { return its[a] * (work[a] + 4.) > its[b] * (work[b] + 4.); });
-  group.assign(blocks, Group{0, 1, 0, 0});
+    order[p] = p;
+  std::sort(order.begin(), order.end(), [&](size_t a, size_t b) { return its[a] * work[a] > its[b] * work[b]; });
+  // groups of one size: the end time of a greedy deal, longest first
+  int size = 0;
+  for (int b = 1; b <= blocks / 2; b = b < 4 ? b + 1 : b + b / 4)
+  {
+    std::priority_queue<double, std::vector<double>, std::greater<double>> busy;
+    for (int g = 0; g < blocks / b; ++g)
+      busy.push(0.);
+    double end = 0.;
+    for (size_t p : order)
+    {
+      double const t = busy.top() + its[p] * (work[p] / b + exchange(b));
+      busy.pop();
+      busy.push(t);
+      end = std::max(end, t);
+    }
+    if (end < hi)
+    {
+      hi = end;
+      size = b;
+    }
+  }
+  group.assign(blocks, Group{0, 1, 0, 0, -1});
   std::vector<Problem> list;
   int64_t share = 0;
-  for (size_t p = 0; p < n; ++p)
-  {
-    int const b = need(p, hi);
-    if (b == 1)
-      continue;
-    for (int k = 0; k < b; ++k)
-      group[used + k] = Group{used, b, (int)list.size(), (int)list.size() + 1};
-    list.push_back(prob[p]);
-    used += b;
-    share = std::max(share, (prob[p].rows + b - 1) / b);
-  }
-  std::vector<std::vector<size_t>> bin(blocks - used);
-  std::vector<double> load(bin.size(), 0.);
-  for (size_t p : alone)
-  {
-    size_t const k = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
-    bin[k].push_back(p);
-    load[k] += its[p] * (work[p] + 4.);
-    share = std::max(share, prob[p].rows);
-  }
-  for (size_t k = 0; k < bin.size(); ++k)
-  {
-    int const beg = (int)list.size();
-    for (size_t p : bin[k])
+  int used = 0;
+  if (size == 0)
+    for (size_t p : order)
+    {
+      int const b = need(p, hi);
+      if (b == 1)
+        continue;
+      for (int k = 0; k < b; ++k)
+        group[used + k] = Group{used, b, (int)list.size(), (int)list.size() + 1, -1};
       list.push_back(prob[p]);
-    group[used + k] = Group{used + (int)k, 1, beg, (int)list.size()};
-  }
+      used += b;
+      share = std::max(share, (prob[p].rows + b - 1) / b);
+    }
+  int const b = std::max(size, 1), beg = (int)list.size();
+  for (size_t p : order)
+    if (size > 0 || need(p, hi) == 1)
+    {
+      list.push_back(prob[p]);
+      share = std::max(share, (prob[p].rows + b - 1) / b);
+    }
+  for (; used + b <= blocks; used += b)
+    for (int k = 0; k < b; ++k)
+      group[used + k] = Group{used, b, beg, (int)list.size(), 0};
+  for (; used < blocks; ++used)
+    group[used] = Group{used, 1, 0, 0, -1};
   prob = list;
   return share;
 }
@@ -363,7 +399,7 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
     PXG_CUDA(c0, S.prob.alloc(nprob * sizeof(Problem)));
     PXG_CUDA(c0, S.group.alloc(blocks * sizeof(Group)));
     PXG_CUDA(c0, S.part.alloc(6 * blocks));
-    PXG_CUDA(c0, S.bar.alloc(blocks + 1)); // and the error flag
+    PXG_CUDA(c0, S.bar.alloc(2 * blocks + 2)); // and the error flag, the queue
     S.nprob = nprob;
   }
   PXG_CUDA(c0, cudaMemcpy(S.prob.p, prob.data(), prob.size() * sizeof(Problem), cudaMemcpyHostToDevice));
@@ -382,6 +418,7 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
   d.part = reinterpret_cast<ulonglong2 *>(S.part.p);
   d.bar = S.bar.p;
   d.err = S.bar.p + blocks;
+  d.next = reinterpret_cast<int *>(S.bar.p) + blocks + 1;
   d.tol2 = rtol * rtol;
   d.maxIter = max_iter;
   d.cap = cap;
@@ -418,7 +455,7 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
         return e;
     }
     PXG_CUDA(c0, cudaMemsetAsync(S.part.p, 0, 6 * blocks * sizeof(double), rs)); // no sum has the tag 0
-    PXG_CUDA(c0, cudaMemsetAsync(S.bar.p, 0, (blocks + 1) * sizeof(unsigned), rs));
+    PXG_CUDA(c0, cudaMemsetAsync(S.bar.p, 0, (2 * blocks + 2) * sizeof(unsigned), rs));
     void * args[] = {&d};
     PXG_CUDA(c0, cudaLaunchCooperativeKernel((void const *)kBatchSolve, dim3(blocks), dim3(kCgT), args, smem, rs));
     for (int i = 0; i < nctx; ++i)

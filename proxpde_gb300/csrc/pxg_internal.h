@@ -250,7 +250,7 @@ struct BatchShared
   int nprob = 0;
   pxg::DevBuf<unsigned char> res, prob, group; // results, problem list, the blocks' groups
   pxg::DevBuf<double> part;                    // the blocks' sums
-  pxg::DevBuf<unsigned> bar;                   // the groups' arrivals, the error flag
+  pxg::DevBuf<unsigned> bar;                   // the groups' arrivals, the error flag, the queue
   cudaGraphExec_t exec = nullptr;
   GraphKey key;
   ~BatchShared()
