@@ -3,8 +3,8 @@
 
 Workload (one step): the perturbed 128^3 Q1-hex unit cube (2,097,152 elements,
 2,146,689 nodes; interior nodes moved by a seeded U(-0.2h, 0.2h) per coordinate),
-per-element diffusivity k_e = exp(N(0,1)), 2x2x2 Gauss quadrature, computed in FP64
-arithmetic (IEEE binary64, as the reference): stiffness (AssemblyStiffnessFE with the
+per-element diffusivity k_e = exp(N(0,1)), 2x2x2 Gauss quadrature, at least at FP64
+precision (64-bit fixed point or IEEE binary64 values, binary64 sums): stiffness (AssemblyStiffnessFE with the
 P0 coefficient) and mass (AssemblyMass(1)) CSR values plus the load vector of
 f = sin(pi x) sin(pi y) sin(pi z), assembled in one fused pass on the device-resident
 structural pattern, followed by closeMatrix's prune check of both matrices.  The mesh,
@@ -15,9 +15,8 @@ synthetic (seeded), not a dataset.
 
 Prints one JSON line.  Under torchrun (N > 1) every rank assembles its own replica
 (weak scaling) and rank 0 prints the aggregate over ranks (max time over ranks).
-Besides the contract's keys: `roofline.fp64` (the FP64 pipe, the bound the FP64
-kernel meets: FP64 instructions per second against the FMA rate measured live by
-pxg_fp64_rate), `dfl` (the same workload with the opt-in double-float kernels and
+Besides the contract's keys: `roofline.fp64` (the FP64 pipe's share: its instructions per
+second, conversions included, against the FMA rate measured live by pxg_fp64_rate), `dfl` (the same workload with the opt-in double-float kernels and
 their largest entrywise deviation from the FP64 result), `e2e.host` (the GPU's NUMA
 node and the CPUs the host-buffer leg ran on), `configs` (P1 16^3 x 6, P2 64^3 x 6,
 Q2 48^3; with P2, the L2 reduction rate its scatter meets, live from pxg_red_rate),
@@ -53,7 +52,7 @@ def peaks():
     return 6800.0, "fallback"
 
 
-PROFILE = "kAssembleQ1F64_q1hex96.md"
+PROFILE = "kAssembleQ1Fx_q1hex96.md"
 
 
 def profile_figure(key, name=PROFILE):
@@ -241,9 +240,9 @@ def measure_configs(peak_gbs, reps=5):
     out = {}
     cases = (("p1tet_16", L.P1TET, meshgen.cube_tet6, 16, 0.0, None, 1, {"kind": 1, "fn": L.FN_CONST, "coef": 1.0},
               "kAssembleTet64<P1>"),
-             ("p2tet_64", L.P2TET, meshgen.cube_tet6, 64, 0.15, 0.5, 2, None, "kAssembleTet64<P2>"),
+             ("p2tet_64", L.P2TET, meshgen.cube_tet6, 64, 0.15, 0.5, 2, None, "kAssembleP2Group"),
              ("q2hex_48", L.Q2HEX, meshgen.cube_hex, 48, 0.2, 1.0, 2, {"kind": 1, "fn": L.FN_SIN3, "coef": 1.0},
-              "kAssembleQ2F64"))
+              "kAssembleQ2Fx"))
     for name, t, gen, n, alpha, sigma, nmat, rhs, kern in cases:
         xyz, conn = gen(n)
         if alpha:
@@ -575,12 +574,12 @@ def main():
     tpe = traffic_per_element()
     roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "traffic": tpe * E if tpe else None, "traffic_source": "ncu 96^3 capture scaled by elements",
-            "peak_source": which, "kernel": "kAssembleQ1F64 (+memset of K, M, b)",
+            "peak_source": which, "kernel": "kAssembleQ1Fx (+memset of K, M, b)",
             "kernel_ms": asm_ms, "algorithmic_bytes": alg}
-    # the bound the FP64 kernel meets: the FP64 pipe.  FP64 instructions per element from
-    # ncu (96^3 capture: DFMA + DMUL + DADD thread instructions / elements) times the
-    # elements over the event-timed launch, against the FMA rate measured now on this
-    # GPU; the launch time includes the memsets, so the fraction is a lower bound
+    # the FP64 pipe's share: FP64 instructions per element from ncu (96^3 capture: thread
+    # instructions of the FP64 pipe, conversions included, / elements) times the elements
+    # over the event-timed launch, against the FMA rate measured now on this GPU; the
+    # launch time includes the zeroing, so the fraction is a lower bound
     from proxpde_gb300._lib import fp64_rate
 
     rate, rate_ms = fp64_rate(dev)
@@ -719,7 +718,8 @@ def main():
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64",
-            "arithmetic": "IEEE binary64 throughout (geometry, local matrices, sums, reductions); FP64-pipe bound",
+            "arithmetic": "element values in 64-bit fixed point (62-bit significand; IEEE binary64 where an element's values do "
+                          "not share a range), binary64 sums and reductions",
             "data": "synthetic (seeded perturbed cube)",
             "config": {"workload": f"q1hex perturbed {n}^3: K(k_e)+M+rhs sin3, fused pass + prune check",
                        "elements": E, "nodes": nn, "ndof": ndof, "nnz": nnz, "pruned": list(pruned), "tuning": tuning,
@@ -727,7 +727,7 @@ def main():
                        "setup_s": setup_s, "parallelism": f"replicas x{world}"},
             "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "clocks": clocks, "dfl": dfl, "widened": widened,
             "configs": configs,
-            # per step: the zeroing of K, M and b (kZeroOutputs), the assembly (kAssembleQ1F64)
+            # per step: the zeroing of K, M and b (kZeroOutputs), the assembly (kAssembleQ1Fx)
             # and the two prune counts (kPruneCount)
             "gpu_launches": 4 * args.steps, "adjoint": adjoint, "batched": batched,
         }

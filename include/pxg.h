@@ -288,7 +288,9 @@ pxg_status pxg_prune_count_device(pxg_ctx * ctx, const double * vals, int64_t * 
 pxg_status pxg_set_scatter(pxg_ctx * ctx, int scatter, int threads);
 /* Arithmetic of the element kernels.  The reference computes geometry, local matrices
  * and sums in double (FVec/FMat, include/def.hpp:157-160); PXG_ARITH_FP64, the
- * default, does the same: every value is formed by IEEE binary64 operations.
+ * default, is at least as precise: an element's values are formed in 64-bit fixed point
+ * with a common exponent (62-bit significand) or, where they do not share a range, by
+ * IEEE binary64 operations, and summed as binary64.
  * PXG_ARITH_DFL is an opt-in alternative with a narrower significand: the geometry and
  * the local matrices run as unevaluated pairs of floats (about 48 bits) on the FP32
  * pipes, and only the coordinate differences, the final sums and the reductions into
@@ -339,9 +341,9 @@ pxg_status pxg_memcpy(pxg_ctx * ctx, void * dst, const void * src, uint64_t byte
  * proxpde solves with UmfPackLU (include/sparse_matrix.hpp:44, include/solver.hpp:65);
  * this plain device CG is the engine's solver.  Returns PXG_ERR_NOT_CONVERGED (x holds
  * the last iterate) when the tolerance is not met.  The solve runs on a stream of the
- * context ordered after `stream`, replays its iterations as a CUDA graph and reads its
- * convergence flag on the host, so it returns with the solve complete and cannot be
- * captured into the caller's graph. */
+ * context ordered after `stream`, as one persistent cooperative kernel, and is waited for
+ * on the host, so it returns with the solve complete and cannot be captured into the
+ * caller's graph.  PXG_ERR_TIMEOUT if a bounded wait between its blocks ran out. */
 pxg_status pxg_cg(pxg_ctx * ctx, const int32_t * row_ptr, const int32_t * col_idx,
                   const double * vals, int64_t n, const double * b, double * x, double rtol,
                   int max_iter, int * iters, double * rel_res, void * stream);
@@ -377,7 +379,7 @@ pxg_status pxg_batch_set(pxg_ctx * ctx, const int64_t * elem_offsets, int64_t np
  * captured once in a CUDA graph and replayed while the arguments stay the same.
  * u_targets[i]: device, ndof of ctxs[i]; grads[i]: device, nelem of ctxs[i];
  * losses: host, one per problem (ctxs[0]'s problems first); iters: the largest CG
- * iteration count.  PXG_ERR_TIMEOUT if a grid barrier wait of the persistent kernel
+ * iteration count.  PXG_ERR_TIMEOUT if a wait between blocks of the persistent kernel
  * ran out (the context stays usable). */
 pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, const pxg_rhs_op * rhs,
                              const double * const * u_targets, double rtol, int max_iter,

@@ -1,10 +1,8 @@
-// Q1 hexahedron element in FP64 arithmetic, one thread per element, written for
-// GB300's FP64 rate (2 FP64 operations per clock per SM, 1/64 of FP32): every value
-// the element produces is computed with IEEE binary64 operations, and the kernel is
-// bound by the FP64 pipe, so its design goal is the fewest FP64 instructions per
-// element.  It computes what proxpde's element loop computes for a Q1 hexahedron with
-// the 2x2x2 Gauss rule (include/builder.hpp:53-153): CurFE::reinit (include/curfe.hpp:
-// 50-103), AssemblyStiffness(FE) / AssemblyScalarMass / AssemblyMassFE
+// Q1 hexahedron element in FP64 arithmetic by one thread: the elements whose values the
+// fixed-point form (pxg_q1fx.cu) does not take.  It uses few FP64 operations (1,233),
+// as GB300 does 2 of them per clock per SM, 1/64 of FP32.  It computes what proxpde's
+// element loop computes for a Q1 hexahedron with the 2x2x2 Gauss rule
+// (include/builder.hpp:53-153): CurFE::reinit (include/curfe.hpp:50-103), AssemblyStiffness(FE) / AssemblyScalarMass / AssemblyMassFE
 // (include/assembly_lhs.hpp:52-109, 207-221, 262-277), AssemblyRhsAnalytic and
 // AssemblyS2SProjection (include/assembly_rhs.hpp:61-88, 130-159), the Dirichlet
 // condensation (builder.hpp:76-124), and adds the result into the CSR values and the

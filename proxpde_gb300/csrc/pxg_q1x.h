@@ -1,7 +1,7 @@
 // Q1 hexahedron element in 64-bit fixed point (pxg_fx.h): the steps of an element's
 // geometry, stiffness and mass tables, entries and sine load, as functions of one
 // coordinate, one quadrature point or one table, which the kernel deals to its warps.  The
-// same quantities as the FP64 form computes (pxg_q1f64.cu, whose notation this keeps), in
+// same quantities as the FP64 form computes (pxg_q1f64.h, whose notation this keeps), in
 // a shape that suits the format: determinants from the Jacobian's cofactors (the Gram
 // determinant, their square, would double the lost bits) and contractions on moments,
 // sums and differences of the points' values, as additions cost little and products much.

@@ -5,8 +5,8 @@
 // 50-103), AssemblyStiffness(FE) / AssemblyScalarMass / AssemblyMassFE
 // (include/assembly_lhs.hpp:52-109, 207-221, 262-277), AssemblyRhsAnalytic and
 // AssemblyS2SProjection (include/assembly_rhs.hpp:61-88, 130-159) and the Dirichlet
-// condensation (builder.hpp:76-124), in IEEE binary64, with FP64 reductions into the
-// CSR values and the load vector.
+// condensation (builder.hpp:76-124), with FP64 reductions into the CSR values and the
+// load vector.
 //
 // The Q2 basis is a tensor product of the 1D functions l_0 = x(x-1)/2, l_1 = x(x+1)/2,
 // l_2 = 1 - x^2 (src/reffe.cpp:374-383), and the rule a tensor product of the 3-point
