@@ -74,6 +74,7 @@ struct SysArgs
   int nops;
   int kind[4];
   double coef[4];
+  int needR, needC; // the operators read the row / column functions' gradients
   int pairPath; // one space, stiffness / tensor stiffness / mass only: the block path
   int32_t const * rowPtr;
   int32_t const * colIdx;
@@ -159,13 +160,24 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
     if (threadIdx.x < 6)
       top[threadIdx.x] = 0;
     __syncthreads();
+    // J into the place of J^-1 (a coordinate per thread), then adj(J), det and the weights, then the
+    // quotients: one warp doing all of a point's 210 FP64 operations in a row kept the others waiting
+    for (int k = threadIdx.x; k < 3 * nq; k += blockDim.x)
+    {
+      int const q = k / 3, r = k % 3;
+      double J[3] = {};
+      for (int v = 0; v < nv; ++v)
+        for (int c = 0; c < 3; ++c)
+          J[c] += X[3 * v + r] * dV[(q * nv + v) * 3 + c];
+      for (int c = 0; c < 3; ++c)
+        Jinv[9 * q + 3 * r + c] = J[c];
+    }
+    __syncthreads();
     for (int q = threadIdx.x; q < nq; q += blockDim.x)
     {
-      double J[3][3] = {};
-      for (int v = 0; v < nv; ++v)
-        for (int r = 0; r < 3; ++r)
-          for (int c = 0; c < 3; ++c)
-            J[r][c] += X[3 * v + r] * dV[(q * nv + v) * 3 + c];
+      double J[3][3];
+      for (int k = 0; k < 9; ++k)
+        J[k / 3][k % 3] = Jinv[9 * q + k];
       double C[3][3]; // adj(J)
       C[0][0] = J[1][1] * J[2][2] - J[1][2] * J[2][1];
       C[0][1] = J[0][2] * J[2][1] - J[0][1] * J[2][2];
@@ -178,19 +190,23 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
       C[2][2] = J[0][0] * J[1][1] - J[0][1] * J[1][0];
       double const det = J[0][0] * C[0][0] + J[0][1] * C[1][0] + J[0][2] * C[2][0];
       for (int k = 0; k < 9; ++k)
-        Jinv[9 * q + k] = C[k / 3][k % 3] / det;
+        Jinv[9 * q + k] = C[k / 3][k % 3];
+      wph[q] = det; // free until the weighted functions
       JxW[q] = fabs(det) * W[q];
     }
     __syncthreads();
-    // mapped gradients: dphi_c = sum_k dphiRef_k Jinv[k][c]
-    for (int k = threadIdx.x; k < nq * Nr; k += blockDim.x)
+    for (int k = threadIdx.x; k < 9 * nq; k += blockDim.x)
+      Jinv[k] /= wph[k / 9];
+    __syncthreads();
+    // mapped gradients where an operator reads them: dphi_c = sum_k dphiRef_k Jinv[k][c]
+    for (int k = threadIdx.x; k < nq * Nr && a.needR; k += blockDim.x)
     {
       int const q = k / Nr;
       double const * g = dpr + 3 * k;
       for (int c = 0; c < 3; ++c)
         dRr[3 * k + c] = g[0] * Jinv[9 * q + c] + g[1] * Jinv[9 * q + 3 + c] + g[2] * Jinv[9 * q + 6 + c];
     }
-    for (int k = threadIdx.x; k < nq * Nc; k += blockDim.x)
+    for (int k = threadIdx.x; k < nq * Nc && a.needC; k += blockDim.x)
     {
       int const q = k / Nc;
       double const * g = dpc + 3 * k;
@@ -353,12 +369,9 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
                 }
                 break;
               case PXG_OP_TENSOR_STIFFNESS:
-              {
-                double const dk = d1 == d2 ? K : 0.;
-                v += c * (dk + B[d1][d2]);
-                vt += c * (dk + B[d2][d1]);
+                v += c * (d1 == d2 ? K + B[d1][d2] : B[d1][d2]);
+                vt += c * (d1 == d2 ? K + B[d1][d2] : B[d2][d1]);
                 break;
-              }
               case PXG_OP_MASS:
                 if (d1 == d2)
                 {
@@ -385,7 +398,7 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
     {
       double const w = JxW[k / Nr];
       wph[k] = w * phr[k];
-      if (!plain)
+      if (!plain && a.needR)
         for (int c = 0; c < 3; ++c)
           dRr[3 * k + c] *= w;
     }
@@ -759,6 +772,13 @@ pxg_status pxg_sys_assemble(pxg_sys * s, int row, int col, int const * kinds, do
   for (int k = 0; k < nops; ++k)
     a.pairPath = a.pairPath && (kinds[k] == PXG_OP_STIFFNESS || kinds[k] == PXG_OP_TENSOR_STIFFNESS ||
                                 kinds[k] == PXG_OP_MASS);
+  // (the block path takes its weighted gradients from the row functions')
+  for (int k = 0; k < nops; ++k)
+  {
+    bool const stiff = kinds[k] == PXG_OP_STIFFNESS || kinds[k] == PXG_OP_TENSOR_STIFFNESS;
+    a.needR = a.needR || stiff || kinds[k] == PXG_OP_GRAD || a.pairPath;
+    a.needC = a.needC || (stiff && !a.pairPath) || kinds[k] == PXG_OP_DIV;
+  }
   int const Lr = Nr * a.dr, Lc = Nc * a.dc;
   size_t const smem =
       (24 + 10 * (size_t)a.nq + 3 * (size_t)a.nq * (Nr + Nc) + Lc + (size_t)a.nq * Nr) * 8 + Lr + Lc;
