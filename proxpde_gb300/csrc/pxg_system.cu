@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kSysThreads) kSysAssemble(SysArgs a)
       // The pattern couples all components of two nodes or none, so a node's rows have the same
       // columns and each component's follow the one before: one search per ordered pair of nodes
       // gives its nine positions (a search per entry, 18 of nine dependent loads per pair:
-      // 2.33 ms for the three blocks of 16^3 Q2-Q1, now 1.73 ms)
+      // 2.33 ms for the three blocks of 16^3 Q2-Q1, 1.73 ms with this)
       if (a.dr > 1)
         for (int i = threadIdx.x; i < Nr; i += blockDim.x)
         {
@@ -784,7 +784,8 @@ pxg_status pxg_sys_assemble(pxg_sys * s, int row, int col, int const * kinds, do
       (24 + 10 * (size_t)a.nq + 3 * (size_t)a.nq * (Nr + Nc) + Lc + (size_t)a.nq * Nr) * 8 + Lr + Lc;
   unsigned const grid = (unsigned)std::min<int64_t>(a.nelem, 152 * 8);
   // The block path is bound by the FP64 pipe where a thread has several pairs of nodes (Q2: 378, 27
-  // points; velocity block of 16^3: fixed point saves 0.40 of 1.73 ms); the smaller elements'
+  // points; the three blocks of 16^3 Q2-Q1: 1.73 ms in FP64, 1.34 ms in fixed point, 1.22 ms with
+  // the geometry spread over the block); the smaller elements'
   // (P2: 55 pairs, 11 points) wait for memory, and the more registers cost more (16^3 x 6: 1.54 ms in
   // FP64, 2.10 ms in fixed point).
   if (a.pairPath && Nr * (Nr + 1) / 2 > kSysThreads)
