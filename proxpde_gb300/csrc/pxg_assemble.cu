@@ -1858,9 +1858,10 @@ void launchAssembleTet64(AsmArgs const & args, cudaStream_t s, int threads)
     if (blocks > 0)
       launchElemKernel(kern, blocks, nt, 0, s, a);
   };
-  // the usual pair without Dirichlet conditions has its own instance: the others' branches
-  // cost its registers (64^3 x 6, K + M: 1.05 ms against 1.12)
-  bool const plain = a.fold.simple && a.fold.needK && a.fold.needM && !a.fold.same && !(a.bcMask && a.fold.bc);
+  // the usual pair without Dirichlet conditions (of the operators or of the load) has its own
+  // instance: the others' branches cost its registers (64^3 x 6, K + M: 1.05 ms against 1.12)
+  bool const plain = a.fold.simple && a.fold.needK && a.fold.needM && !a.fold.same &&
+                     !(a.bcMask && (a.fold.bc || (a.rkind && a.rbc)));
   if (threads == 64)
     return plain ? go(kAssembleTet64<T, 64, true>, 64) : go(kAssembleTet64<T, 64, false>, 64);
   if (threads == 256)
