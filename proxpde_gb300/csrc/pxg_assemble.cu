@@ -976,31 +976,6 @@ __global__ void __launch_bounds__(NT) kAssembleTet(AsmArgs a)
 // folded into |det J|).  P2 tetrahedron: src/reffe.cpp:542-642, vertices then the
 // edges 01 12 20 03 13 23.
 
-// P1 stiffness K_ij = ks C_i . C_j / |det J| (C_1..3 the cofactor vectors, C_0 minus their
-// sum) and |det J| in 64-bit fixed point: 33 FP64 instructions, nearly all conversions, where
-// the FP64 form has about 90.  False for an element the format refuses.
-__device__ __forceinline__ bool p1Fixed(double const (&J)[3][3], double ks, double (&K)[4][4], double & adet)
-{
-  int64_t km, G[6];
-  int ke, eK;
-  bool const okK = fx::decompose(ks, km, ke);
-  if (!tetTensor(J, okK && abs(ke) < 300, km, ke, G, eK, adet))
-    return false;
-  int64_t const Gs[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
-  int64_t cs[3];
-#pragma unroll
-  for (int b = 0; b < 3; ++b)
-  {
-    cs[b] = Gs[0][b] + Gs[1][b] + Gs[2][b];
-    K[0][b + 1] = fx::toDouble(-cs[b], eK);
-#pragma unroll
-    for (int a = 0; a <= b; ++a)
-      K[a + 1][b + 1] = fx::toDouble(Gs[a][b], eK);
-  }
-  K[0][0] = fx::toDouble(cs[0] + cs[1] + cs[2], eK);
-  return true;
-}
-
 // PLAIN: one operator's stiffness and the other's mass, no Dirichlet conditions
 template <int T, int NT, bool PLAIN>
 __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_constant__ a)
@@ -1057,9 +1032,17 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_consta
   bool const both = PLAIN || (needK && needM && !a.fold.same);
   bool const fast = PLAIN || (a.fold.simple && !bcWarp && (T == P1TET || both));
   double const ksf = foldK ? (k0 ? ks0 : ks1) : 1.0;
-  double G[6], K1[4][4], adet;
-  // P1: with G carrying the sum of the Tet4 weights (the reference volume 1/6)
-  bool const fixed = T == P1TET && p1Fixed(J, ksf * cP1Ws, K1, adet);
+  double G[6], adet;
+  // P1 in fixed point (pxg_tetfx.h): 16 conversions instead of about 75 FP64 operations, with G
+  // carrying the sum of the Tet4 weights (the reference volume 1/6)
+  bool fixed = false;
+  if constexpr (T == P1TET)
+  {
+    int64_t km;
+    int ke;
+    bool const okK = fx::decompose(ksf * cP1Ws, km, ke);
+    fixed = tetx::tetGram(J, okK && abs(ke) < 300, km, ke, G, adet);
+  }
   if (!fixed)
   {
     double A[3][3];
@@ -1078,24 +1061,25 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_consta
     else if (fast)
       gs *= 1.0 / 30.0; // s'_(a+1)(b+1) = G_ab of the barycentric form
     gram(A, gs, G);
-    // P1: grad phi_i |det J| are the adjugate rows (i = 1..3) and minus their sum (i = 0),
-    // so K_ij = k / (6 |det J|) A_i . A_j reads the Gram entries of the adjugate directly:
-    // K_(a+1)(b+1) = G_ab, K_0(b+1) = -sum_a G_ab, K_00 = sum_ab G_ab
-    if constexpr (T == P1TET)
+  }
+  // P1: grad phi_i |det J| are the adjugate rows (i = 1..3) and minus their sum (i = 0),
+  // so K_ij = k / (6 |det J|) A_i . A_j reads the Gram entries of the adjugate directly:
+  // K_(a+1)(b+1) = G_ab, K_0(b+1) = -sum_a G_ab, K_00 = sum_ab G_ab
+  double K1[4][4];
+  if constexpr (T == P1TET)
+  {
+    double const Gs[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
+    double cs[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
     {
-      double const Gs[3][3] = {{G[0], G[3], G[4]}, {G[3], G[1], G[5]}, {G[4], G[5], G[2]}};
-      double cs[3];
+      cs[b] = Gs[0][b] + (Gs[1][b] + Gs[2][b]);
+      K1[0][b + 1] = -cs[b];
 #pragma unroll
-      for (int b = 0; b < 3; ++b)
-      {
-        cs[b] = Gs[0][b] + (Gs[1][b] + Gs[2][b]);
-        K1[0][b + 1] = -cs[b];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-          K1[a + 1][b + 1] = Gs[a][b];
-      }
-      K1[0][0] = cs[0] + (cs[1] + cs[2]);
+      for (int a = 0; a < 3; ++a)
+        K1[a + 1][b + 1] = Gs[a][b];
     }
+    K1[0][0] = cs[0] + (cs[1] + cs[2]);
   }
   double const am = foldM ? (m0 ? ms0 : ms1) * adet : adet;
 

@@ -1,6 +1,6 @@
-// P2 tetrahedra in FP64 with the warp-group scatter (pxg_group.cu), a block of two warps per
-// group of 32 elements.  Warp 0 forms the elements' values, one element per lane, in
-// barycentric form (pxg_p2bary.h) and leaves them in shared memory, while warp 1 copies the
+// P2 tetrahedra with the warp-group scatter (pxg_group.cu), a block of two warps per group of 32
+// elements.  Warp 0 forms the elements' values, one element per lane, from the geometry in fixed
+// point (pxg_tetfx.h) and in barycentric form (pxg_p2bary.h), and leaves them in shared memory, while warp 1 copies the
 // group's contribution codes there; then both sum the group's distinct positions and add
 // each sum once.  Shared memory (22.5 KB per group) limits an SM to ten groups: with one warp
 // per group its ten warps left the map's loads and the additions' latency exposed
@@ -32,14 +32,13 @@ __device__ __forceinline__ void red(double * p, double v) { atomicAdd(p, v); }
 
 // s (4 x 4, zero row sums) and E_ab = s_aa + s_bb + s_ab of the six edges from the Gram
 // entries of vertices 1..3
-template <class V>
-__device__ __forceinline__ void gramRows(V const (&G)[6], V (&s)[4][4], V (&E)[6])
+__device__ __forceinline__ void gramRows(double const (&G)[6], double (&s)[4][4], double (&E)[6])
 {
   s[1][1] = G[0], s[2][2] = G[1], s[3][3] = G[2];
   s[1][2] = s[2][1] = G[3];
   s[1][3] = s[3][1] = G[4];
   s[2][3] = s[3][2] = G[5];
-  V const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
+  double const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
   s[0][1] = s[1][0] = -c1;
   s[0][2] = s[2][0] = -c2;
   s[0][3] = s[3][0] = -c3;
@@ -128,25 +127,14 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         for (int k = 0; k < 3; ++k)
           J[r][k] = X[k + 1][r] - X[0][r];
       double const ks = a.fold.coefK ? a.fold.sK * kfac : a.fold.sK;
-      // the entries are integer combinations of s'_(a+1)(b+1) = G_ab, the Gram matrix of the
-      // cofactors times k / (30 |det J|): km carries 16 / 30
-      int64_t km, Gx[6];
-      int ke, eG;
+      // s'_(a+1)(b+1) = G_ab, the Gram matrix of the cofactors times k / (30 |det J|), in fixed
+      // point (16 conversions for about 75 FP64 operations): km carries 16 / 30
+      double G[6];
+      int64_t km;
+      int ke;
       bool const okK = fx::decompose(ks, km, ke);
-      km = q1x::shl(fx::mulc(fx::cst(0x4444444444444444ll), km), 1);
-      if (tetTensor(J, okK && abs(ke) < 300, km, ke - 4, Gx, eG, adet))
-      {
-        if (needK)
-        {
-          int64_t s[4][4], E[6];
-          gramRows(Gx, s, E);
-          p2ForPairs<0, 0>([&](auto I, auto Jj) {
-            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-            at(p2UpperIdx(i, j), lane) = fx::toDouble(p2StiffFixed<i, j>(s, E), eG);
-          });
-        }
-      }
-      else
+      km = (int64_t)((uint64_t)fx::mulc(fx::cst(0x4444444444444444ll), km) << 1);
+      if (!tetx::tetGram(J, okK && abs(ke) < 300, km, ke - 4, G, adet))
       {
         double A[3][3];
         adet = fabs(adj3(J, A));
@@ -156,17 +144,16 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
         double const t = fma(-adet, ra, 1.0);
         ra = fma(ra, fma(t, t, t), ra);
-        double G[6];
         gram(A, ks * ra * (1.0 / 30.0), G);
-        if (needK)
-        {
-          double s[4][4], E[6];
-          gramRows(G, s, E);
-          p2ForPairs<0, 0>([&](auto I, auto Jj) {
-            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-            at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
-          });
-        }
+      }
+      if (needK)
+      {
+        double s[4][4], E[6];
+        gramRows(G, s, E);
+        p2ForPairs<0, 0>([&](auto I, auto Jj) {
+          constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+          at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
+        });
       }
       if (needM)
       {
