@@ -80,8 +80,8 @@ PXG_HD double bitsDouble(int64_t x)
 
 // biased exponent field of a double
 PXG_HD int expoField(double x) { return (hi32(doubleBits(x)) >> 20) & 0x7ff; }
-// x 2^k by an addition to the exponent field; the caller keeps the result normal.
-// Zeros (and subnormals, which no caller passes) stay zero.
+// x 2^k by an addition to the exponent field; the caller keeps the result normal (an
+// unchecked sum wraps into the sign).  Zeros (and subnormals) stay zero.
 PXG_HD double scaleExp(double x, int k)
 {
   int64_t const b = doubleBits(x);
@@ -185,6 +185,24 @@ PXG_HD int64_t mulc(Cst c, int64_t x)
 
 // an integer times 2^k as a double, correctly rounded (k keeps it normal)
 PXG_HD double toDouble(int64_t x, int k) { return scaleExp((double)x, k); }
+// the same for any k whose result is below 2^1023; zero below the normal range (a check that
+// costs 2 % of the hexahedra's kernels where every entry makes it)
+PXG_HD double toDoubleFlush(int64_t x, int k)
+{
+  double const d = (double)x;
+  return expoField(d) + k > 0 ? scaleExp(d, k) : 0.0;
+}
+// the factor m 2^e (F = 62) of values whose last bit is 2^(e - bits), made smaller where that
+// is below the normal range, so that they end at 2^-1022
+PXG_HD void limitFactor(int64_t & m, int & e, int bits)
+{
+  int const low = bits - 1022 - e;
+  if (low > 0)
+  {
+    m >>= low < 63 ? low : 63;
+    e += low;
+  }
+}
 
 // 1 / d for d at F = 60 in [1/2, 1): F = 56, relative error below 2^-55.  A float
 // estimate y0 (relative error e below 2^-21), then y0 (1 + e + e^2), e = 1 - d y0.

@@ -353,9 +353,10 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
     // the coefficient of a single stiffness (mass) operator is folded into its values
     ok = q1x::decompose(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
     ok = q1x::decompose(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
-    ok = ok && abs(ke) < 300 && abs(me) < 300; // every value stays normal
+    ok = ok && abs(ke) < 300 && abs(me) < 300; // the products stay below 2^1023
     int const sg = q1x::productShift(ps);
     eD = q1x::detExponent(sc, s, nd);
+    q1x::limitFactor(mm, me, 61 - eD);
     eK = q1x::tensorExponent(sc, scMin, s, k, sg) + ke - 61;
     if (needK)
     {
@@ -399,7 +400,7 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
     }
     else
       f = fieldPoint(a.field, sh, l, w);
-    sh.rqd[w][l] = a.rc * (q1x::toDouble(det, eD - 60) * f);
+    sh.rqd[w][l] = a.rc * (q1x::toDoubleFlush(det, eD - 60) * f);
   }
   __syncthreads();
   pdlWait(); // the writes start below
@@ -474,7 +475,7 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
           q1x::nodeSums(r);
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            fe[q] = a.rc * q1x::toDouble(r[q], el);
+            fe[q] = a.rc * q1x::toDoubleFlush(r[q], el);
         }
         else
         {

@@ -169,7 +169,7 @@ PXG_HD bool coordScales(int32_t m0, int32_t m1, int32_t m2, int (&sc)[3])
     sc[r] = sc[r] >= hi - 2 ? hi : sc[r];
     lo = sc[r] < lo ? sc[r] : lo;
   }
-  return lo >= -300 && hi <= 59;
+  return lo >= -300 && hi <= 57; // (57: the conversion to F = 57 does not lower an exponent)
 }
 
 // Column shifts from the largest high words cmax[a * 3 + r]: the columns at F = 62 are then

@@ -811,9 +811,10 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
   // the coefficient of a single stiffness (mass) operator is folded into its values
   ok = q1x::decompose(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
   ok = q1x::decompose(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
-  ok = ok && abs(ke) < 300 && abs(me) < 300; // every value stays normal
+  ok = ok && abs(ke) < 300 && abs(me) < 300; // the products stay below 2^1023
   int const sg = q1x::productShift(sh.ps[el]);
   int const eD = q1x::detExponent(sc, s, nd);
+  q1x::limitFactor(mm, me, 60 - eD);
   int const eK = q1x::tensorExponent(sc, scMin, s, k, sg) + ke - 57, eM = eD + me - 60;
   if (x < NQ)
   {
@@ -855,7 +856,7 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
         for (int r = 0; r < 3; ++r)
           p[r] = fma(0.774596669241483, q1x::toDouble(u[r], sc[r] - 61), sh.org[r][el]);
       sh.rq[q][el] =
-          __double_as_longlong(a.rc * (q1x::toDouble(dw, eD - 60) * pointValue(a, sh, el, q, p[0], p[1], p[2])));
+          __double_as_longlong(a.rc * (q1x::toDoubleFlush(dw, eD - 60) * pointValue(a, sh, el, q, p[0], p[1], p[2])));
     }
   }
   if (tid < E)
@@ -937,7 +938,7 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
         uint32_t const dof = sh.dof[el][n];
         if (a.rkind && !(a.rbc && c))
           atomicAdd(a.b + dof,
-                    fixedLoad ? a.rc * q1x::toDouble(rq[L][el], ex) : __longlong_as_double(rq[L][el]));
+                    fixedLoad ? a.rc * q1x::toDoubleFlush(rq[L][el], ex) : __longlong_as_double(rq[L][el]));
         if (c)
         {
           // buildLhs' Dirichlet values, once per operator with BCs (builder.hpp:119)

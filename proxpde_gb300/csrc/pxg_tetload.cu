@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(64) kTetSineLoad(AsmArgs const __grid_constant
       for (int q = 0; q < NQ; ++q)
         s = fx::madw(r[q].h, R.w[i][q].h, s);
       if (!((cons >> i) & 1u))
-        atomicAdd(a.b + dof[i], f0 * fx::toDouble(s, ex - 57 - shiftOf(T)));
+        atomicAdd(a.b + dof[i], f0 * fx::toDoubleFlush(s, ex - 57 - shiftOf(T)));
     }
     return;
   }
