@@ -1040,8 +1040,8 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_consta
   {
     int64_t km;
     int ke;
-    bool const okK = fx::decompose(ksf * cP1Ws, km, ke);
-    fixed = tetx::tetGram(J, okK && abs(ke) < 300, km, ke, G, adet);
+    bool const okK = fx::coefParts(ksf * cP1Ws, km, ke);
+    fixed = tetx::tetGram(J, okK, km, ke, G, adet);
   }
   if (!fixed)
   {

@@ -229,6 +229,17 @@ PXG_HD bool decompose(double x, int64_t & m, int & e)
   e = f - 1022;
   return f != 0 && f != 0x7ff;
 }
+// the same of an operator's coefficient: zero is 0 2^0 (its elements' values are zero in
+// fixed point too); false also beyond 2^+-300
+PXG_HD bool coefParts(double x, int64_t & m, int & e)
+{
+  if (x == 0.)
+  {
+    m = 0, e = 0;
+    return true;
+  }
+  return decompose(x, m, e) && e > -300 && e < 300;
+}
 
 } // namespace fx
 } // namespace pxg

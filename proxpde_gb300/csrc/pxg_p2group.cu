@@ -132,9 +132,9 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
       double G[6];
       int64_t km;
       int ke;
-      bool const okK = fx::decompose(ks, km, ke);
+      bool const okK = fx::coefParts(ks, km, ke);
       km = (int64_t)((uint64_t)fx::mulc(fx::cst(0x4444444444444444ll), km) << 1);
-      if (!tetx::tetGram(J, okK && abs(ke) < 300, km, ke - 4, G, adet))
+      if (!tetx::tetGram(J, okK, km, ke - 4, G, adet))
       {
         double A[3][3];
         adet = fabs(adj3(J, A));

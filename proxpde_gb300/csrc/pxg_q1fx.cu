@@ -351,9 +351,9 @@ __global__ void __launch_bounds__(256, MINB) kAssembleQ1Fx(AsmArgs const __grid_
     }
     ok = q1x::detShifts(lo, hi, nd, k) && ok;
     // the coefficient of a single stiffness (mass) operator is folded into its values
-    ok = q1x::decompose(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
-    ok = q1x::decompose(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
-    ok = ok && abs(ke) < 300 && abs(me) < 300; // the products stay below 2^1023
+    // (their range keeps the products below 2^1023)
+    ok = q1x::coefParts(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
+    ok = q1x::coefParts(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
     int const sg = q1x::productShift(ps);
     eD = q1x::detExponent(sc, s, nd);
     q1x::limitFactor(mm, me, 61 - eD);

@@ -809,9 +809,9 @@ __global__ void __launch_bounds__(q2f::NT, 5) kAssembleQ2Fx(AsmArgs const __grid
   int ke, me, nd, k;
   ok = q1x::detShifts(sh.lo[el], sh.hi[el], nd, k) && ok;
   // the coefficient of a single stiffness (mass) operator is folded into its values
-  ok = q1x::decompose(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
-  ok = q1x::decompose(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
-  ok = ok && abs(ke) < 300 && abs(me) < 300; // the products stay below 2^1023
+  // (their range keeps the products below 2^1023)
+  ok = q1x::coefParts(a.fold.coefK ? a.fold.sK * kfac : a.fold.sK, km, ke) && ok;
+  ok = q1x::coefParts(a.fold.coefM ? a.fold.sM * kfac : a.fold.sM, mm, me) && ok;
   int const sg = q1x::productShift(sh.ps[el]);
   int const eD = q1x::detExponent(sc, s, nd);
   q1x::limitFactor(mm, me, 60 - eD);
