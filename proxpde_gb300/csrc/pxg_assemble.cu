@@ -2145,20 +2145,9 @@ pxg_status pxg_assemble(pxg_ctx * c, pxg_lhs_op const * op0, double * vals0, pxg
           lg.grpBeg = c->groups.beg.p;
           lg.grpItem = c->groups.item.p;
           lg.grpRedMax = c->groupRedMax;
-          // its loads: none or a constant; others in the one-thread kernel
-          bool const other = la.rkind && !(la.rkind == 1 && la.fn == PXG_FN_CONST);
-          if (other)
-            lg.rkind = 0;
           launchAssembleP2Group(lg, s, c->threads);
-          if (other)
-          {
-            AsmArgs l2 = la;
-            l2.op[0].on = l2.op[1].on = 0;
-            l2.pdl = 0;
-            launchAssembleTet64<P2TET>(l2, s, c->threads);
-          }
         }
-        else
+        else if (!launchP2PointLoad(la, s))
           launchAssembleTet64<P2TET>(la, s, c->threads);
       }
       else

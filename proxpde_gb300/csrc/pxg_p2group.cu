@@ -5,6 +5,10 @@
 // each sum once.  Shared memory (22.5 KB per group) limits an SM to ten groups: with one warp
 // per group its ten warps left the map's loads and the additions' latency exposed
 // (13^3 x 6, less than one group per SM sub-partition: 45 us).
+// Loads that need the points (a function but the sine, a DOF field) are warp 1's too, beside the
+// values (K + M with the Poisson right hand side: 57 us at 6^3 x 6 and 0.40 ms at 30^3 x 6; by the
+// one-thread kernel in a second launch 80 us and 0.49 ms), or a kernel's of their own without
+// operators (19 us and 0.095 ms a DOF field at 13^3 x 6 and 30^3 x 6, 37 and 0.199 by the other).
 // Dirichlet conditions: a mask per element leaves its constrained pairs out of the sums, and
 // its lane adds the constrained diagonals and the free rows' lifts (builder.hpp:76-124).
 #include <vector>
@@ -20,6 +24,8 @@ namespace
 // mass values of the seven classes and sum_q w_q phi_i(q), for |det J| = 1
 __constant__ double cMass[7];
 __constant__ double cInt[10];
+// the rule's points, weights and basis values
+__constant__ double cXi[11][3], cW[11], cPhi[11][10];
 
 struct GroupShared
 {
@@ -47,6 +53,86 @@ __device__ __forceinline__ void gramRows(double const (&G)[6], double (&s)[4][4]
   for (int n = 0; n < 6; ++n)
     E[n] = (s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 0)] + s[p2EdgeEnd(4 + n, 1)][p2EdgeEnd(4 + n, 1)]) +
            s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 1)];
+}
+
+// whether a load is one that the element's own points are needed for (the sine has a kernel of its
+// own, pxg_tetload.cu)
+__host__ __device__ __forceinline__ bool pointLoad(AsmArgs const & a)
+{
+  return a.rkind == 2 || (a.rkind == 1 && a.fn != PXG_FN_CONST);
+}
+// such a load of element e in FP64: a function or a DOF field at the points of the rule.  Out of
+// line, its registers are not the other calls'.
+__device__ __noinline__ void elementLoad(AsmArgs const & a, int64_t e)
+{
+  double X[4][3], J[3][3], A[3][3];
+  uint4 const c = reinterpret_cast<uint4 const *>(a.conn)[e];
+  uint32_t const v[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+  for (int n = 0; n < 4; ++n)
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      X[n][d] = a.xyz[3 * (int64_t)v[n] + d];
+  uint32_t dof[10];
+#pragma unroll
+  for (int i = 0; i < 10; ++i)
+    dof[i] = a.emap[e * 10 + i];
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      J[r][k] = X[k + 1][r] - X[0][r];
+  double const f0 = a.rc * fabs(adj3(J, A));
+  double rq[11];
+  if (a.rkind == 1)
+  {
+#pragma unroll
+    for (int q = 0; q < 11; ++q)
+    {
+      double x[3];
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+        x[r] = X[0][r] + (J[r][0] * cXi[q][0] + J[r][1] * cXi[q][1] + J[r][2] * cXi[q][2]);
+      rq[q] = (f0 * cW[q]) * evalFn(a.fn, 1.0, x[0], x[1], x[2]);
+    }
+  }
+  else
+  {
+    double loc[10];
+#pragma unroll
+    for (int n = 0; n < 10; ++n)
+      loc[n] = a.field[dof[n]];
+#pragma unroll
+    for (int q = 0; q < 11; ++q)
+    {
+      double s = 0.;
+#pragma unroll
+      for (int n = 0; n < 10; ++n)
+        s = fma(cPhi[q][n], loc[n], s);
+      rq[q] = (f0 * cW[q]) * s;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 10; ++i)
+  {
+    if (a.rbc && a.bcMask && a.bcMask[dof[i]])
+      continue;
+    double fe = 0.;
+#pragma unroll
+    for (int q = 0; q < 11; ++q)
+      fe = fma(cPhi[q][i], rq[q], fe);
+    red(a.b + dof[i], fe);
+  }
+}
+
+// such a load by itself
+__global__ void __launch_bounds__(64) kP2PointLoad(AsmArgs const __grid_constant__ a)
+{
+  int64_t const i = blockIdx.x * 64ll + threadIdx.x;
+  if (i >= a.nelem)
+    return;
+  pdlWait();
+  elementLoad(a, elemOf(a, i));
 }
 
 // PLAIN: one operator's stiffness and the other's mass, no Dirichlet conditions
@@ -195,6 +281,11 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         if (k0 + 32 * r < n8)
           sh.item[k0 + 32 * r] = t[r];
     }
+    if (!PLAIN && pointLoad(a) && lane < W)
+    {
+      pdlWait(); // its writes start here
+      elementLoad(a, e);
+    }
   }
   __syncthreads();
   pdlWait(); // the writes start here
@@ -332,7 +423,7 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
           red(a.b + dof[i], -z[i]);
     }
   }
-  if (a.rkind) // a constant load
+  if (a.rkind && (PLAIN || !pointLoad(a))) // a constant load
   {
     double const f = a.rc * adet;
 #pragma unroll
@@ -347,9 +438,10 @@ pxg_status initP2Group(pxg_ctx * c)
 {
   std::vector<double> xi, w;
   hostRule(P2TET, xi, w);
-  double M[100] = {}, I[10] = {}, phi[10], dphi[30];
+  double M[100] = {}, I[10] = {}, P[110], dphi[30];
   for (size_t q = 0; q < w.size(); ++q)
   {
+    double * const phi = P + 10 * q;
     hostShape(P2TET, &xi[3 * q], phi, dphi);
     for (int i = 0; i < 10; ++i)
     {
@@ -363,6 +455,9 @@ pxg_status initP2Group(pxg_ctx * c)
     m7[k] = M[10 * p2MassRepI(k) + p2MassRepJ(k)];
   PXG_CUDA(c, cudaMemcpyToSymbol(cMass, m7, sizeof(m7)));
   PXG_CUDA(c, cudaMemcpyToSymbol(cInt, I, sizeof(I)));
+  PXG_CUDA(c, cudaMemcpyToSymbol(cXi, xi.data(), sizeof(cXi)));
+  PXG_CUDA(c, cudaMemcpyToSymbol(cW, w.data(), sizeof(cW)));
+  PXG_CUDA(c, cudaMemcpyToSymbol(cPhi, P, sizeof(P)));
   return PXG_OK;
 }
 
@@ -373,10 +468,20 @@ void launchAssembleP2Group(AsmArgs const & a, cudaStream_t s, int)
     return;
   // the usual pair without Dirichlet conditions has its own instance: the others' branches
   // cost its loops
-  bool const plain = a.fold.needK && a.fold.needM && !a.fold.same && !(a.bcMask && (a.fold.bc || (a.rkind && a.rbc)));
+  bool const plain = a.fold.needK && a.fold.needM && !a.fold.same &&
+                     !(a.bcMask && (a.fold.bc || (a.rkind && a.rbc))) && !pointLoad(a);
   if (plain)
     launchElemKernel(kAssembleP2Group<true>, blocks, 64, 0, s, a);
   else
     launchElemKernel(kAssembleP2Group<false>, blocks, 64, 0, s, a);
+}
+
+bool launchP2PointLoad(AsmArgs const & a, cudaStream_t s)
+{
+  if (a.op[0].on || a.op[1].on || !pointLoad(a))
+    return false;
+  if (a.nelem > 0)
+    launchElemKernel(kP2PointLoad, (unsigned)((a.nelem + 63) / 64), 64, 0, s, a);
+  return true;
 }
 } // namespace pxg
