@@ -970,9 +970,9 @@ __global__ void __launch_bounds__(NT) kAssembleTet(AsmArgs a)
 // kAssembleTet64 (the default for P1/P2) in IEEE binary64 throughout.  Per element:
 // J from the vertex differences, adj(J), |det J|, G = adj adj^T / |det J| (with a
 // single stiffness operator's coefficient folded in).  P1 reads its entries from G
-// directly; P2 with at most one stiffness and one mass uses the barycentric form below,
+// directly; P2 with a stiffness operator and then a mass uses the barycentric form below,
 // and otherwise the six-term products of G with the reference tensor (FP64 constant
-// memory).  A mass entry is |det J| Mhat_ij (a single mass operator's coefficient
+// memory), the rule's own.  A mass entry is |det J| Mhat_ij (a single mass operator's coefficient
 // folded into |det J|).  P2 tetrahedron: src/reffe.cpp:542-642, vertices then the
 // edges 01 12 20 03 13 23.
 
@@ -1027,9 +1027,10 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_consta
   double const ms0 = m0 ? massCoef(op0, kfac) : 0., ms1 = m1 ? massCoef(op1, kfac) : 0.;
   bool const anyBc = cons && ((op0.on && op0.bc) || (op1.on && op1.bc));
   // bcWarp: some lane has constrained entries.  fast: at most one stiffness and one mass
-  // (P2: both), their coefficients folded in, no per-entry operator branches
+  // (P2: the stiffness first, then the mass), their coefficients folded in, no per-entry operator
+  // branches
   bool const bcWarp = !PLAIN && __any_sync(__activemask(), anyBc);
-  bool const both = PLAIN || (needK && needM && !a.fold.same);
+  bool const both = PLAIN || (k0 && m1 && !a.fold.same);
   bool const fast = PLAIN || (a.fold.simple && !bcWarp && (T == P1TET || both));
   double const ksf = foldK ? (k0 ? ks0 : ks1) : 1.0;
   double G[6], adet;
@@ -1041,7 +1042,10 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_consta
     int64_t km;
     int ke;
     bool const okK = fx::coefParts(ksf * cP1Ws, km, ke);
-    fixed = tetx::tetGram(J, okK, km, ke, G, adet);
+    tetx::Gram gr;
+    fixed = tetx::tetGram(J, okK, km, ke, gr);
+    if (fixed)
+      tetx::toDoubles(gr, G, adet);
   }
   if (!fixed)
   {
@@ -1845,7 +1849,7 @@ void launchAssembleTet64(AsmArgs const & args, cudaStream_t s, int threads)
   // the usual pair without Dirichlet conditions (of the operators or of the load) has its own
   // instance: the others' branches cost its registers (64^3 x 6, K + M: 1.05 ms against 1.12)
   bool const plain = a.fold.simple && a.fold.needK && a.fold.needM && !a.fold.same &&
-                     !(a.bcMask && (a.fold.bc || (a.rkind && a.rbc)));
+                     (T == P1TET || a.op[0].stiff) && !(a.bcMask && (a.fold.bc || (a.rkind && a.rbc)));
   if (threads == 64)
     return plain ? go(kAssembleTet64<T, 64, true>, 64) : go(kAssembleTet64<T, 64, false>, 64);
   if (threads == 256)

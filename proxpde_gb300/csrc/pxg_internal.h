@@ -518,7 +518,8 @@ __host__ __device__ constexpr int p2UpperIdx(int i, int j)
 // warp-group scatter of the P2 kernel: the 55 stiffness entries and the 7 mass values of
 // each of a group's 32 elements in shared memory, and its 3,200 contribution codes; a code
 // is lane | pair index << 5 | mass class << 11
-constexpr int kP2GroupValues = 55 + 7;
+constexpr int kP2Pairs = 55;
+constexpr int kP2GroupValues = kP2Pairs + 7;
 constexpr int kP2GroupItems = 32 * 100;
 __host__ __device__ constexpr uint16_t p2GroupCode(int lane, int i, int j)
 {

@@ -1,14 +1,14 @@
 // P2 tetrahedra with the warp-group scatter (pxg_group.cu), a block of two warps per group of 32
 // elements.  Warp 0 forms the elements' values, one element per lane, from the geometry in fixed
-// point (pxg_tetfx.h) and in barycentric form (pxg_p2bary.h), and leaves them in shared memory, while warp 1 copies the
-// group's contribution codes there; then both sum the group's distinct positions and add
-// each sum once.  Shared memory (22.5 KB per group) limits an SM to ten groups: with one warp
-// per group its ten warps left the map's loads and the additions' latency exposed
-// (13^3 x 6, less than one group per SM sub-partition: 45 us).
-// Loads that need the points (a function but the sine, a DOF field) are warp 1's too, beside the
-// values (K + M with the Poisson right hand side: 57 us at 6^3 x 6 and 0.40 ms at 30^3 x 6; by the
-// one-thread kernel in a second launch 80 us and 0.49 ms), or a kernel's of their own without
-// operators (19 us and 0.095 ms a DOF field at 13^3 x 6 and 30^3 x 6, 37 and 0.199 by the other).
+// point (pxg_tetfx.h), in barycentric form (pxg_p2bary.h) or by the rule's tensors, and leaves
+// them in shared memory, while warp 1 copies the group's contribution codes there; then both sum
+// the group's distinct positions and add each sum once.  Shared memory (22.5 KB per group) limits
+// an SM to ten groups: with one warp per group its ten warps left the map's loads and the
+// additions' latency exposed (13^3 x 6, less than one group per SM sub-partition: 45 us).
+// Loads that need the points (a function but the sine, a DOF field) are warp 1's too where there
+// are no conditions (K + M with the Poisson right hand side at 6^3, 30^3 and 64^3 x 6: 51, 339 and
+// 2,865 us; in a launch of their own 57, 391 and 3,200), and a launch of their own elsewhere (with
+// conditions 85, 519 and 4,450 us, together 88, 643 and 7,147).
 // Dirichlet conditions: a mask per element leaves its constrained pairs out of the sums, and
 // its lane adds the constrained diagonals and the free rows' lifts (builder.hpp:76-124).
 #include <vector>
@@ -21,30 +21,35 @@ namespace pxg
 {
 namespace
 {
-// mass values of the seven classes and sum_q w_q phi_i(q), for |det J| = 1
-__constant__ double cMass[7];
-__constant__ double cInt[10];
-// the rule's points, weights and basis values
-__constant__ double cXi[11][3], cW[11], cPhi[11][10];
+// the rule: for |det J| = 1 the mass values of the seven classes and of all 55 pairs and sum_q
+// w_q phi_i(q); the points, weights and basis values; the reference tensors of the pairs (xx yy zz
+// xy xz yz, the mixed ones summed over both orders)
+struct P2Rule
+{
+  double mass7[7], mass[kP2Pairs], integral[10];
+  double xi[11][3], w[11], phi[11][10];
+  double T[6][kP2Pairs];
+};
+__constant__ P2Rule cR;
 
 struct GroupShared
 {
   double val[kP2GroupValues * 32];
   uint4 item[kP2GroupItems / 8];
-  unsigned long long cons[32];
 };
 
 __device__ __forceinline__ void red(double * p, double v) { atomicAdd(p, v); }
 
 // s (4 x 4, zero row sums) and E_ab = s_aa + s_bb + s_ab of the six edges from the Gram
 // entries of vertices 1..3
-__device__ __forceinline__ void gramRows(double const (&G)[6], double (&s)[4][4], double (&E)[6])
+template <class V>
+__device__ __forceinline__ void gramRows(V const (&G)[6], V (&s)[4][4], V (&E)[6])
 {
   s[1][1] = G[0], s[2][2] = G[1], s[3][3] = G[2];
   s[1][2] = s[2][1] = G[3];
   s[1][3] = s[3][1] = G[4];
   s[2][3] = s[3][2] = G[5];
-  double const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
+  V const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
   s[0][1] = s[1][0] = -c1;
   s[0][2] = s[2][0] = -c2;
   s[0][3] = s[3][0] = -c3;
@@ -53,6 +58,25 @@ __device__ __forceinline__ void gramRows(double const (&G)[6], double (&s)[4][4]
   for (int n = 0; n < 6; ++n)
     E[n] = (s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 0)] + s[p2EdgeEnd(4 + n, 1)][p2EdgeEnd(4 + n, 1)]) +
            s[p2EdgeEnd(4 + n, 0)][p2EdgeEnd(4 + n, 1)];
+}
+
+// whether the gradient of P2 function i has a component along reference direction d
+__host__ __device__ constexpr bool hasDir(int i, int d)
+{
+  return i < 4 ? (i == 0 || i == d + 1)
+               : p2EdgeEnd(i, 0) == 0 || p2EdgeEnd(i, 1) == 0 || p2EdgeEnd(i, 0) == d + 1 || p2EdgeEnd(i, 1) == d + 1;
+}
+// entry (I, J) of the stiffness by the rule's tensor, without the 129 terms of 330 that are zero
+template <int I, int J>
+__device__ __forceinline__ double tensorEntry(double const (&G)[6])
+{
+  constexpr int A[6] = {0, 1, 2, 0, 0, 1}, B[6] = {0, 1, 2, 1, 2, 2};
+  double k = 0.;
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+    if ((hasDir(I, A[c]) && hasDir(J, B[c])) || (hasDir(I, B[c]) && hasDir(J, A[c])))
+      k = fma(cR.T[c][p2UpperIdx(I, J)], G[c], k);
+  return k;
 }
 
 // whether a load is one that the element's own points are needed for (the sine has a kernel of its
@@ -92,8 +116,8 @@ __device__ __noinline__ void elementLoad(AsmArgs const & a, int64_t e)
       double x[3];
 #pragma unroll
       for (int r = 0; r < 3; ++r)
-        x[r] = X[0][r] + (J[r][0] * cXi[q][0] + J[r][1] * cXi[q][1] + J[r][2] * cXi[q][2]);
-      rq[q] = (f0 * cW[q]) * evalFn(a.fn, 1.0, x[0], x[1], x[2]);
+        x[r] = X[0][r] + (J[r][0] * cR.xi[q][0] + J[r][1] * cR.xi[q][1] + J[r][2] * cR.xi[q][2]);
+      rq[q] = (f0 * cR.w[q]) * evalFn(a.fn, 1.0, x[0], x[1], x[2]);
     }
   }
   else
@@ -108,8 +132,8 @@ __device__ __noinline__ void elementLoad(AsmArgs const & a, int64_t e)
       double s = 0.;
 #pragma unroll
       for (int n = 0; n < 10; ++n)
-        s = fma(cPhi[q][n], loc[n], s);
-      rq[q] = (f0 * cW[q]) * s;
+        s = fma(cR.phi[q][n], loc[n], s);
+      rq[q] = (f0 * cR.w[q]) * s;
     }
   }
 #pragma unroll
@@ -120,7 +144,7 @@ __device__ __noinline__ void elementLoad(AsmArgs const & a, int64_t e)
     double fe = 0.;
 #pragma unroll
     for (int q = 0; q < 11; ++q)
-      fe = fma(cPhi[q][i], rq[q], fe);
+      fe = fma(cR.phi[q][i], rq[q], fe);
     red(a.b + dof[i], fe);
   }
 }
@@ -135,11 +159,16 @@ __global__ void __launch_bounds__(64) kP2PointLoad(AsmArgs const __grid_constant
   elementLoad(a, elemOf(a, i));
 }
 
-// PLAIN: one operator's stiffness and the other's mass, no Dirichlet conditions
-template <bool PLAIN>
+// PLAIN: the first operator's stiffness and the second's mass, no Dirichlet conditions, in the
+// barycentric form and with one mass value per class of pairs.  The others by the rule's own
+// tensors: its points and weights have 13 to 16 digits, so that they differ by 2e-15 from the exact
+// moments of the barycentric form (the mass by 8e-16 within a class).
+// LOAD (PLAIN only): with a load that needs the points.
+template <bool PLAIN, bool LOAD>
 __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs const __grid_constant__ a)
 {
   __shared__ GroupShared sh;
+  __shared__ unsigned long long conMask[32]; // not PLAIN: without it ten groups fit an SM
   int const lane = threadIdx.x & 31;
   bool const first = threadIdx.x < 32;
   int64_t const g = blockIdx.x, e = g * 32 + lane;
@@ -149,6 +178,9 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
   // values of the same few elements (lanes) for different entries, which this swizzle
   // spreads over the banks
   auto at = [&](uint32_t v, uint32_t l) -> double & { return sh.val[v * 32 + (l ^ (v & 15u))]; };
+  // not PLAIN: the lanes' mass factors are value 55, and cR.mass for the flush's scattered reads follows
+  double * const mass = sh.val + 56 * 32;
+  static_assert(56 * 32 + kP2Pairs <= kP2GroupValues * 32, "mass values in the place of the classes'");
   int const nItems = W * 100;
   int32_t const dBeg = a.grpOff[g], dEnd = a.grpOff[g + 1];
   // the map of the next batch of positions is loaded while this one is summed and reduced
@@ -213,40 +245,68 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         for (int k = 0; k < 3; ++k)
           J[r][k] = X[k + 1][r] - X[0][r];
       double const ks = a.fold.coefK ? a.fold.sK * kfac : a.fold.sK;
-      // s'_(a+1)(b+1) = G_ab, the Gram matrix of the cofactors times k / (30 |det J|), in fixed
-      // point (16 conversions for about 75 FP64 operations): km carries 16 / 30
-      double G[6];
-      int64_t km;
-      int ke;
+      // the Gram matrix of the cofactors times k / |det J|, in fixed point (16 conversions for about
+      // 75 FP64 operations).  PLAIN: over 30, s'_(a+1)(b+1) = G_ab: km carries 16 / 30
+      int64_t km, Gx[6];
+      int ke, eG;
       bool const okK = fx::coefParts(ks, km, ke);
-      km = (int64_t)((uint64_t)fx::mulc(fx::cst(0x4444444444444444ll), km) << 1);
-      if (!tetx::tetGram(J, okK, km, ke - 4, G, adet))
+      if (PLAIN)
+        km = (int64_t)((uint64_t)fx::mulc(fx::cst(0x4444444444444444ll), km) << 1), ke -= 4;
+      tetx::Gram gr;
+      bool const fixed = tetx::tetGram(J, okK, km, ke, gr);
+      if (PLAIN && fixed && tetx::aligned(gr, Gx, eG))
       {
-        double A[3][3];
-        adet = fabs(adj3(J, A));
-        // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + t + t^2),
-        // t = 1 - x y), instead of a full-precision division with its special cases
-        double ra;
-        asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
-        double const t = fma(-adet, ra, 1.0);
-        ra = fma(ra, fma(t, t, t), ra);
-        gram(A, ks * ra * (1.0 / 30.0), G);
-      }
-      if (needK)
-      {
-        double s[4][4], E[6];
-        gramRows(G, s, E);
+        // the entries in integers, where one exponent holds all six products: their conversions do
+        // not wait for one another (64^3 x 6, K + M: 0.98 ms, in FP64 1.05)
+        adet = tetx::detOf(gr);
+        int64_t s[4][4], E[6];
+        gramRows(Gx, s, E);
         p2ForPairs<0, 0>([&](auto I, auto Jj) {
           constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-          at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
+          at(p2UpperIdx(i, j), lane) = fx::toDouble(p2StiffFixed<i, j>(s, E), eG);
         });
+      }
+      else
+      {
+        double G[6];
+        if (fixed)
+          tetx::toDoubles(gr, G, adet);
+        else
+        {
+          double A[3][3];
+          adet = fabs(adj3(J, A));
+          // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + t + t^2),
+          // t = 1 - x y), instead of a full-precision division with its special cases
+          double ra;
+          asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
+          double const t = fma(-adet, ra, 1.0);
+          ra = fma(ra, fma(t, t, t), ra);
+          gram(A, PLAIN ? ks * ra * (1.0 / 30.0) : ks * ra, G);
+        }
+        if (!PLAIN && needK)
+          p2ForPairs<0, 0>([&](auto I, auto Jj) {
+            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+            at(p2UpperIdx(i, j), lane) = tensorEntry<i, j>(G);
+          });
+        if (PLAIN)
+        {
+          double s[4][4], E[6];
+          gramRows(G, s, E);
+          p2ForPairs<0, 0>([&](auto I, auto Jj) {
+            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+            at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
+          });
+        }
       }
       if (needM)
       {
         double const am = (a.fold.coefM ? a.fold.sM * kfac : a.fold.sM) * adet;
+        if (!PLAIN)
+          at(55, lane) = am;
+        else
 #pragma unroll
-        for (int c7 = 0; c7 < 7; ++c7)
-          at(55 + c7, lane) = am * cMass[c7];
+          for (int c7 = 0; c7 < 7; ++c7)
+            at(55 + c7, lane) = am * cR.mass7[c7];
       }
     }
     if (!PLAIN)
@@ -258,7 +318,7 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
           if ((cons & (1u << i)) || (cons & (1u << j)))
             m |= 1ull << p2UpperIdx(i, j);
         });
-      sh.cons[lane] = m;
+      conMask[lane] = m;
     }
     loadBatch(dBeg);
   }
@@ -281,7 +341,10 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         if (k0 + 32 * r < n8)
           sh.item[k0 + 32 * r] = t[r];
     }
-    if (!PLAIN && pointLoad(a) && lane < W)
+    if (!PLAIN && needM)
+      for (int k = lane; k < kP2Pairs; k += 32)
+        mass[k] = cR.mass[k];
+    if (LOAD && lane < W)
     {
       pdlWait(); // its writes start here
       elementLoad(a, e);
@@ -289,7 +352,9 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
   }
   __syncthreads();
   pdlWait(); // the writes start here
-  bool const bc = !PLAIN && a.fold.bc && a.bcMask && __any_sync(0xffffffffu, sh.cons[lane] != 0ull);
+  bool bc = false;
+  if constexpr (!PLAIN)
+    bc = a.fold.bc && a.bcMask && __any_sync(0xffffffffu, conMask[lane] != 0ull);
   uint16_t const * const si = reinterpret_cast<uint16_t const *>(sh.item);
   for (int32_t d0 = dBeg; d0 < dEnd; d0 += U * 64)
   {
@@ -338,9 +403,9 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
       {
         uint32_t const code = si[k], v = (code >> 5) & 63u, l = code & 31u;
         // constrained pairs are left out of the matrices of operators with BCs
-        bool const c = bc && ((sh.cons[l] >> v) & 1ull);
+        bool const c = bc && ((conMask[l] >> v) & 1ull);
         double ka = needK && !(c && a.fold.bcK) ? at(v, l) : 0.;
-        double const ma = needM && !(c && a.fold.bcM) ? at(55 + (code >> 11), l) : 0.;
+        double const ma = needM && !(c && a.fold.bcM) ? at(55, l) * mass[v] : 0.;
         if (a.fold.same)
           ka += ma;
         if (each)
@@ -410,7 +475,7 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
             return;
           double v = needK && f.bcK ? at(p2UpperIdx(i, j), lane) : 0.;
           if (needM && f.bcM)
-            v += at(55 + p2MassClass(i, j), lane);
+            v = fma(at(55, lane), cR.mass[p2UpperIdx(i, j)], v);
           if (cj)
             z[i] = fma(v, hv[j], z[i]);
           else
@@ -423,13 +488,13 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
           red(a.b + dof[i], -z[i]);
     }
   }
-  if (a.rkind && (PLAIN || !pointLoad(a))) // a constant load
+  if (!LOAD && a.rkind) // a constant load
   {
     double const f = a.rc * adet;
 #pragma unroll
     for (int i = 0; i < 10; ++i)
       if (!(a.rbc && ((cons >> i) & 1u)))
-        red(a.b + dof[i], f * cInt[i]);
+        red(a.b + dof[i], f * cR.integral[i]);
   }
 }
 } // namespace
@@ -438,26 +503,33 @@ pxg_status initP2Group(pxg_ctx * c)
 {
   std::vector<double> xi, w;
   hostRule(P2TET, xi, w);
-  double M[100] = {}, I[10] = {}, P[110], dphi[30];
+  P2Rule R{};
   for (size_t q = 0; q < w.size(); ++q)
   {
-    double * const phi = P + 10 * q;
+    double dphi[30], * const phi = R.phi[q];
     hostShape(P2TET, &xi[3 * q], phi, dphi);
+    R.w[q] = w[q];
+    for (int d = 0; d < 3; ++d)
+      R.xi[q][d] = xi[3 * q + d];
     for (int i = 0; i < 10; ++i)
     {
-      I[i] += w[q] * phi[i];
-      for (int j = 0; j < 10; ++j)
-        M[10 * i + j] += w[q] * phi[i] * phi[j];
+      R.integral[i] += w[q] * phi[i];
+      for (int j = i; j < 10; ++j)
+      {
+        int const u = p2UpperIdx(i, j);
+        double const *gi = dphi + 3 * i, *gj = dphi + 3 * j;
+        R.mass[u] += w[q] * phi[i] * phi[j];
+        for (int d = 0; d < 3; ++d)
+          R.T[d][u] += w[q] * gi[d] * gj[d];
+        R.T[3][u] += w[q] * (gi[0] * gj[1] + gi[1] * gj[0]);
+        R.T[4][u] += w[q] * (gi[0] * gj[2] + gi[2] * gj[0]);
+        R.T[5][u] += w[q] * (gi[1] * gj[2] + gi[2] * gj[1]);
+      }
     }
   }
-  double m7[7];
   for (int k = 0; k < 7; ++k)
-    m7[k] = M[10 * p2MassRepI(k) + p2MassRepJ(k)];
-  PXG_CUDA(c, cudaMemcpyToSymbol(cMass, m7, sizeof(m7)));
-  PXG_CUDA(c, cudaMemcpyToSymbol(cInt, I, sizeof(I)));
-  PXG_CUDA(c, cudaMemcpyToSymbol(cXi, xi.data(), sizeof(cXi)));
-  PXG_CUDA(c, cudaMemcpyToSymbol(cW, w.data(), sizeof(cW)));
-  PXG_CUDA(c, cudaMemcpyToSymbol(cPhi, P, sizeof(P)));
+    R.mass7[k] = R.mass[p2UpperIdx(p2MassRepI(k), p2MassRepJ(k))];
+  PXG_CUDA(c, cudaMemcpyToSymbol(cR, &R, sizeof(R)));
   return PXG_OK;
 }
 
@@ -466,14 +538,27 @@ void launchAssembleP2Group(AsmArgs const & a, cudaStream_t s, int)
   unsigned const blocks = (unsigned)((a.nelem + 31) / 32);
   if (blocks == 0)
     return;
-  // the usual pair without Dirichlet conditions has its own instance: the others' branches
-  // cost its loops
-  bool const plain = a.fold.needK && a.fold.needM && !a.fold.same &&
-                     !(a.bcMask && (a.fold.bc || (a.rkind && a.rbc))) && !pointLoad(a);
+  // the usual pair without Dirichlet conditions (a load that needs the points has its own) has an
+  // instance of its own: the others' branches cost its loops
+  bool const load = pointLoad(a);
+  bool const plain = a.fold.needK && a.fold.needM && !a.fold.same && a.op[0].stiff &&
+                     !(a.bcMask && (a.fold.bc || (a.rkind && a.rbc && !load)));
   if (plain)
-    launchElemKernel(kAssembleP2Group<true>, blocks, 64, 0, s, a);
-  else
-    launchElemKernel(kAssembleP2Group<false>, blocks, 64, 0, s, a);
+  {
+    launchElemKernel(load ? kAssembleP2Group<true, true> : kAssembleP2Group<true, false>, blocks, 64, 0, s, a);
+    return;
+  }
+  AsmArgs l = a;
+  if (load)
+    l.rkind = 0;
+  launchElemKernel(kAssembleP2Group<false, false>, blocks, 64, 0, s, l);
+  if (load)
+  {
+    l = a;
+    l.op[0].on = l.op[1].on = 0;
+    l.pdl = 0;
+    launchP2PointLoad(l, s);
+  }
 }
 
 bool launchP2PointLoad(AsmArgs const & a, cudaStream_t s)
