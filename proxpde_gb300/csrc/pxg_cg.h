@@ -391,7 +391,7 @@ struct CgRows
           t += __shfl_xor_sync(0xffffffffu, t, o);
       }
       else
-        t = rowDot<false, LPR, 8>(g.rp, g.ci, g.a, g.p, r0 + v, v < nr);
+        t = rowDot<LPR, 8>(g.rp, g.ci, g.a, g.p, r0 + v, v < nr);
       if (v < nr && lane % LPR == 0)
       {
         q[v] = t;

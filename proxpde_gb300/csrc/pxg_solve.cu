@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(kTpb) kSpmvPlainDot(int32_t const * __restrict
   {
     int64_t const row = r0 + lane / kLpr;
     bool const valid = row < n;
-    double const t = rowDot<false>(rp, ci, a, x, row, valid);
+    double const t = rowDot<>(rp, ci, a, x, row, valid);
     if (valid && (lane & (kLpr - 1)) == 0)
     {
       y[row] = t;
