@@ -2002,6 +2002,16 @@ void threadCandidates(pxg_ctx const * c, int (&out)[4])
   else
     out[0] = 128;
 }
+// whether a call without a colouring takes P2's group kernel, whose blocks have one size
+bool usesP2Group(pxg_ctx const * c, pxg_lhs_op const * op0, pxg_lhs_op const * op1)
+{
+  int stiff = 0, mass = 0;
+  for (pxg_lhs_op const * o : {op0, op1})
+    if (o)
+      stiff += o->stiffness != 0, mass += o->mass != 0;
+  return c->etype == P2TET && c->arith == PXG_ARITH_FP64 && !c->tetGeneric && c->groups.built && c->groupScatter &&
+         stiff <= 1 && mass <= 1 && stiff + mass > 0;
+}
 } // namespace
 
 extern "C"
@@ -2149,7 +2159,7 @@ pxg_status pxg_assemble(pxg_ctx * c, pxg_lhs_op const * op0, double * vals0, pxg
           lg.grpBeg = c->groups.beg.p;
           lg.grpItem = c->groups.item.p;
           lg.grpRedMax = c->groupRedMax;
-          launchAssembleP2Group(lg, s, c->threads);
+          launchAssembleP2Group(lg, s);
         }
         else if (!launchP2PointLoad(la, s))
           launchAssembleTet64<P2TET>(la, s, c->threads);
@@ -2344,6 +2354,16 @@ pxg_status pxg_autotune(pxg_ctx * c, pxg_lhs_op const * op0, pxg_lhs_op const * 
         break;
       c->scatter = sc;
       c->threads = t;
+      // P2's group kernel is the same launch for every block size: timed once
+      bool const again = sc == PXG_SCATTER_REDUCE && rep->ncand > 0 && usesP2Group(c, op0, op1);
+      if (again)
+      {
+        rep->cand_threads[rep->ncand] = t;
+        rep->cand_scatter[rep->ncand] = sc;
+        rep->cand_ms[rep->ncand] = rep->cand_ms[0];
+        ++rep->ncand;
+        continue;
+      }
       auto run = [&] { return pxg_assemble(c, op0, v0.p, op1, v1.p, rhs, bb.p, 0u, s); };
       if ((st = run()) != PXG_OK) // warm-up
         break;

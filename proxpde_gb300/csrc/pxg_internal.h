@@ -624,7 +624,7 @@ pxg_status initQ2Tables(pxg_ctx * c);                      // pxg_q2.cu
 void launchAssembleQ2(AsmArgs const & a, cudaStream_t s, int sms); // pxg_q2.cu
 pxg_status initP2Group(pxg_ctx * c);                              // pxg_p2group.cu
 // P2 tetrahedra with the warp-group map (at most one stiffness and one mass; rhs kinds 0 to 2)
-void launchAssembleP2Group(AsmArgs const & a, cudaStream_t s, int threads);
+void launchAssembleP2Group(AsmArgs const & a, cudaStream_t s);
 // a P2 load by itself that needs the element's points; false where it is another call
 bool launchP2PointLoad(AsmArgs const & a, cudaStream_t s);
 pxg_status initTetLoad(pxg_ctx * c);                              // pxg_tetload.cu

@@ -533,7 +533,7 @@ pxg_status initP2Group(pxg_ctx * c)
   return PXG_OK;
 }
 
-void launchAssembleP2Group(AsmArgs const & a, cudaStream_t s, int)
+void launchAssembleP2Group(AsmArgs const & a, cudaStream_t s)
 {
   unsigned const blocks = (unsigned)((a.nelem + 31) / 32);
   if (blocks == 0)

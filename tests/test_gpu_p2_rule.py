@@ -66,3 +66,21 @@ def test_matrices_are_the_rule_s(engine, ops, bc, scatter):
         # six products and additions an entry, each within half an ulp of the element's norm at most, and the
         # tensors' own rounding (eleven terms, summed in FP64)
         assert (err / ref).max() <= 6 * 2.0 ** -53
+
+
+def test_autotune_times_the_group_kernel_once(engine):
+    """The group kernel has one block size: its three candidates are one launch and one time, and the first of
+    them is kept unless a colouring is faster."""
+    from proxpde_gb300 import Context
+    from helpers import problem
+
+    xyz, conn, k = problem("tet6", 6, 0.15, seed=4, sigma=1.0)
+    ctx = Context(0)
+    ctx.set_mesh(O.P2TET, xyz, conn)
+    ctx.build_dofmap()
+    ctx.build_pattern()
+    ctx.set_coef(k)
+    rep = ctx.autotune(op0=K_OP, op1=M_OP)
+    ms = [c[2] for c in rep["candidates"] if c[1] == "reduce"]
+    assert len(ms) == 3 and len(set(ms)) == 1
+    assert rep["scatter"] != "reduce" or rep["threads"] == rep["candidates"][0][0]
