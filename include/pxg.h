@@ -343,7 +343,11 @@ pxg_status pxg_memcpy(pxg_ctx * ctx, void * dst, const void * src, uint64_t byte
  * the last iterate) when the tolerance is not met.  The solve runs on a stream of the
  * context ordered after `stream`, as one persistent cooperative kernel, and is waited for
  * on the host, so it returns with the solve complete and cannot be captured into the
- * caller's graph.  PXG_ERR_TIMEOUT if a bounded wait between its blocks ran out. */
+ * caller's graph.  Its blocks, up to one per SM with most of the SM's shared memory, run
+ * at the same time and wait for one another: a solve starts when that many SMs are free, so
+ * that large solves of several contexts or streams run one after the other.  PXG_ERR_TIMEOUT
+ * if a bounded wait between its blocks (about half a minute) ran out; the context stays
+ * usable. */
 pxg_status pxg_cg(pxg_ctx * ctx, const int32_t * row_ptr, const int32_t * col_idx,
                   const double * vals, int64_t n, const double * b, double * x, double rtol,
                   int max_iter, int * iters, double * rel_res, void * stream);

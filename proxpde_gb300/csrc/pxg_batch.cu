@@ -434,12 +434,7 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
     d.trace = trace.p;
     use_graph = 0;
   }
-  {
-    // PXG_TEST_BARRIER_SHORTFALL=1 makes every barrier wait for one block more
-    // than the group has, so the bounded waits run out (tests of the timeout path)
-    char const * t = getenv("PXG_TEST_BARRIER_SHORTFALL");
-    d.extra = (t && t[0] == '1') ? 1u : 0u;
-  }
+  d.extra = barrierShortfall();
 
   cudaStream_t const s = (cudaStream_t)stream;
   auto record = [&](cudaStream_t rs) -> pxg_status {

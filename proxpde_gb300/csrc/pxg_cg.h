@@ -17,6 +17,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstdlib>
 #include <type_traits>
 
 #include "pxg_internal.h"
@@ -28,7 +29,17 @@ namespace
 constexpr int kCgT = 512;               // threads of the solver's blocks (one per SM)
 constexpr int kCgWarps = kCgT / 32;
 constexpr int kCgEntries = 896;         // entries of a warp's tile in shared memory (32 rows of 27)
-constexpr unsigned kCgPolls = 1u << 21; // polls of a wait before giving up (some seconds)
+// Polls of a wait before giving up (about half a minute): a block may have to wait for SMs that
+// another stream's kernel holds.  With arrivals missing on purpose (tests): some seconds.
+constexpr unsigned kCgPolls = 1u << 25, kCgPollsTest = 1u << 21;
+
+// PXG_TEST_BARRIER_SHORTFALL=1 makes every barrier wait for one block more than the group has, so
+// that the bounded waits run out (tests of the timeout path)
+inline unsigned barrierShortfall()
+{
+  char const * t = std::getenv("PXG_TEST_BARRIER_SHORTFALL");
+  return t && t[0] == '1' ? 1u : 0u;
+}
 
 struct CgArgs
 {
@@ -91,7 +102,7 @@ struct CgShared
 // over the calling lanes up to one check.
 __device__ __forceinline__ bool cgGiveUp(CgArgs const & g, unsigned polls)
 {
-  bool const up = __any_sync(__activemask(), polls >= kCgPolls || *(unsigned volatile *)g.err != 0u);
+  bool const up = __any_sync(__activemask(), polls >= (g.extra ? kCgPollsTest : kCgPolls) || *(unsigned volatile *)g.err != 0u);
   if (up)
     atomicExch(g.err, 1u);
   return up;

@@ -160,7 +160,7 @@ pxg_status cgSolve(pxg_ctx * c, int32_t const * rp, int32_t const * ci, double c
   unsigned * const counters = reinterpret_cast<unsigned *>(w.scal.p + S_COUNT);
   double * scal = w.scal.p;
   CgArgs g{rp, ci, a, b, x, w.p.p, w.r.p, w.z.p, w.dinv.p, reinterpret_cast<ulonglong2 *>(w.part.p), counters,
-           counters + 1, 0, n, 0u, (unsigned)grid, 0u, rtol * rtol, maxIter, cap, aligned, nullptr, 0};
+           counters + 1, 0, n, 0u, (unsigned)grid, barrierShortfall(), rtol * rtol, maxIter, cap, aligned, nullptr, 0};
   void * args[] = {&g, &scal};
   PXG_CUDA(c, cudaMemsetAsync(w.part.p, 0, 6 * grid * sizeof(double), s)); // no sum has the tag 0
   PXG_CUDA(c, cudaMemsetAsync(w.scal.p, 0, (S_COUNT + 1) * sizeof(double), s));
