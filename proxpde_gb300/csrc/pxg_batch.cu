@@ -316,6 +316,8 @@ pxg_status pxg_batch_set(pxg_ctx * c, int64_t const * elem_offsets, int64_t npro
     return st;
   BatchState & B = c->batch;
   int64_t const n = c->ndof, nnz = c->nnz;
+  B.ready = false;
+  ++B.set;
   B.nprob = nprob;
   PXG_CUDA(c, B.elemOff.alloc(nprob + 1));
   PXG_CUDA(c, B.dofOff.alloc(nprob + 1));
@@ -494,6 +496,14 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
       cudaStreamDestroy(cs);
       if (e != PXG_OK)
       {
+      pxg_ctx const * c = ctxs[i];
+      key.set[i] = c->batch.set;
+      void const * const buf[] = {c->xyz.p, c->conn.p, c->emap.p, c->rowPtr.p, c->colIdx.p,
+                                  c->rank.p, c->kE.p, c->bcMask.p, c->bcVal.p, c->colour.perm.p};
+      static_assert(sizeof(buf) == sizeof(key.buf[0]), "one key entry per buffer");
+      std::memcpy(key.buf[i], buf, sizeof(buf));
+      key.nbc[i] = c->nbc;
+      key.bcDiag[i] = c->bcDiag;
         if (graph)
           cudaGraphDestroy(graph);
         return e;

@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <cstdio>
+#include <cstring>
 #include <string>
 #include <utility>
 #include <vector>
@@ -215,6 +216,7 @@ struct AdjState
 struct BatchState
 {
   bool ready = false;
+  uint64_t set = 0; // number of pxg_batch_set calls so far
   int64_t nprob = 0;
   pxg::DevBuf<int64_t> elemOff, dofOff;
   std::vector<int64_t> dofOffHost;
@@ -234,13 +236,20 @@ struct GraphKey
   int smem = 0;
   int scatter[2] = {0, 0}, threads[2] = {0, 0}; // the element kernels captured in the graph
   int arith[2] = {0, 0};
+  // the buffers and values of the contexts that the captured launches hold
+  uint64_t set[2] = {0, 0}; // pxg_batch_set calls so far
+  void const * buf[2][10] = {};
+  int64_t nbc[2] = {0, 0};
+  double bcDiag[2] = {0., 0.};
   bool operator==(GraphKey const & o) const
   {
     return nctx == o.nctx && ctx[0] == o.ctx[0] && ctx[1] == o.ctx[1] && ut[0] == o.ut[0] && ut[1] == o.ut[1] &&
            grad[0] == o.grad[0] && grad[1] == o.grad[1] && rhs.kind == o.rhs.kind && rhs.fn == o.rhs.fn &&
            rhs.coef == o.rhs.coef && rhs.field == o.rhs.field && rtol == o.rtol && maxIter == o.maxIter && smem == o.smem &&
            scatter[0] == o.scatter[0] && scatter[1] == o.scatter[1] && threads[0] == o.threads[0] &&
-           threads[1] == o.threads[1] && arith[0] == o.arith[0] && arith[1] == o.arith[1];
+           threads[1] == o.threads[1] && arith[0] == o.arith[0] && arith[1] == o.arith[1] &&
+           set[0] == o.set[0] && set[1] == o.set[1] && nbc[0] == o.nbc[0] && nbc[1] == o.nbc[1] &&
+           bcDiag[0] == o.bcDiag[0] && bcDiag[1] == o.bcDiag[1] && std::memcmp(buf, o.buf, sizeof(buf)) == 0;
   }
 };
 
