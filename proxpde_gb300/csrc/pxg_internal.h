@@ -260,6 +260,11 @@ struct BatchShared
   pxg::DevBuf<unsigned char> res, prob, group; // results, problem list, the blocks' groups
   pxg::DevBuf<double> part;                    // the blocks' sums
   pxg::DevBuf<unsigned> bar;                   // the groups' arrivals, the error flag, the queue
+  // what the plan in prob and group was made for (bytes of the problems and their entries), its
+  // largest share of rows and the first group's size
+  std::vector<unsigned char> planProb, planEntries;
+  int64_t planShare = 0;
+  int planBlocks0 = 0;
   cudaGraphExec_t exec = nullptr;
   GraphKey key;
   ~BatchShared()
