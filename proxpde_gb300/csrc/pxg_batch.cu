@@ -81,13 +81,14 @@ struct BatchResult
 struct BatchDev
 {
   SysDev sys[2];
-  Group const * group; // [blocks]
+  Group const * group; // [blocks], and the list entries that single warps solve
   Problem const * prob;
   BatchResult * res;
   ulonglong2 * part; // [3 * blocks]
   unsigned * bar;    // [blocks]
   unsigned * err;
-  int * next;     // [0] entries of the shared queue taken; [1 + block] the entry its group takes
+  int * next;     // [0] entries of the shared queue taken; [1 + block] the entry its group takes;
+                  // [1 + blocks] the warps' entries taken
   unsigned extra; // arrivals expected beyond a group (0; > 0 only to test the timeout path)
   double tol2;
   int maxIter;
@@ -139,6 +140,116 @@ __device__ __forceinline__ bool batchProblem(BatchDev const & d, SysDev const & 
   return true;
 }
 
+// Small problems, where there are many: a warp each, its vectors in the place of its tile.  A block
+// takes some 24 us for a problem of eight rows, most of it barriers and the latency of a few rows
+// (a call on 20,000 cubes of one element: 3.2 ms, 1.35 here; 4,000 of one or two a side 0.89 and 0.40).
+constexpr int kWarpRows = 64;
+struct WarpVec
+{
+  double x[kWarpRows], r[kWarpRows], z[kWarpRows], p[kWarpRows], q[kWarpRows], di[kWarpRows];
+};
+static_assert(sizeof(WarpVec) <= sizeof(CgTile), "a warp's vectors in its tile");
+
+__device__ __forceinline__ double warpAll(double v)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+// q = A v on the problem's rows (a row per lane); returns v.q
+__device__ __forceinline__ double warpProduct(SysDev const & s, Problem const & pr, double const * a,
+                                              double const * v, double * q)
+{
+  double dot = 0.;
+  for (int i = threadIdx.x & 31; i < (int)pr.rows; i += 32)
+  {
+    double t = 0.;
+    for (int32_t k = s.rp[pr.row0 + i], e = s.rp[pr.row0 + i + 1]; k < e; ++k)
+      t = fma(a[k], v[s.ci[k] - (int)pr.row0], t);
+    q[i] = t;
+    dot += v[i] * t;
+  }
+  __syncwarp();
+  return warpAll(dot);
+}
+// the CG of cgRun on v.r = b; the iterations as batchProblem counts them
+__device__ __forceinline__ int warpCg(BatchDev const & d, SysDev const & s, Problem const & pr, WarpVec & v)
+{
+  int const lane = threadIdx.x & 31, n = (int)pr.rows;
+  double rz = 0., rr = 0.;
+  for (int i = lane; i < n; i += 32)
+  {
+    double const b = v.r[i], z = v.di[i] * b;
+    v.x[i] = 0.;
+    v.p[i] = z;
+    rz += b * z;
+    rr += b * b;
+  }
+  rz = warpAll(rz);
+  rr = warpAll(rr);
+  __syncwarp();
+  double const bb = rr;
+  if (bb == 0.)
+    return 0;
+  for (int it = 1;; ++it)
+  {
+    double const al = rz / warpProduct(s, pr, s.K, v.p, v.q);
+    double rz1 = 0.;
+    rr = 0.;
+    for (int i = lane; i < n; i += 32)
+    {
+      v.x[i] += al * v.p[i];
+      double const r = v.r[i] - al * v.q[i], z = v.di[i] * r;
+      v.r[i] = r;
+      v.z[i] = z;
+      rz1 += r * z;
+      rr += r * r;
+    }
+    rz1 = warpAll(rz1);
+    rr = warpAll(rr);
+    if (rr <= d.tol2 * bb)
+      return it;
+    if (it >= d.maxIter || !(rr == rr))
+      return d.maxIter;
+    double const be = rz1 / rz;
+    rz = rz1;
+    for (int i = lane; i < n; i += 32)
+      v.p[i] = v.z[i] + be * v.p[i];
+    __syncwarp();
+  }
+}
+__device__ __noinline__ void warpProblem(BatchDev const & d, Problem const & pr, WarpVec & v)
+{
+  SysDev const & s = d.sys[pr.sys];
+  int const lane = threadIdx.x & 31, n = (int)pr.rows;
+  BatchResult res{0., 0, 0};
+  for (int i = lane; i < n; i += 32)
+  {
+    double di = 0.;
+    for (int32_t k = s.rp[pr.row0 + i]; k < s.rp[pr.row0 + i + 1]; ++k)
+      if (s.ci[k] == (int32_t)(pr.row0 + i))
+        di = s.K[k];
+    v.di[i] = di != 0. ? 1.0 / di : 1.0;
+    v.r[i] = s.b[pr.row0 + i];
+  }
+  __syncwarp();
+  res.itF = warpCg(d, s, pr, v);
+  for (int i = lane; i < n; i += 32)
+  {
+    s.u[pr.row0 + i] = v.x[i];
+    v.p[i] = v.x[i] - s.ut[pr.row0 + i];
+  }
+  __syncwarp();
+  res.J = 0.5 * warpProduct(s, pr, s.M, v.p, v.r); // the right hand side of the adjoint
+  res.itA = warpCg(d, s, pr, v);
+  for (int i = lane; i < n; i += 32)
+    s.lam[pr.row0 + i] = v.x[i];
+  if (lane == 0)
+    d.res[pr.out] = res;
+  __syncwarp();
+}
+
 __global__ void __launch_bounds__(kCgT, 1) kBatchSolve(BatchDev const __grid_constant__ d)
 {
   extern __shared__ __align__(16) unsigned char dyn[];
@@ -176,6 +287,18 @@ __global__ void __launch_bounds__(kCgT, 1) kBatchSolve(BatchDev const __grid_con
     if (!ok)
       return;
   }
+  Group const small = d.group[gridDim.x];
+  __syncthreads(); // the tiles are free
+  for (;;)
+  {
+    int i = 0;
+    if ((threadIdx.x & 31) == 0)
+      i = small.beg < small.end ? small.beg + atomicAdd(d.next + 1 + gridDim.x, 1) : small.end;
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if (i >= small.end)
+      return;
+    warpProblem(d, d.prob[i], *reinterpret_cast<WarpVec *>(tiles + threadIdx.x / 32));
+  }
 }
 
 // Deals `blocks` blocks to the problems so that all end together, by the time an iteration takes: a
@@ -188,10 +311,16 @@ __global__ void __launch_bounds__(kCgT, 1) kBatchSolve(BatchDev const __grid_con
 //  - many problems: groups of one size, which take the problems, longest first, as they become
 //    free (groups of whole blocks per problem waste up to half of the last block each).
 // Returns the largest share of rows.
-int64_t planBatch(std::vector<Problem> & prob, std::vector<double> const & entries, int blocks,
-                  std::vector<Group> & group)
+int64_t planGroups(std::vector<Problem> & prob, std::vector<double> const & entries, int blocks,
+                   std::vector<Group> & group)
 {
   size_t const n = prob.size();
+  if (n == 0)
+  {
+    for (int k = 0; k < blocks; ++k)
+      group.push_back(Group{k, 1, 0, 0, -1});
+    return 1;
+  }
   std::vector<double> its(n), work(n);
   double lo = 0., hi = 0.;
   auto exchange = [](int b) { return b == 1 ? 4. : 7.5 + 0.6 * std::log2((double)b); };
@@ -278,6 +407,33 @@ int64_t planBatch(std::vector<Problem> & prob, std::vector<double> const & entri
   for (; used < blocks; ++used)
     group[used] = Group{used, 1, 0, 0, -1};
   prob = list;
+  return share;
+}
+
+// The whole plan: groups for the larger problems, and a last entry of `group` for those that single
+// warps take: the problems of up to kWarpRows rows, where these are more than two per block (fewer
+// are done sooner by a block each).
+int64_t planBatch(std::vector<Problem> & prob, std::vector<double> const & entries, int blocks,
+                  std::vector<Group> & group)
+{
+  std::vector<Problem> large, small;
+  std::vector<double> e;
+  for (size_t p = 0; p < prob.size(); ++p)
+    if (prob[p].rows <= kWarpRows)
+      small.push_back(prob[p]);
+  bool const warps = small.size() > 2 * (size_t)blocks;
+  if (!warps)
+    small.clear();
+  for (size_t p = 0; p < prob.size(); ++p)
+    if (!warps || prob[p].rows > kWarpRows)
+    {
+      large.push_back(prob[p]);
+      e.push_back(entries[p]);
+    }
+  int64_t const share = planGroups(large, e, blocks, group);
+  group.push_back(Group{0, 0, (int)large.size(), (int)(large.size() + small.size()), -1});
+  prob = large;
+  prob.insert(prob.end(), small.begin(), small.end());
   return share;
 }
 
@@ -405,9 +561,9 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
       S.nprob = 0;
       PXG_CUDA(c0, S.res.alloc(nprob * sizeof(BatchResult)));
       PXG_CUDA(c0, S.prob.alloc(nprob * sizeof(Problem)));
-      PXG_CUDA(c0, S.group.alloc(blocks * sizeof(Group)));
+      PXG_CUDA(c0, S.group.alloc((blocks + 1) * sizeof(Group)));
       PXG_CUDA(c0, S.part.alloc(6 * blocks));
-      PXG_CUDA(c0, S.bar.alloc(2 * blocks + 2)); // and the error flag, the queue
+      PXG_CUDA(c0, S.bar.alloc(2 * blocks + 3)); // and the error flag, the queues
       S.nprob = nprob;
     }
     PXG_CUDA(c0, cudaMemcpy(S.prob.p, order.data(), order.size() * sizeof(Problem), cudaMemcpyHostToDevice));
@@ -471,7 +627,7 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
         return e;
     }
     PXG_CUDA(c0, cudaMemsetAsync(S.part.p, 0, 6 * blocks * sizeof(double), rs)); // no sum has the tag 0
-    PXG_CUDA(c0, cudaMemsetAsync(S.bar.p, 0, (2 * blocks + 2) * sizeof(unsigned), rs));
+    PXG_CUDA(c0, cudaMemsetAsync(S.bar.p, 0, (2 * blocks + 3) * sizeof(unsigned), rs));
     void * args[] = {&d};
     PXG_CUDA(c0, cudaLaunchCooperativeKernel((void const *)kBatchSolve, dim3(blocks), dim3(kCgT), args, smem, rs));
     for (int i = 0; i < nctx; ++i)
