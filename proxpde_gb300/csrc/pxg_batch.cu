@@ -539,7 +539,7 @@ pxg_status pxg_batch_adjoint(pxg_ctx * const * ctxs, int nctx, pxg_rhs_op const 
     }
   }
   // the plan depends on the problems' rows and entries alone, and the last call's, which is on the
-  // device, is kept for calls with the same ones (of 4,000 cubes of 1 or 2 elements a side 0.97 of 1.86 ms a call, with the copies)
+  // device, is kept for calls with the same ones (with 4,000 problems it and its copies took 0.97 ms)
   auto same = [](auto const & v, std::vector<unsigned char> const & bytes) {
     return bytes.size() == v.size() * sizeof(v[0]) && std::memcmp(v.data(), bytes.data(), bytes.size()) == 0;
   };
