@@ -3,9 +3,9 @@
 
 Workload (one step): the perturbed 128^3 Q1-hex unit cube (2,097,152 elements,
 2,146,689 nodes; interior nodes moved by a seeded U(-0.2h, 0.2h) per coordinate),
-per-element diffusivity k_e = exp(N(0,1)), 2x2x2 Gauss quadrature, at least at FP64
-precision (64-bit fixed point or IEEE binary64 values, binary64 sums): stiffness (AssemblyStiffnessFE with the
-P0 coefficient) and mass (AssemblyMass(1)) CSR values plus the load vector of
+per-element diffusivity k_e = exp(N(0,1)), 2x2x2 Gauss quadrature, at FP64 precision or
+better (64-bit fixed point or IEEE binary64 values, binary64 sums): stiffness
+(AssemblyStiffnessFE with the P0 coefficient) and mass (AssemblyMass(1)) CSR values plus the load vector of
 f = sin(pi x) sin(pi y) sin(pi z), assembled in one fused pass on the device-resident
 structural pattern, followed by closeMatrix's prune check of both matrices.  The mesh,
 DOF map and pattern are built once (timed separately as `setup_s`).  Inputs are

@@ -132,7 +132,9 @@ typedef enum pxg_scatter
 /* Outcome of pxg_autotune: the chosen configuration and every candidate's time. */
 typedef struct pxg_tune_report
 {
-  int threads;  /* threads per block of the element kernel (8 per element for Q1 hexahedra) */
+  int threads;  /* block size variant of the element kernel: threads per block, but for Q1 hexahedra
+                   in FP64 arithmetic (64, 128: three, four blocks of 256 threads per SM) and P2's
+                   reduction scatter, which has one */
   int scatter;  /* pxg_scatter */
   int ncolours; /* colour classes of the colouring (0 if it was not built) */
   int ncand;
@@ -288,9 +290,10 @@ pxg_status pxg_prune_count_device(pxg_ctx * ctx, const double * vals, int64_t * 
 pxg_status pxg_set_scatter(pxg_ctx * ctx, int scatter, int threads);
 /* Arithmetic of the element kernels.  The reference computes geometry, local matrices
  * and sums in double (FVec/FMat, include/def.hpp:157-160); PXG_ARITH_FP64, the
- * default, is at least as precise: an element's values are formed in 64-bit fixed point
- * with a common exponent (62-bit significand) or, where they do not share a range, by
- * IEEE binary64 operations, and summed as binary64.
+ * default, computes at that precision or better: hexahedra and the geometry of tetrahedra
+ * in 64-bit fixed point (62-bit significands under common exponents), whose errors stay at
+ * or below those of the binary64 forms of the same kernels, and everything else and the
+ * elements that the format does not hold by those forms; values are summed as binary64.
  * PXG_ARITH_DFL is an opt-in alternative with a narrower significand: the geometry and
  * the local matrices run as unevaluated pairs of floats (about 48 bits) on the FP32
  * pipes, and only the coordinate differences, the final sums and the reductions into

@@ -13,11 +13,14 @@
 // units the Jacobian columns (half edges) are shifted left by n_a until a bound of their
 // 1-norm over the points is in [1/2, 1), and cofactors, their products and the
 // determinants all stay below one.  The determinants' reciprocals and the products are
-// normalised once more, per point and per element.  A rounding of 2^-60 of the largest
-// value thus stands where the FP64 form has one of 2^-53, at every step; the smaller
-// values lose the same bits in both.  Refused are non-finite coordinates and coefficients,
-// zeros, elements whose determinant is below 2^-28 of their edges' product at some point,
-// and sizes whose exponents the results could not hold.
+// normalised once more, per point and per element.  Every step rounds at 2^-60 of its largest
+// value, so that cancellation loses bits from there: a rotated thin element of aspect a has
+// entries within about a 2^-53 of their bounds, one sheared until its edges meet at 1 / a
+// a 2^-52.  The FP64 form (pxg_q1f64.h), whose Gram determinant squares the condition, is 5 to
+// 10^5 times further off in every shape (tests/test_fixed_point_host.py); FP64 cofactors of an
+// axis-aligned shear would lose less than either.  Refused are non-finite coordinates and
+// coefficients, elements whose determinant is below 2^-28 of their edges' product at some
+// point, and sizes whose exponents the results could not hold.
 #pragma once
 
 #include "pxg_fx.h"

@@ -46,3 +46,17 @@ def test_tetrahedra(tmp_path):
         assert int(single) >= 0.97 * taken or name != "kuhn"
         # and no further off than the plain FP64 formulas, up to the last rounding
         assert det <= det64 + 2 * ULP and gram <= gram64 + 2 * ULP, (name, eps)
+
+
+def test_hexahedra(tmp_path):
+    lines = run("hex_fixed_point", tmp_path)
+    assert len(lines) == 1 + 6 * 5
+    for name, eps, taken, refused, k, m, k64, m64 in lines:
+        taken, refused, k, m, k64, m64 = int(taken), int(refused), *map(float, (k, m, k64, m64))
+        assert refused <= 0.02 * (taken + refused), (name, eps)
+        # nowhere further off than the FP64 form with the Gram determinant, up to the last rounding
+        assert not k > k64 + ULP and not m > m64 + ULP, (name, eps)
+        # in ordinary elements within a few roundings: a dozen steps of 2^-60 of the largest value each, which is
+        # at most 2^5 times an entry's bound, and the conversion
+        if name in ("cube", "small"):
+            assert k <= 4 * ULP and m <= 3 * ULP, (name, eps)
