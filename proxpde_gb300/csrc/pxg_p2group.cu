@@ -11,6 +11,7 @@
 // conditions 85, 519 and 4,450 us, together 88, 643 and 7,147).
 // Dirichlet conditions: a mask per element leaves its constrained pairs out of the sums, and
 // its lane adds the constrained diagonals and the free rows' lifts (builder.hpp:76-124).
+#include <cmath>
 #include <vector>
 
 #include "pxg_internal.h"
@@ -29,6 +30,7 @@ struct P2Rule
   double mass7[7], mass[kP2Pairs], integral[10];
   double xi[11][3], w[11], phi[11][10];
   double T[6][kP2Pairs];
+  fx::Sp Tx[6][kP2Pairs]; // T at F = 63
 };
 __constant__ P2Rule cR;
 
@@ -76,6 +78,19 @@ __device__ __forceinline__ double tensorEntry(double const (&G)[6])
   for (int c = 0; c < 6; ++c)
     if ((hasDir(I, A[c]) && hasDir(J, B[c])) || (hasDir(I, B[c]) && hasDir(J, A[c])))
       k = fma(cR.T[c][p2UpperIdx(I, J)], G[c], k);
+  return k;
+}
+
+// half of the same in fixed point, G below 2^62 (sum_c |T_c| < 2, so that it stays below 2^62)
+template <int I, int J>
+__device__ __forceinline__ int64_t tensorEntryFixed(fx::Sp const (&G)[6])
+{
+  constexpr int A[6] = {0, 1, 2, 0, 0, 1}, B[6] = {0, 1, 2, 1, 2, 2};
+  int64_t k = 0;
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+    if ((hasDir(I, A[c]) && hasDir(J, B[c])) || (hasDir(I, B[c]) && hasDir(J, A[c])))
+      k = fx::mulAdd(G[c], cR.Tx[c][p2UpperIdx(I, J)], k);
   return k;
 }
 
@@ -254,7 +269,7 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         km = (int64_t)((uint64_t)fx::mulc(fx::cst(0x4444444444444444ll), km) << 1), ke -= 4;
       tetx::Gram gr;
       bool const fixed = tetx::tetGram(J, okK, km, ke, gr);
-      if (PLAIN && fixed && tetx::aligned(gr, Gx, eG))
+      if (PLAIN && fixed && tetx::aligned<57>(gr, Gx, eG))
       {
         // the entries in integers, where one exponent holds all six products: their conversions do
         // not wait for one another (64^3 x 6, K + M: 0.98 ms, in FP64 1.05)
@@ -264,6 +279,19 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         p2ForPairs<0, 0>([&](auto I, auto Jj) {
           constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
           at(p2UpperIdx(i, j), lane) = fx::toDouble(p2StiffFixed<i, j>(s, E), eG);
+        });
+      }
+      else if (!PLAIN && needK && fixed && tetx::aligned<62>(gr, Gx, eG))
+      {
+        // the tensors' sums likewise: 201 products of 8 cycles instead of 64
+        adet = tetx::detOf(gr);
+        fx::Sp G[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c)
+          G[c] = fx::split(Gx[c]);
+        p2ForPairs<0, 0>([&](auto I, auto Jj) {
+          constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+          at(p2UpperIdx(i, j), lane) = fx::toDouble(tensorEntryFixed<i, j>(G), eG + 1);
         });
       }
       else
@@ -499,7 +527,7 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
 }
 } // namespace
 
-pxg_status initP2Group(pxg_ctx * c)
+pxg_status initP2Group(pxg_ctx * ctx)
 {
   std::vector<double> xi, w;
   hostRule(P2TET, xi, w);
@@ -527,9 +555,16 @@ pxg_status initP2Group(pxg_ctx * c)
       }
     }
   }
+  for (int c = 0; c < 6; ++c)
+    for (int u = 0; u < kP2Pairs; ++u)
+    {
+      if (std::fabs(R.T[c][u]) >= 0.75)
+        return fail(ctx, PXG_ERR_UNSUPPORTED, "P2 stiffness tensors");
+      R.Tx[c][u] = fx::split((int64_t)(R.T[c][u] * 9223372036854775808.0)); // exact from 2^-10
+    }
   for (int k = 0; k < 7; ++k)
     R.mass7[k] = R.mass[p2UpperIdx(p2MassRepI(k), p2MassRepJ(k))];
-  PXG_CUDA(c, cudaMemcpyToSymbol(cR, &R, sizeof(R)));
+  PXG_CUDA(ctx, cudaMemcpyToSymbol(cR, &R, sizeof(R)));
   return PXG_OK;
 }
 

@@ -164,10 +164,11 @@ PXG_HD void toDoubles(Gram const & o, double (&G)[6], double & adet)
   adet = detOf(o);
 }
 
-// The products as integers with one exponent, the largest in [2^56, 2^57), so that sums of up to
-// 36 times the largest fit.  False where that costs bits that FP64 keeps (a diagonal product
-// below 1/16 of the largest; 1 in 12,000 Kuhn tetrahedra with vertices moved by 0.2 of the edge),
-// the sum of all, vertex 0's, is above twice the largest.
+// The products as integers with one exponent, the largest in [2^(TOP - 1), 2^TOP).  False where that
+// costs bits that FP64 keeps: a diagonal product below 1/16 of the largest (1 in 12,000 Kuhn
+// tetrahedra with vertices moved by 0.2 of the edge).  TOP = 57: sums of up to 36 times the largest
+// fit, and the sum of all, vertex 0's, is at most twice the largest.
+template <int TOP>
 PXG_HD bool aligned(Gram const & o, int64_t (&g)[6], int & e)
 {
   bool const none = (o.g[0] | o.g[1] | o.g[2]) == 0; // km = 0
@@ -179,15 +180,18 @@ PXG_HD bool aligned(Gram const & o, int64_t (&g)[6], int & e)
     t = n > t ? n : t;
   }
   // (the diagonal ones are above 2^50, so that the upper words have their length)
-  e = t + 32 - 57;
+  e = t + 32 - TOP;
 #pragma unroll
   for (int i = 0; i < 6; ++i)
   {
     int const r = e - o.e[i];
     g[i] = r > 0 ? (o.g[i] + (1ll << ((r < 62 ? r : 62) - 1))) >> (r < 62 ? r : 62) : (int64_t)((uint64_t)o.g[i] << -r);
   }
-  int64_t const m = 1ll << 53, all = g[0] + g[1] + g[2] + 2 * (g[3] + g[4] + g[5]);
-  return none || (g[0] >= m && g[1] >= m && g[2] >= m && all <= 1ll << 58);
+  int64_t const m = 1ll << (TOP - 4);
+  bool const ok = g[0] >= m && g[1] >= m && g[2] >= m;
+  if (TOP < 60)
+    return none || (ok && g[0] + g[1] + g[2] + 2 * (g[3] + g[4] + g[5]) <= 1ll << (TOP + 1));
+  return none || ok;
 }
 } // namespace tetx
 } // namespace pxg

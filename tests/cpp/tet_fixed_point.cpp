@@ -104,22 +104,22 @@ int main()
         // one exponent for the six: the diagonal ones of the largest's size, the sums in 64 bits
         int64_t g[6];
         int e;
-        if (tetx::aligned(gr, g, e))
-        {
-          ++single;
+        Quad R[6], rd;
+        plain<Quad>(J, k, R, rd);
+        auto single1 = [&](int top) {
           double A[6];
           for (int i = 0; i < 6; ++i)
             A[i] = fx::toDouble(g[i], e);
-          Quad S[6], sd;
-          plain<Quad>(J, k, S, sd);
-          error(S, sd, A, d, one);
+          error(R, rd, A, d, one);
           for (int64_t x : g)
-            if (std::abs(x) >= 1ll << 57)
+            if (std::abs(x) >= 1ll << top)
               one[1] = 1.;
-        }
+        };
+        if (tetx::aligned<57>(gr, g, e))
+          ++single, single1(57);
+        if (tetx::aligned<62>(gr, g, e))
+          single1(62);
         ++taken;
-        Quad R[6], rd;
-        plain<Quad>(J, k, R, rd);
         plain<double>(J, k, Gd, dd);
         error(R, rd, G, d, fx);
         error(R, rd, Gd, dd, fp);
