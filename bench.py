@@ -718,8 +718,8 @@ def main():
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
             "vs_baseline": None, "dtype": "f64",
-            "arithmetic": "element values in 64-bit fixed point (62-bit significand; IEEE binary64 where an element's values do "
-                          "not share a range), binary64 sums and reductions",
+            "arithmetic": "element values in 64-bit fixed point (62-bit significands; IEEE binary64 where the format does "
+                          "not hold an element), binary64 sums and reductions",
             "data": "synthetic (seeded perturbed cube)",
             "config": {"workload": f"q1hex perturbed {n}^3: K(k_e)+M+rhs sin3, fused pass + prune check",
                        "elements": E, "nodes": nn, "ndof": ndof, "nnz": nnz, "pruned": list(pruned), "tuning": tuning,

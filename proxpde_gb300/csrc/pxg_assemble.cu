@@ -2140,8 +2140,8 @@ pxg_status pxg_assemble(pxg_ctx * c, pxg_lhs_op const * op0, double * vals0, pxg
     case P1TET:
       if (c->tetGeneric)
         launchAssemble<P1TET>(la, s, c->threads);
-      else if (fp64)
-        launchAssembleTet64<P1TET>(la, s, c->threads ? c->threads : 64); // 96^3 x 6: 0.79 ms, 128 threads 0.80
+      else if (fp64) // 64 threads: 16^3 and 96^3 x 6 13.5 and 755 us, 128: 14.3 and 763, 256: 14.9 and 929
+        launchAssembleTet64<P1TET>(la, s, c->threads ? c->threads : 64);
       else
         launchAssembleTet<P1TET>(la, s, c->threads);
       break;
@@ -2187,9 +2187,9 @@ pxg_status pxg_assemble(pxg_ctx * c, pxg_lhs_op const * op0, double * vals0, pxg
   };
   auto launch = [&](AsmArgs const & la) {
     // sin sin sin on tetrahedra in the FP64 arithmetic: its own fixed-point kernel (P2
-    // 30^3 x 6 with K and M: in one FP64 kernel 0.53 ms, in the two 0.20; P1 16^3 x 6 38 and
-    // 32 us, 6^3 x 6 23 and 30: a second launch costs more than P1's twelve sines on few
-    // elements)
+    // 30^3 x 6 with K and M: in one FP64 kernel 0.45 ms, in the two 0.23).  On few P1 elements a
+    // second launch costs more than twelve sines (K and M, one kernel against two, us: 6^3 x 6 19.3
+    // and 29.5, 10^3 19.3 and 21.1, 12^3 22.3 and 22.2, 13^3 26.7 and 23.1, 16^3 34.8 and 27.1)
     if (la.rkind == 1 && la.fn == PXG_FN_SIN3 && c->arith == PXG_ARITH_FP64 && !c->tetGeneric &&
         (c->etype == P2TET || (c->etype == P1TET && la.nelem >= 12000)))
     {

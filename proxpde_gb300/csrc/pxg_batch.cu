@@ -330,7 +330,8 @@ int64_t planGroups(std::vector<Problem> & prob, std::vector<double> const & entr
     work[p] = 0.33e-3 * (entries[p] + 8. * (double)prob[p].rows);
     hi += its[p] * (work[p] + 4.);
   }
-  // blocks of problem p for the end time t (one: it may share); a share has at least 128 rows
+  // blocks of problem p for the end time t (one: it may share); a share has at least 128 rows (a single
+  // solve's 192 is within 5 % of it)
   auto need = [&](size_t p, double t) {
     if (its[p] * (work[p] + 4.) <= t)
       return 1;

@@ -11,7 +11,7 @@
 // an entry is one FMA, every unused slot and every shuffle addition costs one too, so a
 // lane has a whole row where there are enough rows.
 // 884,736 Q1 hexahedra (912,673 rows): 113 us an iteration as three kernels replayed from a
-// captured graph (product 64-71), now 79 us (product 57, of which 42.5 is the FP64 pipe's
+// captured graph (product 64-71), now 82 us (product 57, of which 42.5 is the FP64 pipe's
 // and 42 the matrix's time in memory; the updates 11, the three exchanges the rest); at
 // 32^3 elements 17 us, now 13 us, bound by the exchanges.
 #pragma once

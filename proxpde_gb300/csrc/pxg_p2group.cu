@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
       if (PLAIN && fixed && tetx::aligned<57>(gr, Gx, eG))
       {
         // the entries in integers, where one exponent holds all six products: their conversions do
-        // not wait for one another (64^3 x 6, K + M: 0.98 ms, in FP64 1.05)
+        // not wait for one another (64^3 x 6, K + M: 1.01 ms, in FP64 1.05)
         adet = tetx::detOf(gr);
         int64_t s[4][4], E[6];
         gramRows(Gx, s, E);

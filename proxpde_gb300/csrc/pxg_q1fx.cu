@@ -15,7 +15,7 @@
 // 255 registers, which two warps per scheduler cannot hide and the instruction caches do
 // not hold (0.20 instructions per cycle, 2.8 of 10 cycles per instruction waiting for
 // code, 3.4 ms at 128^3).  Dealt over warps, each executes a tenth of it, 64 registers
-// suffice and 32 warps are resident: 2.14 ms (in FP64, one thread per element, 4.97 ms:
+// suffice and 32 warps are resident: 2.16 ms (in FP64, one thread per element, 4.97 ms:
 // 1,233 operations at 64 issue cycles a warp).  What is left is latency: the barriers
 // between the steps, instruction fetches and the reductions' queue.
 // Elements the format refuses (pxg_q1x.h) are computed in FP64 by a thread of their own.

@@ -3,8 +3,7 @@
 // with K lambda = M (u - u_t), K_e = k_e K0_e the element stiffness and C zeroing the
 // DOFs constrained by the essential BCs (the derivative of the condensed matrix
 // C K C + D is C K0_e C).  proxpde itself solves with UmfPackLU
-// (include/sparse_matrix.hpp:44); the CG here is plain and not an optimisation
-// target.
+// (include/sparse_matrix.hpp:44).
 //
 // The solver is pxg_cg.h's, all rows as one group of blocks, one block per SM.
 #include <cub/block/block_reduce.cuh>
@@ -141,9 +140,10 @@ pxg_status cgSolve(pxg_ctx * c, int32_t const * rp, int32_t const * ci, double c
   cudaStream_t const s = w.stream;
   PXG_CUDA(c, cudaEventRecord(w.evIn, user));
   PXG_CUDA(c, cudaStreamWaitEvent(s, w.evIn, 0));
-  // one block per SM, at least 192 rows (six warps) each: fewer blocks exchange faster (24^3 elements,
-  // the Poisson program and the adjoint gradient: 128 rows 2.05 and 3.09 ms, 192 1.83 and 2.69, 256
-  // 1.88 and 2.76, 512 2.12 and 3.48)
+  // one block per SM, at least 192 rows (six warps) each: fewer blocks exchange faster, more have
+  // less work.  An iteration with 128, 192, 256, 384 rows, us: Q1 12^3 10.6, 10.4, 10.9, 12.2, 24^3
+  // 12.6, 12.0, 12.1, 13.3, 30^3 13.1, 13.1, 14.2, 13.9; P1 24^3 x 6 11.6, 10.9, 11.2, 12.1.  The longer
+  // rows of Q2 (64 entries) are faster with 128: 12^3 16.7, 18.6, 23.8, 26.1
   int64_t const grid = std::min<int64_t>(c->sms, (n + 191) / 192);
   cudaFuncAttributes fa;
   PXG_CUDA(c, cudaFuncGetAttributes(&fa, kCgSolve));
