@@ -290,8 +290,8 @@ pxg_status pxg_prune_count_device(pxg_ctx * ctx, const double * vals, int64_t * 
 pxg_status pxg_set_scatter(pxg_ctx * ctx, int scatter, int threads);
 /* Arithmetic of the element kernels.  The reference computes geometry, local matrices
  * and sums in double (FVec/FMat, include/def.hpp:157-160); PXG_ARITH_FP64, the
- * default, computes at that precision or better: hexahedra and the geometry of tetrahedra
- * in 64-bit fixed point (62-bit significands under common exponents), whose errors stay at
+ * default, computes at that precision or better: hexahedra and the geometry of P1
+ * tetrahedra in 64-bit fixed point (62-bit significands under common exponents), whose errors stay at
  * or below those of the binary64 forms of the same kernels, and everything else and the
  * elements that the format does not hold by those forms; values are summed as binary64.
  * PXG_ARITH_DFL is an opt-in alternative with a narrower significand: the geometry and

@@ -1042,10 +1042,7 @@ __global__ void __launch_bounds__(NT) kAssembleTet64(AsmArgs const __grid_consta
     int64_t km;
     int ke;
     bool const okK = fx::coefParts(ksf * cP1Ws, km, ke);
-    tetx::Gram gr;
-    fixed = tetx::tetGram(J, okK, km, ke, gr);
-    if (fixed)
-      tetx::toDoubles(gr, G, adet);
+    fixed = tetx::tetGram(J, okK, km, ke, G, adet);
   }
   if (!fixed)
   {

@@ -92,40 +92,6 @@ __device__ __forceinline__ double p2Stiff(double const (&s)[4][4], double const 
     }
   }
 }
-// the same in 64-bit fixed point
-template <int I, int J>
-__device__ __forceinline__ int64_t p2StiffFixed(int64_t const (&s)[4][4], int64_t const (&E)[6])
-{
-  if constexpr (J < 4)
-    return I == J ? 3 * s[I][I] : -s[I][J];
-  else
-  {
-    constexpr int c = p2EdgeEnd(J, 0), d = p2EdgeEnd(J, 1);
-    if constexpr (I < 4)
-    {
-      if constexpr (I == c)
-        return 3 * s[I][d] - s[I][I];
-      else if constexpr (I == d)
-        return 3 * s[I][c] - s[I][I];
-      else
-        return -s[I][c] - s[I][d];
-    }
-    else
-    {
-      constexpr int a = p2EdgeEnd(I, 0), b = p2EdgeEnd(I, 1);
-      if constexpr (I == J)
-        return 8 * E[I - 4];
-      else if constexpr (a == c || a == d || b == c || b == d)
-      {
-        constexpr int v = (a == c || a == d) ? a : b, p = v == a ? b : a, q = c == v ? d : c;
-        constexpr int r = 6 - v - p - q;
-        return 8 * s[p][q] - 4 * s[v][r];
-      }
-      else
-        return -4 * (E[I - 4] + s[a][b]);
-    }
-  }
-}
 // a representative entry of each P2 mass class
 __host__ __device__ constexpr int p2MassRepI(int c) { return c < 4 ? 0 : 4; }
 __host__ __device__ constexpr int p2MassRepJ(int c)

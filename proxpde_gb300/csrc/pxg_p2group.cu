@@ -1,7 +1,6 @@
 // P2 tetrahedra with the warp-group scatter (pxg_group.cu), a block of two warps per group of 32
-// elements.  Warp 0 forms the elements' values, one element per lane, from the geometry in fixed
-// point (pxg_tetfx.h), in barycentric form (pxg_p2bary.h) or by the rule's tensors, and leaves
-// them in shared memory, while warp 1 copies the group's contribution codes there; then both sum
+// elements.  Warp 0 forms the elements' values in FP64, one element per lane, in barycentric form
+// (pxg_p2bary.h) or by the rule's tensors, and leaves them in shared memory, while warp 1 copies the group's contribution codes there; then both sum
 // the group's distinct positions and add each sum once.  Shared memory (22.5 KB per group) limits
 // an SM to ten groups: with one warp per group its ten warps left the map's loads and the
 // additions' latency exposed (13^3 x 6, less than one group per SM sub-partition: 45 us).
@@ -11,12 +10,10 @@
 // conditions 85, 519 and 4,450 us, together 88, 643 and 7,147).
 // Dirichlet conditions: a mask per element leaves its constrained pairs out of the sums, and
 // its lane adds the constrained diagonals and the free rows' lifts (builder.hpp:76-124).
-#include <cmath>
 #include <vector>
 
 #include "pxg_internal.h"
 #include "pxg_p2bary.h"
-#include "pxg_tetfx.h"
 
 namespace pxg
 {
@@ -30,7 +27,6 @@ struct P2Rule
   double mass7[7], mass[kP2Pairs], integral[10];
   double xi[11][3], w[11], phi[11][10];
   double T[6][kP2Pairs];
-  fx::Sp Tx[6][kP2Pairs]; // T at F = 63
 };
 __constant__ P2Rule cR;
 
@@ -44,14 +40,13 @@ __device__ __forceinline__ void red(double * p, double v) { atomicAdd(p, v); }
 
 // s (4 x 4, zero row sums) and E_ab = s_aa + s_bb + s_ab of the six edges from the Gram
 // entries of vertices 1..3
-template <class V>
-__device__ __forceinline__ void gramRows(V const (&G)[6], V (&s)[4][4], V (&E)[6])
+__device__ __forceinline__ void gramRows(double const (&G)[6], double (&s)[4][4], double (&E)[6])
 {
   s[1][1] = G[0], s[2][2] = G[1], s[3][3] = G[2];
   s[1][2] = s[2][1] = G[3];
   s[1][3] = s[3][1] = G[4];
   s[2][3] = s[3][2] = G[5];
-  V const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
+  double const c1 = G[0] + (G[3] + G[4]), c2 = G[3] + (G[1] + G[5]), c3 = G[4] + (G[5] + G[2]);
   s[0][1] = s[1][0] = -c1;
   s[0][2] = s[2][0] = -c2;
   s[0][3] = s[3][0] = -c3;
@@ -78,19 +73,6 @@ __device__ __forceinline__ double tensorEntry(double const (&G)[6])
   for (int c = 0; c < 6; ++c)
     if ((hasDir(I, A[c]) && hasDir(J, B[c])) || (hasDir(I, B[c]) && hasDir(J, A[c])))
       k = fma(cR.T[c][p2UpperIdx(I, J)], G[c], k);
-  return k;
-}
-
-// half of the same in fixed point, G below 2^62 (sum_c |T_c| < 2, so that it stays below 2^62)
-template <int I, int J>
-__device__ __forceinline__ int64_t tensorEntryFixed(fx::Sp const (&G)[6])
-{
-  constexpr int A[6] = {0, 1, 2, 0, 0, 1}, B[6] = {0, 1, 2, 1, 2, 2};
-  int64_t k = 0;
-#pragma unroll
-  for (int c = 0; c < 6; ++c)
-    if ((hasDir(I, A[c]) && hasDir(J, B[c])) || (hasDir(I, B[c]) && hasDir(J, A[c])))
-      k = fx::mulAdd(G[c], cR.Tx[c][p2UpperIdx(I, J)], k);
   return k;
 }
 
@@ -260,71 +242,48 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
         for (int k = 0; k < 3; ++k)
           J[r][k] = X[k + 1][r] - X[0][r];
       double const ks = a.fold.coefK ? a.fold.sK * kfac : a.fold.sK;
-      // the Gram matrix of the cofactors times k / |det J|, in fixed point (16 conversions for about
-      // 75 FP64 operations).  PLAIN: over 30, s'_(a+1)(b+1) = G_ab: km carries 16 / 30
-      int64_t km, Gx[6];
-      int ke, eG;
-      bool const okK = fx::coefParts(ks, km, ke);
-      if (PLAIN)
-        km = (int64_t)((uint64_t)fx::mulc(fx::cst(0x4444444444444444ll), km) << 1), ke -= 4;
-      tetx::Gram gr;
-      bool const fixed = tetx::tetGram(J, okK, km, ke, gr);
-      if (PLAIN && fixed && tetx::aligned<57>(gr, Gx, eG))
-      {
-        // the entries in integers, where one exponent holds all six products: their conversions do
-        // not wait for one another (64^3 x 6, K + M: 1.01 ms, in FP64 1.05)
-        adet = tetx::detOf(gr);
-        int64_t s[4][4], E[6];
-        gramRows(Gx, s, E);
-        p2ForPairs<0, 0>([&](auto I, auto Jj) {
-          constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-          at(p2UpperIdx(i, j), lane) = fx::toDouble(p2StiffFixed<i, j>(s, E), eG);
-        });
-      }
-      else if (!PLAIN && needK && fixed && tetx::aligned<62>(gr, Gx, eG))
-      {
-        // the tensors' sums likewise: 201 products of 8 cycles instead of 64
-        adet = tetx::detOf(gr);
-        fx::Sp G[6];
+      // lengths beyond 2^+-200, whose cofactors' squares leave the range, in units of their size
+      int size = 0;
 #pragma unroll
-        for (int c = 0; c < 6; ++c)
-          G[c] = fx::split(Gx[c]);
+      for (int k = 0; k < 9; ++k)
+        size = max(size, __double2hiint(J[k / 3][k % 3]) & 0x7fffffff);
+      size = (size >> 20) - 1023;
+      bool const scaled = abs(size) > 200 && abs(size) < 1000;
+      if (scaled)
+#pragma unroll
+        for (int k = 0; k < 9; ++k)
+          J[k / 3][k % 3] = ldexp(J[k / 3][k % 3], -size);
+      double A[3][3];
+      adet = fabs(adj3(J, A));
+      // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + t + t^2),
+      // t = 1 - x y), instead of a full-precision division with its special cases
+      double ra;
+      asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
+      double const t = fma(-adet, ra, 1.0);
+      ra = fma(ra, fma(t, t, t), ra);
+      // the Gram matrix of the cofactors times k / |det J|; PLAIN: over 30, s'_(a+1)(b+1) = G_ab
+      double G[6];
+      gram(A, PLAIN ? ks * ra * (1.0 / 30.0) : ks * ra, G);
+      if (scaled)
+      {
+        adet = ldexp(adet, 3 * size);
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+          G[k] = ldexp(G[k], size);
+      }
+      if (!PLAIN && needK)
         p2ForPairs<0, 0>([&](auto I, auto Jj) {
           constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-          at(p2UpperIdx(i, j), lane) = fx::toDouble(tensorEntryFixed<i, j>(G), eG + 1);
+          at(p2UpperIdx(i, j), lane) = tensorEntry<i, j>(G);
         });
-      }
-      else
+      if (PLAIN)
       {
-        double G[6];
-        if (fixed)
-          tetx::toDoubles(gr, G, adet);
-        else
-        {
-          double A[3][3];
-          adet = fabs(adj3(J, A));
-          // 1/|det J|: hardware estimate and one third-order Newton step (y (1 + t + t^2),
-          // t = 1 - x y), instead of a full-precision division with its special cases
-          double ra;
-          asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(ra) : "d"(adet));
-          double const t = fma(-adet, ra, 1.0);
-          ra = fma(ra, fma(t, t, t), ra);
-          gram(A, PLAIN ? ks * ra * (1.0 / 30.0) : ks * ra, G);
-        }
-        if (!PLAIN && needK)
-          p2ForPairs<0, 0>([&](auto I, auto Jj) {
-            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-            at(p2UpperIdx(i, j), lane) = tensorEntry<i, j>(G);
-          });
-        if (PLAIN)
-        {
-          double s[4][4], E[6];
-          gramRows(G, s, E);
-          p2ForPairs<0, 0>([&](auto I, auto Jj) {
-            constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-            at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
-          });
-        }
+        double s[4][4], E[6];
+        gramRows(G, s, E);
+        p2ForPairs<0, 0>([&](auto I, auto Jj) {
+          constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+          at(p2UpperIdx(i, j), lane) = p2Stiff<i, j>(s, E);
+        });
       }
       if (needM)
       {
@@ -527,7 +486,7 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
 }
 } // namespace
 
-pxg_status initP2Group(pxg_ctx * ctx)
+pxg_status initP2Group(pxg_ctx * c)
 {
   std::vector<double> xi, w;
   hostRule(P2TET, xi, w);
@@ -555,16 +514,9 @@ pxg_status initP2Group(pxg_ctx * ctx)
       }
     }
   }
-  for (int c = 0; c < 6; ++c)
-    for (int u = 0; u < kP2Pairs; ++u)
-    {
-      if (std::fabs(R.T[c][u]) >= 0.75)
-        return fail(ctx, PXG_ERR_UNSUPPORTED, "P2 stiffness tensors");
-      R.Tx[c][u] = fx::split((int64_t)(R.T[c][u] * 9223372036854775808.0)); // exact from 2^-10
-    }
   for (int k = 0; k < 7; ++k)
     R.mass7[k] = R.mass[p2UpperIdx(p2MassRepI(k), p2MassRepJ(k))];
-  PXG_CUDA(ctx, cudaMemcpyToSymbol(cR, &R, sizeof(R)));
+  PXG_CUDA(c, cudaMemcpyToSymbol(cR, &R, sizeof(R)));
   return PXG_OK;
 }
 

@@ -9,9 +9,13 @@
 // 2^-8 of the largest) in an element whose faces or volume are small enough to show it, an
 // element whose volume cancels against every face, and non-finite, zero and extreme values.
 // About 450 integer instructions and 16 conversions take the place of 75 FP64 operations of 64
-// cycles each: P1 96^3 x 6 in 0.76 ms, 1.14 ms in FP64.  (One exponent for the six products of
-// every element, as P2 has for its regular ones, takes 0.79 ms and loses the small entries:
-// 2^-45 of themselves at a shear of 0.1, 2^-18 beside an edge of 1e-3.)
+// cycles each: P1 96^3 x 6 in 0.75 ms, 1.14 ms in FP64; elements flat along an axis are told by
+// their coordinates' extents before most of it (96^3 x 6 flattened by 1e-3 1.04 ms; refused after
+// the attempt 1.60).  Not kept: one exponent for all six products (0.79 ms), which loses the small
+// entries (2^-45 of themselves at a shear of 0.1, 2^-18 beside an edge of 1e-3); weights of the
+// coordinates for the flat ones (0.84 ms flattened, but 0.81 for all others: 128 registers).  P2's
+// group kernel takes longer with this form (K + M and a load at 64^3 x 6 1.05 to 1.3 ms by shape,
+// FP64 1.01).
 #pragma once
 
 #include "pxg_fx.h"
@@ -66,18 +70,11 @@ PXG_HD uint32_t absHi(int64_t x)
   return (uint32_t)(h < 0 ? -h : h);
 }
 
-// six products g 2^e (xx yy zz xy xz yz) and the determinant det 2^(eD - 60)
-struct Gram
-{
-  int64_t g[6], det;
-  int e[6], eD;
-};
-
-// The products km 2^ke C_a . C_b / |det J| (C the cofactor vectors of J[r][a], the difference of
-// coordinate r of vertex a + 1 to vertex 0; km at F = 62, or zero) and |det J|, each within a few
-// 2^-54 (the mixed ones of |C_a| |C_b|) of the given J's.  False for an element the form refuses,
-// or with ok false.
-PXG_HD bool tetGram(double const (&J)[3][3], bool ok, int64_t km, int ke, Gram & o)
+// G = km 2^ke C_a . C_b / |det J| (xx yy zz xy xz yz; C the cofactor vectors of J[r][a], the
+// difference of coordinate r of vertex a + 1 to vertex 0; km at F = 62, or zero) and |det J|, each
+// within a few 2^-54 (the mixed ones of |C_a| |C_b|) of the given J's.  False for an element the
+// form refuses, or with ok false.
+PXG_HD bool tetGram(double const (&J)[3][3], bool ok, int64_t km, int ke, double (&G)[6], double & adet)
 {
   // edges at F = 61 - e, their largest component in [1/2, 1) 2^e
   Sp x[3][3];
@@ -96,6 +93,24 @@ PXG_HD bool tetGram(double const (&J)[3][3], bool ok, int64_t km, int ke, Gram &
 #pragma unroll
     for (int r = 0; r < 3; ++r)
       x[k][r] = split(roundToInt(scaleExp(J[r][k], 61 - e[k])));
+  }
+  // an element flat along an axis by more than 2^6: nearly all of these would be refused below
+  // (here, not before the conversions: there the kernel takes 100 registers instead of 96, a fifth of
+  // its warps)
+  {
+    int m[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+    {
+      int const a = hi32(doubleBits(J[r][0])) & 0x7fffffff, b = hi32(doubleBits(J[r][1])) & 0x7fffffff,
+                c = hi32(doubleBits(J[r][2])) & 0x7fffffff;
+      m[r] = a > b ? a : b;
+      m[r] = m[r] > c ? m[r] : c;
+    }
+    int const hi = m[0] > m[1] ? (m[0] > m[2] ? m[0] : m[2]) : (m[1] > m[2] ? m[1] : m[2]),
+              lo = m[0] < m[1] ? (m[0] < m[2] ? m[0] : m[2]) : (m[1] < m[2] ? m[1] : m[2]);
+    if (hi - lo > (6 << 20))
+      return false;
   }
   // cofactor vectors, the largest component in [1/4, 1/2) at F = 62: times 2^E
   Sp c[3][3];
@@ -141,57 +156,18 @@ PXG_HD bool tetGram(double const (&J)[3][3], bool ok, int64_t km, int ke, Gram &
   ok = ok && nd >= 0 && nd <= 8 && (exact || (nk + nd <= 12 && nk <= 10));
   if (!ok)
     return false;
-  o.det = nd ? wideShl(d, nd) : d.hi; // F = 60, in [1/2, 1): |det J| = det 2^-60 2^eD
-  o.eD = e[0] + e[1] + e[2] + 5 - nk - nd;
+  int64_t const det = nd ? wideShl(d, nd) : d.hi; // F = 60, in [1/2, 1): |det J| = det 2^-60 2^eD
+  int const eD = e[0] + e[1] + e[2] + 5 - nk - nd;
   // km / det at F = 61
-  Sp const y = split((int64_t)((uint64_t)mul(split((int64_t)((uint64_t)recip(o.det) << 5)), split(km)) << 2));
+  Sp const y = split((int64_t)((uint64_t)mul(split((int64_t)((uint64_t)recip(det) << 5)), split(km)) << 2));
 #pragma unroll
   for (int i = 0; i < 6; ++i)
   {
     int const a = i < 3 ? i : (i == 5 ? 1 : 0), b = i < 3 ? i : (i == 3 ? 1 : 2);
-    o.g[i] = mul(split(dot3(c[a], c[b]) * 4), y);
-    o.e[i] = 65 + E[a] + E[b] - o.eD + ke;
+    G[i] = toDouble(mul(split(dot3(c[a], c[b]) * 4), y), 65 + E[a] + E[b] - eD + ke);
   }
+  adet = toDouble(det, eD - 60);
   return true;
-}
-
-PXG_HD double detOf(Gram const & o) { return toDouble(o.det, o.eD - 60); }
-PXG_HD void toDoubles(Gram const & o, double (&G)[6], double & adet)
-{
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-    G[i] = toDouble(o.g[i], o.e[i]);
-  adet = detOf(o);
-}
-
-// The products as integers with one exponent, the largest in [2^(TOP - 1), 2^TOP).  False where that
-// costs bits that FP64 keeps: a diagonal product below 1/16 of the largest (1 in 12,000 Kuhn
-// tetrahedra with vertices moved by 0.2 of the edge).  TOP = 57: sums of up to 36 times the largest
-// fit, and the sum of all, vertex 0's, is at most twice the largest.
-template <int TOP>
-PXG_HD bool aligned(Gram const & o, int64_t (&g)[6], int & e)
-{
-  bool const none = (o.g[0] | o.g[1] | o.g[2]) == 0; // km = 0
-  int t = -4096;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-  {
-    int const n = o.e[i] + 32 - clz32((uint32_t)hi32(o.g[i]));
-    t = n > t ? n : t;
-  }
-  // (the diagonal ones are above 2^50, so that the upper words have their length)
-  e = t + 32 - TOP;
-#pragma unroll
-  for (int i = 0; i < 6; ++i)
-  {
-    int const r = e - o.e[i];
-    g[i] = r > 0 ? (o.g[i] + (1ll << ((r < 62 ? r : 62) - 1))) >> (r < 62 ? r : 62) : (int64_t)((uint64_t)o.g[i] << -r);
-  }
-  int64_t const m = 1ll << (TOP - 4);
-  bool const ok = g[0] >= m && g[1] >= m && g[2] >= m;
-  if (TOP < 60)
-    return none || (ok && g[0] + g[1] + g[2] + 2 * (g[3] + g[4] + g[5]) <= 1ll << (TOP + 1));
-  return none || ok;
 }
 } // namespace tetx
 } // namespace pxg
