@@ -272,10 +272,9 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
           G[k] = ldexp(G[k], size);
       }
       if (!PLAIN && needK)
-        p2ForPairs<0, 0>([&](auto I, auto Jj) {
-          constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
-          at(p2UpperIdx(i, j), lane) = tensorEntry<i, j>(G);
-        });
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+          at(k, lane) = G[k];
       if (PLAIN)
       {
         double s[4][4], E[6];
@@ -336,6 +335,28 @@ __global__ void __launch_bounds__(64, PLAIN ? 10 : 7) kAssembleP2Group(AsmArgs c
       pdlWait(); // its writes start here
       elementLoad(a, e);
     }
+  }
+  if (!PLAIN && needK)
+  {
+    // the tensors' 201 products are dealt to the two warps (13^3 x 6 with conditions and the sine
+    // load: 65.6 us, by the first alone 67.6; K alone at 6^3 x 6 23.5 and 27.3)
+    __syncthreads();
+    double G[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+      G[k] = at(k, lane);
+    __syncthreads();
+    auto half = [&](auto odd) {
+      p2ForPairs<0, 0>([&](auto I, auto Jj) {
+        constexpr int i = decltype(I)::value, j = decltype(Jj)::value;
+        if constexpr ((p2UpperIdx(i, j) & 1) == decltype(odd)::value)
+          at(p2UpperIdx(i, j), lane) = tensorEntry<i, j>(G);
+      });
+    };
+    if (first)
+      half(std::integral_constant<int, 0>{});
+    else
+      half(std::integral_constant<int, 1>{});
   }
   __syncthreads();
   pdlWait(); // the writes start here
