@@ -102,7 +102,8 @@ struct CgShared
 // over the calling lanes up to one check.
 __device__ __forceinline__ bool cgGiveUp(CgArgs const & g, unsigned polls)
 {
-  bool const up = __any_sync(__activemask(), polls >= (g.extra ? kCgPollsTest : kCgPolls) || *(unsigned volatile *)g.err != 0u);
+  unsigned const most = g.extra ? kCgPollsTest : kCgPolls;
+  bool const up = __any_sync(__activemask(), polls >= most || *(unsigned volatile *)g.err != 0u);
   if (up)
     atomicExch(g.err, 1u);
   return up;

@@ -1,7 +1,8 @@
 // P2 tetrahedra with the warp-group scatter (pxg_group.cu), a block of two warps per group of 32
-// elements.  Warp 0 forms the elements' values in FP64, one element per lane, in barycentric form
-// (pxg_p2bary.h) or by the rule's tensors, and leaves them in shared memory, while warp 1 copies the group's contribution codes there; then both sum
-// the group's distinct positions and add each sum once.  Shared memory (22.5 KB per group) limits
+// elements.  Warp 0 forms the elements' geometry in FP64, one element per lane, and their entries
+// in barycentric form (pxg_p2bary.h), or both warps those by the rule's tensors, while warp 1
+// copies the group's contribution codes to shared memory, where the entries go too; then both sum
+// the group's distinct positions and add each sum once.  Shared memory (22.3 KB per group) limits
 // an SM to ten groups: with one warp per group its ten warps left the map's loads and the
 // additions' latency exposed (13^3 x 6, less than one group per SM sub-partition: 45 us).
 // Loads that need the points (a function but the sine, a DOF field) are warp 1's too where there
